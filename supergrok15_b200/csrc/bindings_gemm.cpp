@@ -3,6 +3,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include "bindings_decl.h"
 #include "mt_host.h"
+#include "newton_schulz.h"
+#include <map>
 
 namespace sg {
 void gemm_plain_tile_coords(int tile, int n_tiles_m, int n_tiles_n, int* mt, int* nt);
@@ -109,6 +111,66 @@ void gemm_tn_reducescatter(const Tensor& a, const Tensor& b, const std::vector<i
                                                   epoch_dev.has_value() ? epoch_dev->data_ptr<int>() : nullptr);
     TORCH_CHECK(rc == 0, "gemm_tn_reducescatter launch failed (code ", rc, ")");
 }
+
+// Newton-Schulz iteration of fp32 matrices [r, c] scaled by inv[i] (device scalars; none: 1), all matrices together; returns the fp32
+// results.  Matrices of one shape are laid out one after the other in a workspace of this call.
+std::vector<Tensor> newton_schulz(const std::vector<Tensor>& mats, const c10::optional<Tensor>& inv, int64_t steps, double a, double b, double c, Tensor err) {
+    const int n = (int)mats.size();
+    std::vector<Tensor> out(n);
+    if (n == 0) return out;
+    TORCH_CHECK(steps >= 1, "newton_schulz needs at least one step");
+    const auto dev = mats[0].device();
+    std::map<std::pair<int64_t, int64_t>, std::vector<int>> shapes;
+    for (int i = 0; i < n; ++i) {
+        const Tensor& m = mats[i];
+        TORCH_CHECK(m.is_cuda() && m.device() == dev && m.scalar_type() == at::kFloat && m.dim() == 2 && m.is_contiguous(), "newton_schulz needs contiguous fp32 CUDA matrices on one device");
+        TORCH_CHECK(m.size(0) < (1 << 30) && m.size(1) < (1 << 30), "newton_schulz: matrix too large");
+        if (m.numel()) shapes[{m.size(0), m.size(1)}].push_back(i);
+        else out[i] = at::empty_like(m);
+    }
+    if (inv.has_value()) TORCH_CHECK(inv->is_cuda() && inv->device() == dev && inv->scalar_type() == at::kFloat && inv->is_contiguous() && inv->numel() >= n, "inv: fp32 [n] on the matrices' device");
+    TORCH_CHECK(err.is_cuda() && err.device() == dev && err.scalar_type() == at::kInt, "err: int32 on the matrices' device");
+    if (shapes.empty()) return out;
+    c10::cuda::CUDAGuard guard(dev);
+    cudaStream_t st = at::cuda::getCurrentCUDAStream();
+    const auto up = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
+    int64_t bytes = 0;
+    for (const auto& kv : shapes) {
+        const int64_t r = kv.first.first, cc = kv.first.second, nb = (int64_t)kv.second.size(), k = std::min(r, cc);
+        bytes += 2 * up(nb * r * ((cc + 7) / 8 * 8) * 2) + 2 * up(nb * k * ((k + 7) / 8 * 8) * 2);
+    }
+    Tensor ws = at::empty({bytes}, mats[0].options().dtype(at::kByte));
+    uint8_t* base = ws.data_ptr<uint8_t>();
+    std::vector<sg::NsGroup> groups;
+    std::vector<const float*> src(n);
+    std::vector<void*> dst(n);
+    std::vector<int> rows(n), cols(n);
+    std::vector<Tensor> keep;
+    for (const auto& kv : shapes) {
+        const int64_t r = kv.first.first, cc = kv.first.second, nb = (int64_t)kv.second.size(), k = std::min(r, cc);
+        const int64_t ld = (cc + 7) / 8 * 8, ld4 = (cc + 3) / 4 * 4, lk = (k + 7) / 8 * 8;
+        const auto take = [&](int64_t elems) { void* p = base; base += up(elems * 2); return reinterpret_cast<__nv_bfloat16*>(p); };
+        sg::NsGroup g{};
+        g.r = (int)r; g.c = (int)cc; g.batch = (int)nb;
+        g.x0 = take(nb * r * ld); g.x1 = take(nb * r * ld);
+        g.g = take(nb * k * lk); g.p = take(nb * k * lk);
+        Tensor o = at::empty({nb, r, ld4}, mats[0].options());
+        g.out32 = o.data_ptr<float>();
+        keep.push_back(o);
+        for (int64_t z = 0; z < nb; ++z) {
+            const int i = kv.second[z];
+            src[i] = mats[i].data_ptr<float>();
+            dst[i] = g.x0 + z * r * ld;
+            rows[i] = (int)r; cols[i] = (int)cc;
+            out[i] = o.select(0, z).narrow(1, 0, cc);
+        }
+        groups.push_back(g);
+    }
+    sg::ns_cast(src.data(), dst.data(), rows.data(), cols.data(), n, inv.has_value() ? inv->data_ptr<float>() : nullptr, st);
+    const int rc = sg::ns_iterate(groups.data(), (int)groups.size(), (int)steps, (float)a, (float)b, (float)c, err.data_ptr<int>(), st);
+    TORCH_CHECK(rc == 0, "newton_schulz launch failed (code ", rc, ")");
+    return out;
+}
 }  // namespace
 
 void register_gemm(pybind11::module_& m) {
@@ -120,6 +182,16 @@ void register_gemm(pybind11::module_& m) {
             order.emplace_back(mt, nt);
         }
         return order;
+    });
+    m.def("newton_schulz", &newton_schulz, py::arg("mats"), py::arg("inv"), py::arg("steps"), py::arg("a"), py::arg("b"), py::arg("c"), py::arg("err"));
+    m.def("ns_sym_tiles", [](int64_t n, int64_t bn) {                             // (row, column, mirrored) of the tiles of a symmetric product
+        std::vector<std::tuple<int64_t, int64_t, bool>> v;
+        for (int t = 0; t < sg::ns_sym_tile_count((int)n, (int)bn); ++t) {
+            int m0, n0, mirror;
+            sg::ns_sym_tile_coords(t, (int)bn, &m0, &n0, &mirror);
+            v.emplace_back(m0, n0, mirror != 0);
+        }
+        return v;
     });
     m.def("gemm_tn", &gemm_tn, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("alpha") = 1.0, py::arg("beta") = 0.0,
           py::arg("d") = c10::nullopt, py::arg("bias") = c10::nullopt, py::arg("diag") = 0.0, py::arg("act") = 0,

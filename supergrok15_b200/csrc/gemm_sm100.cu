@@ -534,13 +534,11 @@ __global__ void __launch_bounds__(256) gemm_splitk_reduce_kernel(const float* __
 // ---- host side -------------------------------------------------------------------------------------------------
 }  // namespace
 static int g_map_error = 0;                      // CUresult of the most recent encode (diagnostics only)
-bool tc::make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld_elems, int box_rows, int box_cols, bool bf16) {
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld_elems * (bf16 ? 2 : 4)};
-    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    // The driver entry point is looked up through the runtime, so that the module links against cudart only and loads on a host
-    // that has no driver library (a build-only machine).
+namespace {
+// Encodes a tiled map of `rank` dimensions.  The driver entry point is looked up through the runtime, so that the module links
+// against cudart only and loads on a host that has no driver library (a build-only machine).
+bool encode_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box, bool bf16,
+                bool swizzle128) {
     using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     static EncodeFn encode = [] {
@@ -550,18 +548,36 @@ bool tc::make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols
         return reinterpret_cast<EncodeFn>(fn);
     }();
     if (!encode) { g_map_error = -1; return false; }
-    CUresult r = encode(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
-                                              const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const auto go = [&] {
+        return encode(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, (cuuint32_t)rank, const_cast<void*>(base), dims, strides,
+                      box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = go();
     if (r == CUDA_ERROR_INVALID_CONTEXT) {
         // A host thread that has made no runtime call yet (an autograd worker thread, for one) has no current context for the
         // driver API: bind the primary context of the current device and try once more.
         cudaFree(nullptr);
-        r = encode(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        r = go();
     }
     g_map_error = (int)r;
     return r == CUDA_SUCCESS;
+}
+}  // namespace
+bool tc::make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld_elems, int box_rows, int box_cols, bool bf16) {
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld_elems * (bf16 ? 2 : 4)};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+    return encode_map(map, base, 2, dims, strides, box, bf16, true);
+}
+bool tc::make_map_batched(CUtensorMap* map, const void* base, int64_t batch, int64_t rows, int64_t cols, int64_t ld_elems, int box_rows, int box_cols, bool bf16,
+                          bool swizzle128) {
+    const cuuint64_t row = (cuuint64_t)ld_elems * (bf16 ? 2 : 4);
+    const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
+    const cuuint64_t strides[2] = {row, row * (cuuint64_t)rows};
+    const cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
+    return encode_map(map, base, 3, dims, strides, box, bf16, swizzle128);
 }
 int tc::last_map_error() { return g_map_error; }
 namespace {

@@ -131,12 +131,12 @@ def _mm3(a32: torch.Tensor, b32: torch.Tensor, *, alpha=1.0, beta=0.0, d=None, d
 
 
 def newton_schulz(X: torch.Tensor, steps: int, coeffs, precision: str = "bf16") -> torch.Tensor:
-    """X <- aX + b(XX^T)X + c(XX^T)^2X, `steps` times, on the tcgen05 GEMM.  X fp32 [r,c] -> fp32 [r,c].
+    """X <- aX + b(XX^T)X + c(XX^T)^2X, `steps` times, on the tensor cores.  X fp32 [r,c] -> fp32 [r,c].
 
     rows >= cols: right-Gram form  G = X^T X, P = aI + bG + cG^2, X <- X P   (cols^2-sized intermediates);
     rows <  cols: left form        A = X X^T, Q = aI + bA + cA^2, X <- Q X.
-    ``precision="bf16"``: operands are rounded to bf16 once per product (fp32 accumulation in TMEM); X and X^T are both kept,
-    so every GEMM is K-major on both operands.  The reference iterates in fp32 (``torch::mm`` with TF32 off, reference
+    ``precision="bf16"``: operands are rounded to bf16 once per product (fp32 accumulation in TMEM), on the grouped kernel of
+    ``csrc/newton_schulz.cu`` (many matrices at once: ``ops/muon.py``).  The reference iterates in fp32 (``torch::mm`` with TF32 off, reference
     csrc/ops.cpp:713-727); the bf16 iteration differs from it by a few per cent in Frobenius norm, which Muon tolerates (the
     iteration is a contraction towards the orthogonal factor).  ``precision="bf16x3"``: every product is three bf16 products of
     hi / lo splits with fp32 results carried between the products (~16 bits per product, 3x the tensor-core work): within
@@ -155,36 +155,5 @@ def newton_schulz(X: torch.Tensor, steps: int, coeffs, precision: str = "bf16") 
             Pm = _mm3(G, G, alpha=c, beta=b, d=G, diag=a)                # symmetric
             X32 = _mm3(X32, Pm) if tall else _mm3(Pm, X32.t().contiguous())
         return X32
-    rp, cp = -(-r // 8) * 8, -(-cc // 8) * 8
-    dev = X.device
-    Xb = torch.zeros(r, cp, dtype=torch.bfloat16, device=dev)[:, :cc]
-    XTb = torch.zeros(cc, rp, dtype=torch.bfloat16, device=dev)[:, :r]
-    Xb.copy_(X)
-    XTb.copy_(X.t())
-    tall = r >= cc
-    n = cc if tall else r
-    npad = -(-n // 8) * 8
-    G = torch.zeros(n, npad, dtype=torch.bfloat16, device=dev)[:, :n]
-    P = torch.zeros(n, npad, dtype=torch.bfloat16, device=dev)[:, :n]
-    out32 = torch.empty(r, -(-cc // 4) * 4, dtype=torch.float32, device=dev)[:, :cc]
-    # ping-pong operand buffers allocated once per call (not once per iteration)
-    Xn = torch.empty(r, cp, dtype=torch.bfloat16, device=dev)[:, :cc]
-    XTn = torch.empty(cc, rp, dtype=torch.bfloat16, device=dev)[:, :r]
-    for it in range(steps):
-        last = it == steps - 1
-        src = XTb if tall else Xb
-        gemm_tn(src, src, out=G)                                            # Gram matrix (symmetric)
-        gemm_tn(G, G, out=P, alpha=c, beta=b, d=G, diag=a)                  # aI + bG + cG^2 (symmetric)
-        if last:
-            if tall:
-                gemm_tn(Xb, P, out=out32)                                   # X P
-            else:
-                gemm_tn(P, XTb, out=out32)                                  # Q X   (B operand = X^T [c, r])
-        else:
-            if tall:
-                gemm_tn(Xb, P, out=Xn, out_t=XTn)
-            else:
-                gemm_tn(P, XTb, out=Xn, out_t=XTn)
-            Xb, Xn = Xn, Xb
-            XTb, XTn = XTn, XTb
-    return out32
+    C = _build.require()
+    return C.newton_schulz([X.float().contiguous()], None, steps, a, b, c, _err_flag(X.device))[0]

@@ -19,15 +19,20 @@ from . import oracle
 NS_COEFFS = oracle.NS_COEFFS
 
 
+# Matrix elements per run of the grouped iteration: 10 to 12 bytes of workspace each (two bf16 iterates, the fp32 result, G and P), so
+# at most ~3 GB; a run of this size is several milliseconds of tensor-core work, its launches are not what bounds it.
+NS_RUN_ELEMS = 1 << 28
+
+
 def newton_schulz_cuda(X: torch.Tensor, steps: int, precision: str = "bf16") -> torch.Tensor:
     """Newton-Schulz on the tcgen05 GEMM kernels.  X fp32 [r,c] (already normalised); returns fp32 [r,c]."""
     from . import gemm
     return gemm.newton_schulz(X, steps, NS_COEFFS, precision)
 
 
-# Newton-Schulz chains captured as CUDA graphs, keyed by the momentum buffers they read: a step over 21 owned matrices is ~450
-# short launches (15 GEMMs plus casts per matrix) that the host cannot issue as fast as the GPU runs them; replayed from a graph they
-# are one launch.  The first call for a set of buffers runs eagerly (lazy initialisation), the second is captured.
+# Split-precision Newton-Schulz chains captured as CUDA graphs, keyed by the momentum buffers they read: a step over 21 owned matrices
+# is over a thousand short launches that the host cannot issue as fast as the GPU runs them; replayed from a graph they are one launch.
+# The first call for a set of buffers runs eagerly (lazy initialisation), the second is captured.
 _ns_graphs = {}
 
 
@@ -75,5 +80,18 @@ def muon_step(params: List[torch.Tensor], grads, bufs, lr: float, momentum: floa
                per_tensor_out=pt)
     inv = ew.workspace(dev, "muon_inv", n)
     C.scalar_finalize(C.ops["SC_MUON_NORMS"], pt, n, inv, 0.0, 0.0, 0.0)
-    xs = _ns_graphed(list(bufs), inv, ns_steps, precision)
-    C.mt_apply(C.ops["OP_MUON_UPDATE"], [params, xs], [], [0, 0, 0, 0, 0, 0, 0, 0, -0.2 * lr, 1.0 - lr * wd])
+    scalars = [0, 0, 0, 0, 0, 0, 0, 0, -0.2 * lr, 1.0 - lr * wd]
+    if precision != "bf16":
+        C.mt_apply(C.ops["OP_MUON_UPDATE"], [params, _ns_graphed(list(bufs), inv, ns_steps, precision)], [], scalars)
+        return
+    # all matrices of the step share the launches of the iteration; long lists go in runs that bound the workspace
+    from . import gemm
+    i = 0
+    while i < n:
+        j, elems = i, 0
+        while j < n and (j == i or elems + bufs[j].numel() <= NS_RUN_ELEMS):
+            elems += bufs[j].numel()
+            j += 1
+        xs = C.newton_schulz(list(bufs[i:j]), inv[i:j], ns_steps, *NS_COEFFS, gemm._err_flag(dev))
+        C.mt_apply(C.ops["OP_MUON_UPDATE"], [list(params[i:j]), [x.contiguous() for x in xs]], [], scalars)
+        i = j
