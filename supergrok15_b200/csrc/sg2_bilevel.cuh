@@ -164,8 +164,8 @@ __device__ __forceinline__ void bl_advance_tile(const ColConst<DIR>& cc, const f
             float abe, abo, cs, sn;
             pair_coeffs(dt, cc.ah[2 * p], cc.ah[2 * p + 1], cc.f[p], abe, abo, cs, sn);
             const float he = h[2 * p], ho = h[2 * p + 1];
-            h[2 * p] = fmaf(abe, he * cs - ho * sn, dtx * row[2 * p]);
-            h[2 * p + 1] = fmaf(abo, ho * cs + he * sn, dtx * row[2 * p + 1]);
+            h[2 * p] = fmaf(abe, he * cs - ho * sn, dtx * row[row_pos(2 * p)]);
+            h[2 * p + 1] = fmaf(abo, ho * cs + he * sn, dtx * row[row_pos(2 * p + 1)]);
         }
     }
 }

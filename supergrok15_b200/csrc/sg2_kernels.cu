@@ -10,15 +10,14 @@
 //   scan 1    per-chunk aggregate 2x2 affine maps        (only tensors split into several chunks)
 //   scan 2    carry-in state of every chunk              (tiny)
 //   scan 3    re-run every chunk from its carry-in, apply SiLU gate / D skip / out_proj and write the
-//             8-float context straight to the element's ORIGINAL index (no un-sort gathers)
+//             8-float context straight to the element's ORIGINAL index (no un-sort gathers); two forms, a warp or half a warp per chunk
 //   elem      GRU + 4-head product-key routing + expert MLPs (shared memory) + mu EMA + Adam
 //
 // Scan decomposition: the sequence of a tensor is cut into chunks of `chunk_len` timesteps; an item is
-// (tensor, direction, chunk).  Sixteen lanes (one per d_inner column) own an item; each lane keeps the
-// 16 state values of its column (8 RoPE pairs) in registers, so y is accumulated in registers and
-// nothing is read-modify-written in global memory.  Per 16-timestep tile the lanes first act as
-// "one lane per timestep" to compute x, z, dt, B, C with warp-uniform weights from constant memory,
-// park them in shared memory, then act as "one lane per column" for the recurrence.
+// (tensor, direction, chunk).  The lanes of an item each own states of one d_inner column (RoPE pairs) in
+// registers, so y is accumulated in registers and nothing is read-modify-written in global memory.  Per tile
+// of timesteps the lanes first act as "one lane per timestep" to compute B and C with warp-uniform weights
+// from constant memory, park them in shared memory, then act as "lane = column" for the recurrence.
 // The meta-net weights (11,580 floats) live in __constant__ memory; the 144 experts are staged in
 // shared memory by the element kernel because their index is data dependent.
 #include "sg_native.h"
@@ -35,11 +34,9 @@ using P = SG2Pack;
 constexpr int TILE_T = 16;                 // timesteps per tile
 constexpr int ROW = 52;                    // floats per timestep row in shared memory: B[16] C[16] (g,s,-,-) out[16]; 13 float4 (odd) keeps 128-bit stores conflict free
 constexpr int SCAN_THREADS = 128;          // 8 items per CTA
-#ifndef SG_SCAN_MINB
-#define SG_SCAN_MINB 3                     // resident CTAs per SM the scan kernel is compiled for (phase 3 at 18.9 M parameters: 6.07 / 6.00 / 6.39 ms with 2 / 3 / 4)
-#endif
-
+constexpr int COL_MINB = 4, WARP_MINB = 5;  // resident CTAs per SM of the two forms of phase 3
 constexpr int ITEMS_PER_CTA = SCAN_THREADS / 16;
+constexpr int SCAN3_THREADS = 128, ITEMS3 = SCAN3_THREADS / 32;      // phase 3: a warp per item
 
 __device__ __forceinline__ float softplus20(float x) { return x > 20.f ? x : __logf(1.f + __expf(x)); }
 __device__ __forceinline__ float silu(float x) { return x / (1.f + __expf(-x)); }
@@ -184,7 +181,10 @@ struct TensorDir {     // 32 bytes
 // the chain into five [16][3] tables per direction (SG2Pack::AFF*: coefficient of g, coefficient of s, constant), computed in
 // fp64.  Per timestep the precompute is then 160 FMAs instead of 1040, and x / z / dt are evaluated by the column's own lane.
 //
-// Stage A: lane l = timestep (u0 + l): B[16], C[16] and (g, s) of that timestep go to its shared-memory row.
+// Stage A: lane l = timestep (u0 + l): B[16], C[16] and (g, s) of that timestep go to its shared-memory row.  The 16 states are stored in
+// the order row_pos() gives: the even states of two neighbouring RoPE pairs side by side, then their odd states, so that one 16-byte load
+// hands the recurrence two packed f32x2 operands.
+__host__ __device__ constexpr int row_pos(int s) { return (s & ~3) | ((s & 1) << 1) | ((s >> 1) & 1); }      // its own inverse
 template <int DIR>
 __device__ __forceinline__ void stage_a(float* __restrict__ tile, const float2* __restrict__ gs, int64_t off, int n, int u, bool valid,
                                         int l) {
@@ -200,7 +200,7 @@ __device__ __forceinline__ void stage_a(float* __restrict__ tile, const float2* 
         bc[k] = fmaf(c_w[w], v.x, fmaf(c_w[w + 1], v.y, c_w[w + 2]));
     }
 #pragma unroll
-    for (int q = 0; q < 8; ++q) row[q] = make_float4(bc[4 * q], bc[4 * q + 1], bc[4 * q + 2], bc[4 * q + 3]);
+    for (int q = 0; q < 8; ++q) row[q] = make_float4(bc[4 * q], bc[4 * q + 2], bc[4 * q + 1], bc[4 * q + 3]);
     row[8] = make_float4(v.x, v.y, 0.f, 0.f);
 }
 
@@ -224,6 +224,69 @@ __device__ __forceinline__ void pair_coeffs(float dt, float ah_e, float ah_o, fl
     __sincosf(dt * f, &sn, &cs);
 }
 
+// ---- two RoPE pairs at a time: packed f32x2 arithmetic ----
+// One issue slot does two FMAs, but the register file still delivers two 32-bit operands per lane and cycle: measured 2.4 to 3.1 cycles
+// for fma.rn.f32x2 against 1.5 to 2.1 for a scalar FMA (148 SMs, all warps), 8.1 for a special function.  The scan needs ~290 operand
+// cycles, 200 issue slots and 28 special functions (226 cycles) per 32 lanes and timestep and takes ~345; the scalar form (257 issue
+// slots) took ~395.  18.9 M parameters, phase 3: 6.36 ms -> 5.53 ms.  Scalar forms of single operations (immediate operands, free
+// negation), one reciprocal per four denominators, 3 / 4 / 5 CTAs per SM and an unrolled pair of timesteps all measured 5.5 to 5.9.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pk(float lo, float hi) { f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ void upk(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) { f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+
+// Transitions of a group (two RoPE pairs).  One reciprocal serves both states of a pair (1/de = dn / (de dn)); sharing one among all four
+// denominators was measured equal (the special-function pipe is not what bounds the scan, see scan_phase3).
+// Denominators grow with dt; from dt = 1e8 on Abar is -1 to the last bit whatever the exact value, so dt is capped there and the
+// product of two denominators cannot overflow.
+__device__ __forceinline__ void quad_coeffs(f2 ndt, f2 dt, f2 ah_e, f2 ah_o, f2 f, f2& abe, f2& abo, f2& cs, f2& sn) {
+    const f2 one = pk(1.f, 1.f), mone = pk(-1.f, -1.f);
+    const f2 de = fma2(ndt, ah_e, one), dn = fma2(ndt, ah_o, one);
+    float p0, p1, t0, t1;
+    upk(mul2(de, dn), p0, p1);
+    const f2 r2 = mul2(pk(rcp_approx(p0), rcp_approx(p1)), pk(2.f, 2.f));
+    abe = fma2(dn, r2, mone);
+    abo = fma2(de, r2, mone);
+    upk(mul2(dt, f), t0, t1);
+    float s0, c0, s1, c1;
+    __sincosf(t0, &s0, &c0);
+    __sincosf(t1, &s1, &c1);
+    cs = pk(c0, c1);
+    sn = pk(s0, s1);
+}
+
+// constants of lane j for the packed recurrence: group q holds the RoPE pairs 2q and 2q + 1
+template <int DIR>
+struct ColPacked {
+    f2 ahe[4], aho[4], f[4];
+    float ux[3], uz[3], ud[3], Dj;
+    __device__ __forceinline__ void load(int j) {
+        constexpr int W = (DIR == 0) ? P::DIR0 : P::DIR1;
+        constexpr int AF = (DIR == 0) ? P::AFF0 : P::AFF1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int w = W + P::D_ALOG + j * 16 + 4 * q;
+            ahe[q] = pk(-0.5f * __expf(c_w[w]), -0.5f * __expf(c_w[w + 2]));
+            aho[q] = pk(-0.5f * __expf(c_w[w + 1]), -0.5f * __expf(c_w[w + 3]));
+            f[q] = pk(c_w[W + P::D_ROPE + j * 8 + 2 * q], c_w[W + P::D_ROPE + j * 8 + 2 * q + 1]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            ux[k] = c_w[AF + P::A_X + 3 * j + k]; uz[k] = c_w[AF + P::A_Z + 3 * j + k]; ud[k] = c_w[AF + P::A_DT + 3 * j + k];
+        }
+        Dj = c_w[W + P::D_D + j];
+        // The values differ from lane to lane, so a load from __constant__ memory takes one pass per lane.  Without this fence the compiler
+        // finds it cheaper to load (and exponentiate) them again in every timestep than to hold them in registers.
+#pragma unroll
+        for (int q = 0; q < 4; ++q) asm volatile("" : "+l"(ahe[q]), "+l"(aho[q]), "+l"(f[q]));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) asm volatile("" : "+f"(ux[k]), "+f"(uz[k]), "+f"(ud[k]));
+        asm volatile("" : "+f"(Dj));
+    }
+};
+constexpr float DT_CAP = 1e8f;
+
 // column constants of lane j: A/2, rope frequencies, and the affine tables of x_j, z_j, dt_j
 template <int DIR>
 struct ColConst {
@@ -244,54 +307,185 @@ struct ColConst {
 };
 
 // PHASE 3: run a chunk forward from its carry-in; apply SiLU gate, D skip and out_proj; write the contexts.
-// The recurrence stays scalar with sin.approx / cos.approx on the special-function unit: two rewrites that take the sincos off
-// that unit (packed f32x2 arithmetic over pairs of RoPE pairs; degree-5 / degree-6 polynomials for |theta| <= 0.25) were measured
-// at 18.9 M parameters and ran this phase in 23.5 ms and 24.2 ms against 6.4 ms for this form; so did a hand-made software
-// pipeline that computes the coefficients of step l + 1 during the recurrence of step l (10.5 ms at two CTAs per SM, 34.8 ms at three).
+// Warp-per-item form: lane = (half, column j), a lane carries four of the column's eight RoPE pairs (two packed groups), which halves the
+// instructions of a timestep per warp; it is used while every item has its own warp at once and the chain of one chunk takes the time
+// (422,755 parameters, 1,678 items: column form 212 us, this form 177 us; at 18.9 M parameters 5.5 ms against 6.1 ms).
+// Per 32-timestep tile the 32 lanes stand for the timesteps (B, C; later the output projection); per 16 timesteps the lanes then
+// evaluate dt, x and the SiLU gate of all columns, which depend on nothing but (g, s); the recurrence only loads them.
+constexpr int T3 = 32, R3 = 36;                         // tile rows: B[16] / out[16], C[16], (g, s, -, -): 9 float4, conflict free
+constexpr int PRE3 = 16 * 48;                            // dt[16] x[16] gate[16] of 16 timesteps
+constexpr int SM3 = T3 * R3 + PRE3;
 template <int DIR>
 __device__ void scan_phase3(const Item& it, const TensorDir* __restrict__ tds, const float2* __restrict__ gs,
                             const uint32_t* __restrict__ vals_sorted, const float* __restrict__ carry, float* __restrict__ ctx,
+                            float* __restrict__ tile, const float* __restrict__ ucol, int item_idx, int lane) {
+    constexpr int W = (DIR == 0) ? P::DIR0 : P::DIR1;
+    constexpr int AF = (DIR == 0) ? P::AFF0 : P::AFF1;
+    const int j = lane & 15, half = lane >> 4;
+    float* pre = tile + T3 * R3;
+    f2 ahe[2], aho[2], f[2], he[2], ho[2];
+    float Dj = c_w[W + P::D_D + j];
+    {
+        const float* cin = carry + ((int64_t)item_idx * 16 + j) * 16 + 8 * half;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int w = W + P::D_ALOG + j * 16 + 8 * half + 4 * q, r = W + P::D_ROPE + j * 8 + 4 * half + 2 * q;
+            ahe[q] = pk(-0.5f * __expf(c_w[w]), -0.5f * __expf(c_w[w + 2]));
+            aho[q] = pk(-0.5f * __expf(c_w[w + 1]), -0.5f * __expf(c_w[w + 3]));
+            f[q] = pk(c_w[r], c_w[r + 1]);
+            const float4 t = reinterpret_cast<const float4*>(cin)[q];
+            he[q] = pk(t.x, t.z); ho[q] = pk(t.y, t.w);
+            // the constants differ from lane to lane, so a load from __constant__ memory takes one pass per lane: without this fence the
+            // compiler loads (and exponentiates) them again in every timestep rather than hold them in registers (2.6 times slower)
+            asm volatile("" : "+l"(ahe[q]), "+l"(aho[q]), "+l"(f[q]));
+        }
+        asm volatile("" : "+f"(Dj));
+    }
+    const auto where = [&](int u) { return it.off + ((DIR == 0) ? u : (it.n - 1 - u)); };
+    float2 v = make_float2(0.f, 0.f);
+    uint32_t orig = 0;
+    if (it.ub + lane < it.ue) { v = gs[where(it.ub + lane)]; orig = vals_sorted[where(it.ub + lane)]; }
+    for (int u0 = it.ub; u0 < it.ue; u0 += T3) {
+        const int cnt = (it.ue - u0 < T3) ? (it.ue - u0) : T3;
+        {   // lane = timestep: B and C of its row
+            float4* row = reinterpret_cast<float4*>(tile + lane * R3);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                float bc[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int w = AF + P::A_B + 3 * (4 * q + k);
+                    bc[k] = fmaf(c_w[w], v.x, fmaf(c_w[w + 1], v.y, c_w[w + 2]));
+                }
+                row[q] = make_float4(bc[0], bc[2], bc[1], bc[3]);
+            }
+            *reinterpret_cast<float2*>(tile + lane * R3 + 32) = v;
+        }
+        uint32_t orig_n = 0;
+        if (u0 + T3 + lane < it.ue) { v = gs[where(u0 + T3 + lane)]; orig_n = vals_sorted[where(u0 + T3 + lane)]; }      // next tile
+        __syncwarp();
+#pragma unroll 1
+        for (int l0 = 0; l0 < cnt; l0 += 16) {
+            {   // lane = column, the halves take every other timestep
+                const float4 ua = reinterpret_cast<const float4*>(ucol)[0], ub = reinterpret_cast<const float4*>(ucol)[1];
+                const float uc = ucol[8];
+#pragma unroll 4
+                for (int i = 0; i < 8; ++i) {
+                    const int l = 2 * i + half;
+                    const float2 w = *reinterpret_cast<const float2*>(tile + (l0 + l) * R3 + 32);
+                    const float x = fmaf(ua.x, w.x, fmaf(ua.y, w.y, ua.z));
+                    const float z = fmaf(ua.w, w.x, fmaf(ub.x, w.y, ub.y));
+                    const float dt = softplus20(fmaf(ub.z, w.x, fmaf(ub.w, w.y, uc)));
+                    pre[l * 48 + j] = dt;
+                    pre[l * 48 + 16 + j] = x;
+                    pre[l * 48 + 32 + j] = silu(z);
+                }
+            }
+            __syncwarp();
+            const int lc = cnt - l0 < 16 ? cnt - l0 : 16;
+#pragma unroll 1
+            for (int l = 0; l < lc; ++l) {
+                float* row = tile + (l0 + l) * R3;
+                const float dt = pre[l * 48 + j], x = pre[l * 48 + 16 + j];
+                const float ndtc = -fminf(dt, DT_CAP), dtx = dt * x;
+                const f2 ndt2 = pk(ndtc, ndtc), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
+                f2 ysum = pk(0.f, 0.f);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const ulonglong2 B = reinterpret_cast<const ulonglong2*>(row + 8 * half)[q], C = reinterpret_cast<const ulonglong2*>(row + 16 + 8 * half)[q];
+                    f2 abe, abo, cs, sn;
+                    quad_coeffs(ndt2, dt2, ahe[q], aho[q], f[q], abe, abo, cs, sn);
+                    const f2 re = fma2(ho[q], mul2(sn, mone), mul2(he[q], cs)), ro = fma2(he[q], sn, mul2(ho[q], cs));
+                    he[q] = fma2(abe, re, mul2(dtx2, B.x));
+                    ho[q] = fma2(abo, ro, mul2(dtx2, B.y));
+                    ysum = fma2(he[q], C.x, fma2(ho[q], C.y, ysum));
+                }
+                float ya, yb;
+                upk(ysum, ya, yb);
+                ya += yb;
+                ya += __shfl_xor_sync(0xffffffffu, ya, 16);
+                // out_j of this timestep takes the place of its B, which every lane has read (the shuffle waited for their sums)
+                if (half == 0) row[j] = fmaf(ya, pre[l * 48 + 32 + j], Dj * x);
+            }
+            __syncwarp();
+        }
+        if (lane < cnt) {                                 // lane = timestep again: ctx = out_proj . out at the ORIGINAL index
+            const float* row = tile + lane * R3;
+            float o[16];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) { const float4 t = reinterpret_cast<const float4*>(row)[q]; o[4 * q] = t.x; o[4 * q + 1] = t.y; o[4 * q + 2] = t.z; o[4 * q + 3] = t.w; }
+            float c8[8];
+#pragma unroll
+            for (int d = 0; d < 8; ++d) {
+                float acc = 0.f;
+#pragma unroll
+                for (int k = 0; k < 16; ++k) acc = fmaf(c_w[W + P::D_OUT + d * 16 + k], o[k], acc);
+                c8[d] = acc;
+            }
+            float4* dst = reinterpret_cast<float4*>(ctx + (int64_t)orig * 16 + DIR * 8);
+            dst[0] = make_float4(c8[0], c8[1], c8[2], c8[3]);
+            dst[1] = make_float4(c8[4], c8[5], c8[6], c8[7]);
+        }
+        orig = orig_n;
+        __syncwarp();
+    }
+    if (it.last) {
+        float* dst = tds[it.td].h + j * 16 + 8 * half;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            float4 t;
+            upk(he[q], t.x, t.z); upk(ho[q], t.y, t.w);
+            reinterpret_cast<float4*>(dst)[q] = t;
+        }
+    }
+}
+
+// PHASE 3, sixteen lanes per item (a lane carries a whole column, eight RoPE pairs): the form for steps with more chunks than the
+// warp-per-item form holds at once, where the column's own work (dt, x, gate, loads) should not be split over two lanes.
+template <int DIR>
+__device__ void scan_phase3_col(const Item& it, const TensorDir* __restrict__ tds, const float2* __restrict__ gs,
+                            const uint32_t* __restrict__ vals_sorted, const float* __restrict__ carry, float* __restrict__ ctx,
                             float* __restrict__ tile, int item_idx, int j, unsigned hmask) {
     constexpr int W = (DIR == 0) ? P::DIR0 : P::DIR1;
-    ColConst<DIR> cc;
+    ColPacked<DIR> cc;
     cc.load(j);
-    float h[16];
+    f2 he[4], ho[4];
     {
         const float* cin = carry + ((int64_t)item_idx * 16 + j) * 16;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) { const float4 t = reinterpret_cast<const float4*>(cin)[q]; h[4 * q] = t.x; h[4 * q + 1] = t.y; h[4 * q + 2] = t.z; h[4 * q + 3] = t.w; }
+        for (int q = 0; q < 4; ++q) { const float4 t = reinterpret_cast<const float4*>(cin)[q]; he[q] = pk(t.x, t.z); ho[q] = pk(t.y, t.w); }
     }
     for (int u0 = it.ub; u0 < it.ue; u0 += TILE_T) {
         const int cnt = (it.ue - u0 < TILE_T) ? (it.ue - u0) : TILE_T;
         stage_a<DIR>(tile, gs, it.off, it.n, u0 + j, j < cnt, j);
         __syncwarp(hmask);
-        for (int l = 0; l < cnt; ++l) {                 // lane j = column (unrolling two timesteps together was measured 4 % slower)
+        float2 v = *reinterpret_cast<const float2*>(tile + 32);
+        float dt = softplus20(fmaf(cc.ud[0], v.x, fmaf(cc.ud[1], v.y, cc.ud[2])));
+#pragma unroll 1
+        for (int l = 0; l < cnt; ++l) {                 // lane j = column
             float* row = tile + l * ROW;
-            const float2 v = *reinterpret_cast<const float2*>(row + 32);
             const float x = fmaf(cc.ux[0], v.x, fmaf(cc.ux[1], v.y, cc.ux[2]));
             const float z = fmaf(cc.uz[0], v.x, fmaf(cc.uz[1], v.y, cc.uz[2]));
-            const float dt = softplus20(fmaf(cc.ud[0], v.x, fmaf(cc.ud[1], v.y, cc.ud[2])));
-            float B[16], C[16];
+            const float ndtc = -fminf(dt, DT_CAP), dtx = dt * x;
+            const f2 ndt2 = pk(ndtc, ndtc), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
+            // dt of the next timestep: its logarithm and exponential start a step ahead of the recurrence that needs them
+            const float2 vn = *reinterpret_cast<const float2*>(row + (l + 1 < cnt ? ROW : 0) + 32);
+            const float dtn = softplus20(fmaf(cc.ud[0], vn.x, fmaf(cc.ud[1], vn.y, cc.ud[2])));
+            f2 y2 = pk(0.f, 0.f);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const float4 t = reinterpret_cast<const float4*>(row)[q];
-                B[4 * q] = t.x; B[4 * q + 1] = t.y; B[4 * q + 2] = t.z; B[4 * q + 3] = t.w;
-                const float4 c = reinterpret_cast<const float4*>(row + 16)[q];
-                C[4 * q] = c.x; C[4 * q + 1] = c.y; C[4 * q + 2] = c.z; C[4 * q + 3] = c.w;
+                const ulonglong2 B = reinterpret_cast<const ulonglong2*>(row)[q], C = reinterpret_cast<const ulonglong2*>(row + 16)[q];
+                f2 abe, abo, cs, sn;
+                quad_coeffs(ndt2, dt2, cc.ahe[q], cc.aho[q], cc.f[q], abe, abo, cs, sn);
+                const f2 re = fma2(ho[q], mul2(sn, mone), mul2(he[q], cs)), ro = fma2(he[q], sn, mul2(ho[q], cs));
+                he[q] = fma2(abe, re, mul2(dtx2, B.x));
+                ho[q] = fma2(abo, ro, mul2(dtx2, B.y));
+                y2 = fma2(he[q], C.x, fma2(ho[q], C.y, y2));
             }
-            const float dtx = dt * x;
-            float y = 0.f;
-#pragma unroll
-            for (int p = 0; p < 8; ++p) {
-                float abe, abo, cs, sn;
-                pair_coeffs(dt, cc.ah[2 * p], cc.ah[2 * p + 1], cc.f[p], abe, abo, cs, sn);
-                const float he = h[2 * p], ho = h[2 * p + 1];
-                const float ne = fmaf(abe, he * cs - ho * sn, dtx * B[2 * p]);
-                const float no = fmaf(abo, ho * cs + he * sn, dtx * B[2 * p + 1]);
-                h[2 * p] = ne; h[2 * p + 1] = no;
-                y = fmaf(ne, C[2 * p], fmaf(no, C[2 * p + 1], y));
-            }
-            row[36 + j] = fmaf(y, silu(z), cc.Dj * x);    // out_j of this timestep
+            float ya, yb;
+            upk(y2, ya, yb);
+            row[36 + j] = fmaf(ya + yb, silu(z), cc.Dj * x);    // out_j of this timestep
+            v = vn; dt = dtn;
         }
         __syncwarp(hmask);
         if (j < cnt) {                                    // lane = timestep again: ctx = out_proj . out at the ORIGINAL index
@@ -319,7 +513,11 @@ __device__ void scan_phase3(const Item& it, const TensorDir* __restrict__ tds, c
     if (it.last) {
         float* dst = tds[it.td].h + j * 16;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) reinterpret_cast<float4*>(dst)[q] = make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+        for (int q = 0; q < 4; ++q) {
+            float4 t;
+            upk(he[q], t.x, t.z); upk(ho[q], t.y, t.w);
+            reinterpret_cast<float4*>(dst)[q] = t;
+        }
     }
 }
 
@@ -332,13 +530,14 @@ __device__ void scan_phase3(const Item& it, const TensorDir* __restrict__ tds, c
 template <int DIR>
 __device__ void scan_phase1(const Item& it, const float2* __restrict__ gs, float* __restrict__ agg, float* __restrict__ tile,
                             int item_idx, int j, unsigned hmask) {
-    ColConst<DIR> cc;
+    ColPacked<DIR> cc;
     cc.load(j);
-    float b[16], m[32];
+    f2 be[4], bo[4], m[4][4];                            // per group of two pairs: b (even, odd) and the 2x2 product a b / c d
 #pragma unroll
-    for (int s = 0; s < 16; ++s) b[s] = 0.f;
-#pragma unroll
-    for (int p = 0; p < 8; ++p) { m[4 * p] = 1.f; m[4 * p + 1] = 0.f; m[4 * p + 2] = 0.f; m[4 * p + 3] = 1.f; }
+    for (int q = 0; q < 4; ++q) {
+        be[q] = bo[q] = m[q][1] = m[q][2] = pk(0.f, 0.f);
+        m[q][0] = m[q][3] = pk(1.f, 1.f);
+    }
     const int len = it.ue - it.ub;
     const int ntile = (len + TILE_T - 1) / TILE_T;
     for (int tI = ntile - 1; tI >= 0; --tI) {
@@ -346,55 +545,57 @@ __device__ void scan_phase1(const Item& it, const float2* __restrict__ gs, float
         const int cnt = (it.ue - u0 < TILE_T) ? (it.ue - u0) : TILE_T;
         stage_a<DIR>(tile, gs, it.off, it.n, u0 + j, j < cnt, j);
         __syncwarp(hmask);
+#pragma unroll 1
         for (int l = cnt - 1; l >= 0; --l) {
             const float* row = tile + l * ROW;
             const float2 v = *reinterpret_cast<const float2*>(row + 32);
             const float x = fmaf(cc.ux[0], v.x, fmaf(cc.ux[1], v.y, cc.ux[2]));
             const float dt = softplus20(fmaf(cc.ud[0], v.x, fmaf(cc.ud[1], v.y, cc.ud[2])));
-            float B[16];
+            const float ndtc = -fminf(dt, DT_CAP), dtx = dt * x;
+            const f2 ndt2 = pk(ndtc, ndtc), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const float4 t = reinterpret_cast<const float4*>(row)[q];
-                B[4 * q] = t.x; B[4 * q + 1] = t.y; B[4 * q + 2] = t.z; B[4 * q + 3] = t.w;
-            }
-            const float dtx = dt * x;
-#pragma unroll
-            for (int p = 0; p < 8; ++p) {
-                float abe, abo, cs, sn;
-                pair_coeffs(dt, cc.ah[2 * p], cc.ah[2 * p + 1], cc.f[p], abe, abo, cs, sn);
-                const float a0 = m[4 * p], b0 = m[4 * p + 1], c0 = m[4 * p + 2], d0 = m[4 * p + 3];
-                const float be = dtx * B[2 * p], bo = dtx * B[2 * p + 1];
-                b[2 * p]     = fmaf(a0, be, fmaf(b0, bo, b[2 * p]));
-                b[2 * p + 1] = fmaf(c0, be, fmaf(d0, bo, b[2 * p + 1]));
-                const float p1 = abe * cs, p2 = abe * sn, p3 = abo * sn, p4 = abo * cs;   // M_t = [[p1,-p2],[p3,p4]]
-                m[4 * p]     = fmaf(a0, p1, b0 * p3);
-                m[4 * p + 1] = fmaf(b0, p4, -a0 * p2);
-                m[4 * p + 2] = fmaf(c0, p1, d0 * p3);
-                m[4 * p + 3] = fmaf(d0, p4, -c0 * p2);
+                const ulonglong2 B = reinterpret_cast<const ulonglong2*>(row)[q];
+                f2 abe, abo, cs, sn;
+                quad_coeffs(ndt2, dt2, cc.ahe[q], cc.aho[q], cc.f[q], abe, abo, cs, sn);
+                const f2 a0 = m[q][0], b0 = m[q][1], c0 = m[q][2], d0 = m[q][3];
+                const f2 ie = mul2(dtx2, B.x), io = mul2(dtx2, B.y);
+                be[q] = fma2(a0, ie, fma2(b0, io, be[q]));
+                bo[q] = fma2(c0, ie, fma2(d0, io, bo[q]));
+                const f2 p1 = mul2(abe, cs), np2 = mul2(abe, mul2(sn, mone)), p3 = mul2(abo, sn), p4 = mul2(abo, cs);   // M_t = [[p1, np2], [p3, p4]]
+                m[q][0] = fma2(a0, p1, mul2(b0, p3));
+                m[q][1] = fma2(b0, p4, mul2(a0, np2));
+                m[q][2] = fma2(c0, p1, mul2(d0, p3));
+                m[q][3] = fma2(d0, p4, mul2(c0, np2));
             }
         }
         bool zero = true;
 #pragma unroll
-        for (int k = 0; k < 32; ++k) zero = zero && (fabsf(m[k]) < 3.5527e-15f);   // 2^-48
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float lo, hi;
+                upk(m[q][k], lo, hi);
+                zero = zero && (fabsf(lo) < 3.5527e-15f) && (fabsf(hi) < 3.5527e-15f);   // 2^-48
+            }
         __syncwarp(hmask);
         if (__all_sync(hmask, zero)) break;
     }
     float* dst = agg + ((int64_t)item_idx * 16 + j) * 48;      // [pair][a b c d e o]
 #pragma unroll
-    for (int p = 0; p < 8; ++p) {
-        dst[6 * p] = m[4 * p]; dst[6 * p + 1] = m[4 * p + 1]; dst[6 * p + 2] = m[4 * p + 2]; dst[6 * p + 3] = m[4 * p + 3];
-        dst[6 * p + 4] = b[2 * p]; dst[6 * p + 5] = b[2 * p + 1];
-    }
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            float lo, hi;
+            upk(k < 4 ? m[q][k] : k == 4 ? be[q] : bo[q], lo, hi);
+            dst[12 * q + k] = lo; dst[12 * q + 6 + k] = hi;
+        }
 }
 
 // items [0, n_items0) are direction 0, [n_items0_padded, ...) direction 1; n_items0_padded is a multiple of 8,
 // so one CTA (8 items) never mixes directions.
-template <int PHASE>
-__global__ void __launch_bounds__(SCAN_THREADS, SG_SCAN_MINB) sg2_scan_kernel(const Item* __restrict__ items, int n_items, int dir1_start,
-                                                                   const TensorDir* __restrict__ tds, const float2* __restrict__ gs,
-                                                                   const uint32_t* __restrict__ vals_sorted, float* __restrict__ agg,
-                                                                   const float* __restrict__ carry, float* __restrict__ ctx,
-                                                                   const int* __restrict__ status) {
+__global__ void __launch_bounds__(SCAN_THREADS, 3) sg2_scan1_kernel(const Item* __restrict__ items, int n_items, int dir1_start,
+                                                                    const float2* __restrict__ gs, float* __restrict__ agg, const int* __restrict__ status) {
     __shared__ __align__(16) float tiles[ITEMS_PER_CTA][TILE_T * ROW];
     if (status && (*status & 0xff) != STATUS_OK) return;              // a wait on a peer timed out earlier in this step: the persistent scan states stay
     const int slot = threadIdx.x >> 4, j = threadIdx.x & 15;
@@ -403,14 +604,46 @@ __global__ void __launch_bounds__(SCAN_THREADS, SG_SCAN_MINB) sg2_scan_kernel(co
     if (item_idx >= n_items) return;
     const Item it = items[item_idx];
     if (it.tensor < 0) return;
-    if (PHASE == 1 && it.last) return;            // nobody consumes the aggregate of a last chunk
-    if (PHASE == 1) {
-        if (item_idx < dir1_start) scan_phase1<0>(it, gs, agg, tiles[slot], item_idx, j, hmask);
-        else                       scan_phase1<1>(it, gs, agg, tiles[slot], item_idx, j, hmask);
-    } else {
-        if (item_idx < dir1_start) scan_phase3<0>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], item_idx, j, hmask);
-        else                       scan_phase3<1>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], item_idx, j, hmask);
+    if (it.last) return;                          // nobody consumes the aggregate of a last chunk
+    if (item_idx < dir1_start) scan_phase1<0>(it, gs, agg, tiles[slot], item_idx, j, hmask);
+    else                       scan_phase1<1>(it, gs, agg, tiles[slot], item_idx, j, hmask);
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS, COL_MINB) sg2_scan3_col_kernel(const Item* __restrict__ items, int n_items, int dir1_start,
+                                                                   const TensorDir* __restrict__ tds, const float2* __restrict__ gs,
+                                                                   const uint32_t* __restrict__ vals_sorted, const float* __restrict__ carry,
+                                                                   float* __restrict__ ctx, const int* __restrict__ status) {
+    __shared__ __align__(16) float tiles[ITEMS_PER_CTA][TILE_T * ROW];
+    if (status && (*status & 0xff) != STATUS_OK) return;              // a wait on a peer timed out earlier in this step: the persistent scan states stay
+    const int slot = threadIdx.x >> 4, j = threadIdx.x & 15;
+    const int item_idx = blockIdx.x * ITEMS_PER_CTA + slot;
+    const unsigned hmask = 0xffffu << (16 * ((threadIdx.x >> 4) & 1));
+    if (item_idx >= n_items) return;
+    const Item it = items[item_idx];
+    if (it.tensor < 0) return;
+    if (item_idx < dir1_start) scan_phase3_col<0>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], item_idx, j, hmask);
+    else                       scan_phase3_col<1>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], item_idx, j, hmask);
+}
+
+__global__ void __launch_bounds__(SCAN3_THREADS, WARP_MINB) sg2_scan3_kernel(const Item* __restrict__ items, int n_items, int dir1_start,
+                                                                   const TensorDir* __restrict__ tds, const float2* __restrict__ gs,
+                                                                   const uint32_t* __restrict__ vals_sorted, const float* __restrict__ carry,
+                                                                   float* __restrict__ ctx, const int* __restrict__ status) {
+    __shared__ __align__(16) float tiles[ITEMS3][SM3];
+    __shared__ __align__(16) float ucols[16][12];                     // affine tables of x, z, dt per column (a CTA never mixes directions)
+    if (status && (*status & 0xff) != STATUS_OK) return;              // a wait on a peer timed out earlier in this step: the persistent scan states stay
+    for (int i = threadIdx.x; i < 144; i += SCAN3_THREADS) {
+        const int col = i / 9, k = i % 9, tab = k < 3 ? P::A_X : k < 6 ? P::A_Z : P::A_DT;
+        ucols[col][k] = c_w[((int)blockIdx.x * ITEMS3 < dir1_start ? P::AFF0 : P::AFF1) + tab + 3 * col + k % 3];
     }
+    __syncthreads();
+    const int slot = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int item_idx = blockIdx.x * ITEMS3 + slot;
+    if (item_idx >= n_items) return;
+    const Item it = items[item_idx];
+    if (it.tensor < 0) return;
+    if (item_idx < dir1_start) scan_phase3<0>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], ucols[lane & 15], item_idx, lane);
+    else                       scan_phase3<1>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], ucols[lane & 15], item_idx, lane);
 }
 
 // Phase 2: carry-in of every chunk.  One CTA of 128 threads (column j, pair p) per (tensor, direction).  The recurrence over the
@@ -664,6 +897,10 @@ void sg2_gather(const uint32_t* vals_sorted, const float* g_packed, const float*
                                                                        reinterpret_cast<float2*>(gs_sorted), total);
 }
 
+// Up to this many items every one has a warp (and its share of registers) at once, and the chain of a single chunk is what takes the time:
+// the warp-per-item form of phase 3 runs it faster.  Beyond, throughput counts and the column form wins.
+constexpr int SCAN_WARP_ITEMS = 148 * WARP_MINB * ITEMS3;
+
 void sg2_scan(const void* items_dev, int n_items, int dir1_start, const void* tds_dev, int n_td, bool any_multi,
               const float* gs_sorted, const uint32_t* vals_sorted, float* agg, float* carry, float* ctx, const int* status, cudaStream_t s) {
     if (n_items <= 0) return;
@@ -672,12 +909,13 @@ void sg2_scan(const void* items_dev, int n_items, int dir1_start, const void* td
     const TensorDir* tds = reinterpret_cast<const TensorDir*>(tds_dev);
     const float2* gs = reinterpret_cast<const float2*>(gs_sorted);
     count_launch(any_multi ? 3 : 2);
-    if (any_multi) sg2_scan_kernel<1><<<blocks, SCAN_THREADS, 0, s>>>(items, n_items, dir1_start, tds, gs, vals_sorted, agg, carry, ctx, status);
+    if (any_multi) sg2_scan1_kernel<<<blocks, SCAN_THREADS, 0, s>>>(items, n_items, dir1_start, gs, agg, status);
     sg2_carry_kernel<<<n_td, 128, 0, s>>>(tds, agg, carry);
-    sg2_scan_kernel<3><<<blocks, SCAN_THREADS, 0, s>>>(items, n_items, dir1_start, tds, gs, vals_sorted, agg, carry, ctx, status);
+    if (n_items <= SCAN_WARP_ITEMS) sg2_scan3_kernel<<<(n_items + ITEMS3 - 1) / ITEMS3, SCAN3_THREADS, 0, s>>>(items, n_items, dir1_start, tds, gs, vals_sorted, carry, ctx, status);
+    else sg2_scan3_col_kernel<<<blocks, SCAN_THREADS, 0, s>>>(items, n_items, dir1_start, tds, gs, vals_sorted, carry, ctx, status);
 }
 
-int sg2_scan_ctas_per_sm() { return SG_SCAN_MINB; }
+int sg2_scan_resident_items() { return COL_MINB * ITEMS_PER_CTA; }
 
 void sg2_elem(int dtype, const MTArgs& a, float beta2, float eps, float rescale, const float* dyn, const float* w_global, const int* status,
               const float* g_packed, const float* s_packed, const float* ctx, int* expert_counts, int n_peers, void* local_base,

@@ -19,17 +19,25 @@ import torch
 from .. import _build
 from . import oracle
 
-# Scan items that are resident at once: 148 SMs x the CTAs per SM the kernel is compiled for (three; 26.6 KB shared memory each) x 8 items per CTA.  All chunks
-# take about the same time, so the items should fill WHOLE waves of that many: one item too many starts a second wave that costs as
-# much as the first.  One wave for small steps (longer chunks: the per-chunk aggregate pass of phase 1 costs a fixed ~300 timesteps
-# per chunk), two for large ones.
+# Scan items that are resident at once: 148 SMs x the items an SM holds (column form of phase 3: four CTAs of eight).  All chunks take about
+# the same time, so the items should fill WHOLE waves of that many: one item too many starts a second wave that costs as much as the
+# first.  One wave for small steps (longer chunks: the per-chunk aggregate pass of phase 1 costs a fixed ~300 timesteps per chunk), two
+# for large ones (18.9 M parameters, scan phases together: two waves 5.82 ms, three 5.82, one and a partial one 6.43 to 7.5).
 _MIN_CHUNK = 512
 
 
 def _wave_items() -> int:
     C = _build.load()
-    ctas = C.sg2_scan_ctas_per_sm() if C is not None and hasattr(C, "sg2_scan_ctas_per_sm") else 4
-    return 148 * ctas * 8
+    return 148 * (C.sg2_scan_resident_items() if C is not None and hasattr(C, "sg2_scan_resident_items") else 32)
+
+
+def _chunk_len(numels: Sequence[int]) -> int:
+    """Chunk length of a plan.  Steps that do not fill the GPU with 512-step chunks are bound by the chain of one chunk (phase 3) and a
+    serial pass over the chunks (carry): about 1,000 items balance the two (50 k parameters: 104 us at 128 steps, 167 at 512, 107 at 64)."""
+    total2 = 2 * sum(numels)
+    if total2 < 1000 * _MIN_CHUNK:
+        return max(128, -(-total2 // 16000) * 16)
+    return _pick_chunk_len(numels)
 
 
 def _pick_chunk_len(numels: Sequence[int]) -> int:
@@ -42,6 +50,7 @@ def _pick_chunk_len(numels: Sequence[int]) -> int:
     while 2 * sum(max(1, -(-n // L)) for n in numels) > cap and L < (1 << 30):      # partial last chunks of the tensors must fit as well
         L += 16
     return L
+
 
 _FALLBACK_LAYOUT = None
 
@@ -163,7 +172,7 @@ class Plan:
         if max(self.numels) >= 2 ** 31 or self.total >= 2 ** 32:
             raise ValueError("a v2 step handles < 2^31 elements per tensor and < 2^32 in total per call")
         if chunk_len <= 0:
-            chunk_len = _pick_chunk_len(self.numels)
+            chunk_len = _chunk_len(self.numels)
         chunk_len = -(-chunk_len // 16) * 16
         self.chunk_len = chunk_len
         items, tds = [], []
