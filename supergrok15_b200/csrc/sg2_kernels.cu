@@ -48,14 +48,15 @@ __device__ __forceinline__ float sigmoidf(float x) { return 1.f / (1.f + __expf(
 template <typename T, bool PACKED>
 __global__ void __launch_bounds__(MT_THREADS) sg2_prep_kernel(const __grid_constant__ MTArgs a, const float* __restrict__ tclip,
                                                               float* g_packed, float* __restrict__ s_packed,
-                                                              uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+                                                              uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, int sub_shift) {
     int lo = 0, hi = a.n;
-    const int b = blockIdx.x;
+    const int b = blockIdx.x >> sub_shift;
     while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (a.blk_start[mid] <= b) lo = mid; else hi = mid; }
     const int t = lo;
-    const int64_t begin = (int64_t)(b - a.blk_start[t]) * MT_CHUNK;
+    const int part = MT_CHUNK >> sub_shift;
+    const int64_t begin = (int64_t)(b - a.blk_start[t]) * MT_CHUNK + (int64_t)(blockIdx.x & ((1 << sub_shift) - 1)) * part;
     const int64_t n = a.numel[t];
-    const int64_t end = (begin + MT_CHUNK < n) ? begin + MT_CHUNK : n;
+    const int64_t end = (begin + part < n) ? begin + part : n;
     const int64_t off = (int64_t)reinterpret_cast<intptr_t>(a.ptr[6][t]);
     const T* g = reinterpret_cast<const T*>(a.ptr[1][t]);
     const float* sh = reinterpret_cast<const float*>(a.ptr[2][t]);
@@ -692,33 +693,39 @@ struct ElemParams {
     int* expert_counts;                // [144] or nullptr
     // optional replication of the updated parameter into the same offset of peer buffers (fused all-gather):
     // a parameter at local address local_base + d is also stored to peer_base[r] + d for r < n_peers
-    int n_peers; int n_inline; char* local_base; char* peer_base[8];
+    int n_peers; int n_inline; int sub_shift; char* local_base; char* peer_base[8];
 };
 
 // roles: 0 = param (launch dtype), 1 = m, 2 = v, 3 = mu, 4 = gru [n,4], 5 = fp32 master (optional), 6 = packed offset.
 // Step scalars come from the device table prm.dyn (layout: DYN_* in sg_native.h).
 template <typename T>
 __global__ void __launch_bounds__(MT_THREADS) sg2_elem_kernel(const __grid_constant__ MTArgs a, const __grid_constant__ ElemParams prm) {
-    // Expert rows are padded to 17 floats: lanes pick different experts, and with a row pitch of 16 the word k of every expert
-    // falls into one of only two banks (16-way conflicts); with 17 the rows of 32 consecutive experts spread over all banks.
-    constexpr int EP = SG2_EH + 1;
+    // Expert rows: per four hidden units W1[4] b1[4] W2[4], so a head reads its expert with twelve 16-byte loads; 52 floats (13 float4,
+    // odd) per row spread the rows that the lanes pick over all banks.  Bound by instruction issue (75 % of the slots); single-word loads
+    // cost 144 more instructions per element: 18.9 M parameters 2.05 -> 1.80 ms together with the finer parts below.
+    constexpr int EP = 52;
     if (prm.status && (*prm.status & 0xff) != STATUS_OK) return;      // gradients of a timed-out step are incomplete: keep every state as it is
-    __shared__ float sW1[SG2_NE * EP], sB1[SG2_NE * EP], sW2[SG2_NE * EP], sB2[SG2_NE];
+    // A CTA takes 1 / (1 << sub_shift) of a chunk: small steps have too few chunks to fill the GPU (422,755 parameters: 52 full chunks,
+    // 178 us in chunks, 50 us in sixteenths), large ones a nearly empty last wave.
+    const int b = blockIdx.x >> prm.sub_shift;
+    int lo = 0, hi = a.n;
+    while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (a.blk_start[mid] <= b) lo = mid; else hi = mid; }
+    const int t = lo;
+    const int part = MT_CHUNK >> prm.sub_shift;
+    const int64_t begin = (int64_t)(b - a.blk_start[t]) * MT_CHUNK + (int64_t)(blockIdx.x & ((1 << prm.sub_shift) - 1)) * part;
+    const int64_t n = a.numel[t];
+    const int64_t end = (begin + part < n) ? begin + part : n;
+    if (begin >= end) return;
+    __shared__ __align__(16) float sE[SG2_NE * EP];
+    __shared__ float sB2[SG2_NE];
     __shared__ int scount[SG2_NE];
     for (int i = threadIdx.x; i < SG2_NE * SG2_EH; i += MT_THREADS) {
-        const int j = (i / SG2_EH) * EP + i % SG2_EH;
+        const int k = i % SG2_EH, j = (i / SG2_EH) * EP + (k >> 2) * 12 + (k & 3);
         // lanes read consecutive words: from global memory that is one coalesced request, from __constant__ memory 32 serial ones
-        sW1[j] = prm.w_global[P::EW1 + i]; sB1[j] = prm.w_global[P::EB1 + i]; sW2[j] = prm.w_global[P::EW2 + i];
+        sE[j] = prm.w_global[P::EW1 + i]; sE[j + 4] = prm.w_global[P::EB1 + i]; sE[j + 8] = prm.w_global[P::EW2 + i];
     }
     for (int i = threadIdx.x; i < SG2_NE; i += MT_THREADS) { sB2[i] = prm.w_global[P::EB2 + i]; scount[i] = 0; }
     __syncthreads();
-    int lo = 0, hi = a.n;
-    const int b = blockIdx.x;
-    while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (a.blk_start[mid] <= b) lo = mid; else hi = mid; }
-    const int t = lo;
-    const int64_t begin = (int64_t)(b - a.blk_start[t]) * MT_CHUNK;
-    const int64_t n = a.numel[t];
-    const int64_t end = (begin + MT_CHUNK < n) ? begin + MT_CHUNK : n;
     const int64_t off = (int64_t)reinterpret_cast<intptr_t>(a.ptr[6][t]);
     T* param = reinterpret_cast<T*>(a.ptr[0][t]);
     float* M = reinterpret_cast<float*>(a.ptr[1][t]);
@@ -796,7 +803,14 @@ __global__ void __launch_bounds__(MT_THREADS) sg2_elem_kernel(const __grid_const
             if (prm.expert_counts) atomicAdd(&scount[e], 1);
             float ho = sB2[e];
 #pragma unroll
-            for (int k = 0; k < SG2_EH; ++k) ho = fmaf(sW2[e * EP + k], fmaxf(fmaf(sW1[e * EP + k], g, sB1[e * EP + k]), 0.f), ho);
+            for (int k = 0; k < SG2_EH / 4; ++k) {
+                const float4* row = reinterpret_cast<const float4*>(sE + e * EP + 12 * k);
+                const float4 w1 = row[0], b1 = row[1], w2 = row[2];
+                ho = fmaf(w2.x, fmaxf(fmaf(w1.x, g, b1.x), 0.f), ho);
+                ho = fmaf(w2.y, fmaxf(fmaf(w1.y, g, b1.y), 0.f), ho);
+                ho = fmaf(w2.z, fmaxf(fmaf(w1.z, g, b1.z), 0.f), ho);
+                ho = fmaf(w2.w, fmaxf(fmaf(w1.w, g, b1.w), 0.f), ho);
+            }
             total += ho;
         }
         const float smart = g + prm.rescale * total * (1.f / SG2_HEADS);
@@ -847,6 +861,9 @@ void sg2_upload_weights(const float* packed_dev, cudaStream_t s) {
     cudaMemcpyToSymbolAsync(c_w, packed_dev, sizeof(float) * SG2Pack::TOTAL, 0, cudaMemcpyDeviceToDevice, s);
 }
 
+// Parts per chunk of MT_CHUNK elements: 4, and 16 (one or two elements per thread) while the chunks do not give every SM its resident CTAs.
+static int sub_shift_for(int blocks, int ctas_per_sm) { return blocks < 148 * ctas_per_sm ? 4 : 2; }
+
 void sg2_sqnorm(int dtype, const MTArgs& a, float* partials, cudaStream_t s) {
     const int blocks = a.blk_start[a.n];
     if (blocks <= 0) return;
@@ -863,11 +880,13 @@ void sg2_prep(int dtype, bool packed_src, const MTArgs& a, const float* tclip, f
     const int blocks = a.blk_start[a.n];
     if (blocks <= 0) return;
     count_launch();
-    if (packed_src) { sg2_prep_kernel<float, true><<<blocks, MT_THREADS, 0, s>>>(a, tclip, g_packed, s_packed, keys, vals); return; }
+    const int sub = sub_shift_for(blocks, 8);
+    const unsigned grid = (unsigned)blocks << sub;
+    if (packed_src) { sg2_prep_kernel<float, true><<<grid, MT_THREADS, 0, s>>>(a, tclip, g_packed, s_packed, keys, vals, sub); return; }
     switch (dtype) {
-        case F32:  sg2_prep_kernel<float, false><<<blocks, MT_THREADS, 0, s>>>(a, tclip, g_packed, s_packed, keys, vals); break;
-        case BF16: sg2_prep_kernel<__nv_bfloat16, false><<<blocks, MT_THREADS, 0, s>>>(a, tclip, g_packed, s_packed, keys, vals); break;
-        default:   sg2_prep_kernel<__half, false><<<blocks, MT_THREADS, 0, s>>>(a, tclip, g_packed, s_packed, keys, vals); break;
+        case F32:  sg2_prep_kernel<float, false><<<grid, MT_THREADS, 0, s>>>(a, tclip, g_packed, s_packed, keys, vals, sub); break;
+        case BF16: sg2_prep_kernel<__nv_bfloat16, false><<<grid, MT_THREADS, 0, s>>>(a, tclip, g_packed, s_packed, keys, vals, sub); break;
+        default:   sg2_prep_kernel<__half, false><<<grid, MT_THREADS, 0, s>>>(a, tclip, g_packed, s_packed, keys, vals, sub); break;
     }
 }
 
@@ -928,10 +947,12 @@ void sg2_elem(int dtype, const MTArgs& a, float beta2, float eps, float rescale,
     p.g_packed = g_packed; p.s_packed = s_packed; p.ctx = ctx; p.expert_counts = expert_counts;
     p.n_peers = n_peers; p.n_inline = 0; p.local_base = reinterpret_cast<char*>(local_base);
     for (int r = 0; r < n_peers && r < 8; ++r) p.peer_base[r] = reinterpret_cast<char*>(peer_base[r]);
+    p.sub_shift = sub_shift_for(blocks, 3);
+    const unsigned grid = (unsigned)blocks << p.sub_shift;
     switch (dtype) {
-        case F32:  sg2_elem_kernel<float><<<blocks, MT_THREADS, 0, s>>>(a, p); break;
-        case BF16: sg2_elem_kernel<__nv_bfloat16><<<blocks, MT_THREADS, 0, s>>>(a, p); break;
-        default:   sg2_elem_kernel<__half><<<blocks, MT_THREADS, 0, s>>>(a, p); break;
+        case F32:  sg2_elem_kernel<float><<<grid, MT_THREADS, 0, s>>>(a, p); break;
+        case BF16: sg2_elem_kernel<__nv_bfloat16><<<grid, MT_THREADS, 0, s>>>(a, p); break;
+        default:   sg2_elem_kernel<__half><<<grid, MT_THREADS, 0, s>>>(a, p); break;
     }
 }
 
