@@ -1,0 +1,65 @@
+"""Row widths, row counts and alignments at which the norm and short-attention kernels change their form."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from supergrok15_b200.ops import nn_ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _close(a, b, dtype, sums=False):
+    # fp32: sums of up to 3072 products; 16 bits: one rounding of the result and one of the stored sum x + r (2^-9 each, times a few
+    # units); parameter gradients add up to 40,000 rows before their one rounding
+    rel = float((a.double() - b).norm() / b.norm())
+    assert rel < (3e-6 if dtype == torch.float32 else 1e-2 if sums else 5e-3), rel
+
+
+# one vector, a partial warp, whole warps, a partial last warp of a row, the most warps per row; too few rows for the four-row form,
+# enough, and a remainder; widths of half a vector (the general kernel)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,D", [(1, 8), (3, 64), (5, 264), (17, 768), (2369, 2048), (40001, 72), (9475, 256), (4739, 520), (131, 3072), (2400, 1544), (33, 132), (1190, 3000)])
+@pytest.mark.parametrize("rms,res", [(False, True), (False, False), (True, True)])
+def test_norm_matches_fp64(rows, D, rms, res, dtype):
+    g = torch.Generator(device="cuda").manual_seed(rows + D)
+    x, r, dy, dzo = (torch.randn(rows, D, generator=g, device="cuda").to(dtype) for _ in range(4))
+    w, b = ((1 + torch.randn(D, generator=g, device="cuda") * 0.1).to(dtype) for _ in range(2))
+    leaves = [t.requires_grad_() for t in ([x, r, w] if rms else [x, r, w, b] if res else [x, w, b])]
+    ref = [t.detach().double().requires_grad_() for t in leaves]
+    if rms:
+        y, z = nn_ops.norm_residual(x, r, w, None, 1e-5, rms=True)
+        got = torch.autograd.grad((y, z), leaves, (dy, dzo))
+        zr = ref[0] + ref[1]
+        if dtype != torch.float32:
+            zr = zr + (z.detach().double() - zr.detach())               # the stored (rounded) sum is what the norm sees
+        yr = zr * torch.rsqrt(zr.square().mean(-1, keepdim=True) + 1e-5) * ref[2]
+        want = torch.autograd.grad((yr, zr), ref, (dy.double(), dzo.double()))
+    else:
+        y = nn_ops.layer_norm(x, r if res else None, w, b)
+        got = torch.autograd.grad(y, leaves, dy)
+        zr = ref[0] + ref[1] if res else ref[0]
+        if dtype != torch.float32 and res:
+            zr = zr + ((x.detach() + r.detach()).double() - zr.detach())
+        yr = F.layer_norm(zr, (D,), ref[-2], ref[-1], 1e-5)
+        want = torch.autograd.grad(yr, ref, dy.double())
+    _close(y.detach(), yr.detach(), dtype)
+    for k, (a, c) in enumerate(zip(got, want)):
+        _close(a, c, dtype, sums=a.dim() == 1)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("B,S,H,hd,off", [(1, 4, 1, 64, 0), (37, 4, 3, 64, 0), (129, 4, 5, 32, 0), (11, 8, 3, 64, 0), (33, 8, 1, 32, 0), (7, 4, 3, 64, 2), (5, 8, 3, 32, 2)])
+def test_short_attention_matches_fp64(B, S, H, hd, off, causal, dtype):
+    """``off``: the input starts that many elements into a buffer, which breaks the 16-byte alignment that the wide loads need."""
+    g = torch.Generator(device="cuda").manual_seed(B + S)
+    n = B * S * 3 * H * hd
+    qkv = torch.randn(n + off, generator=g, device="cuda").to(dtype)[off:].view(B, S, 3 * H * hd).requires_grad_()
+    do = torch.randn(B, S, H * hd, generator=g, device="cuda").to(dtype)
+    o = nn_ops.attention_small(qkv, H, causal)
+    (got,) = torch.autograd.grad(o, qkv, do)
+    ref = qkv.detach().double().requires_grad_()
+    orf = nn_ops.attention_small_reference(ref, H, causal)
+    (want,) = torch.autograd.grad(orf, ref, do.double())
+    _close(o.detach(), orf.detach(), dtype)
+    _close(got, want, dtype)
