@@ -4,6 +4,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include "bindings_decl.h"
 #include "mt_host.h"
+#include "sg2_meta.h"
 #include "sg2_routing_math.h"
 #include "sg2_gru_math.h"
 
@@ -191,6 +192,55 @@ void sg2_scan_backward(Tensor items, int64_t n_items, int64_t dir1_start, Tensor
                           W("gs").data_ptr<float>(), vs, dctx.data_ptr<float>(), W("carry").data_ptr<float>(), W("agg").data_ptr<float>(),
                           W("dcarry").data_ptr<float>(), snaps.data_ptr<float>(), partial.data_ptr<float>(), grads.data_ptr<float>(),
                           (int)snap_every, at::cuda::getCurrentCUDAStream());
+}
+
+// Packed meta-network weights (sg_native.h: SG2Pack) from its 42 parameter tensors, folded tables included
+Tensor sg2_pack(const TL& tensors, int64_t expert_hidden) {
+    TORCH_CHECK((int)tensors.size() == sg::SG2_META_TENSORS && expert_hidden >= 1 && expert_hidden <= sg::SG2_EH, "42 meta-network tensors expected");
+    const float* src[sg::SG2_META_TENSORS];
+    for (int k = 0; k < sg::SG2_META_TENSORS; ++k) {
+        const Tensor& t = tensors[k];
+        TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.device() == tensors[0].device() &&
+                    t.numel() == sg::sg2_pack_numel(k, (int)expert_hidden), "meta-network tensor ", k, ": contiguous fp32 CUDA tensor of ",
+                    sg::sg2_pack_numel(k, (int)expert_hidden), " elements");
+        src[k] = t.data_ptr<float>();
+    }
+    c10::cuda::CUDAGuard guard(tensors[0].device());
+    Tensor out = at::empty({sg::SG2Pack::TOTAL}, tensors[0].options().requires_grad(false));
+    sg::sg2_pack(src, (int)expert_hidden, out.data_ptr<float>(), at::cuda::getCurrentCUDAStream());
+    return out;
+}
+
+// grads [2 * ng] of the scan adjoint -> gradients of input_proj and of both directions' parameters, in the packed layout
+Tensor sg2_fold_backward(Tensor packed, Tensor grads, int64_t ng) {
+    TORCH_CHECK(packed.is_cuda() && packed.scalar_type() == at::kFloat && packed.is_contiguous() && packed.numel() == sg::SG2Pack::TOTAL, "packed weights expected");
+    TORCH_CHECK(grads.device() == packed.device() && grads.scalar_type() == at::kFloat && grads.is_contiguous() && ng >= 768 && grads.numel() >= 2 * ng, "grads: fp32 [2, ng]");
+    c10::cuda::CUDAGuard guard(packed.device());
+    Tensor out = at::empty({sg::SG2Pack::GRU_WZ}, packed.options());
+    sg::sg2_fold_bwd(packed.data_ptr<float>(), grads.data_ptr<float>(), (int)ng, out.data_ptr<float>(), at::cuda::getCurrentCUDAStream());
+    return out;
+}
+
+// Every tensor divided by its 2-norm, packed at `offsets`; a tensor with a non-finite entry becomes zeros, one of norm <= 1e-12 stays
+Tensor sg2_unit_vectors(const TL& vs, const std::vector<int64_t>& offsets, int64_t total) {
+    TORCH_CHECK(!vs.empty() && vs.size() == offsets.size(), "one offset per tensor");
+    const int dt = dtype_code(vs[0]);
+    int64_t blocks = 0;
+    for (size_t i = 0; i < vs.size(); ++i) {
+        TORCH_CHECK(dtype_code(vs[i]) == dt && vs[i].device() == vs[0].device() && offsets[i] >= 0 && offsets[i] + vs[i].numel() <= total,
+                    "unit vectors: tensors of one dtype and device inside the packed length");
+        blocks += (vs[i].numel() + sg::MT_CHUNK - 1) / sg::MT_CHUNK;
+    }
+    c10::cuda::CUDAGuard guard(vs[0].device());
+    cudaStream_t st = at::cuda::getCurrentCUDAStream();
+    auto f32 = vs[0].options().dtype(at::kFloat).requires_grad(false);
+    Tensor out = at::empty({total}, f32), partials = at::empty({3 * std::max<int64_t>(blocks, 1)}, f32), tot = at::empty({3 * (int64_t)vs.size()}, f32);
+    for_each_launch({{}, vs}, {}, &offsets, [&](sg::MTArgs& a) {
+        sg::sg2_unit_norm(dt, a, partials.data_ptr<float>(), st);
+        sg::mt_finalize_per_tensor(a, partials.data_ptr<float>(), tot.data_ptr<float>(), st);
+        sg::sg2_unit_write(dt, a, tot.data_ptr<float>(), out.data_ptr<float>(), st);
+    });
+    return out;
 }
 
 void sg2_upload_weights(Tensor packed) {
@@ -466,6 +516,9 @@ void register_sg2(pybind11::module_& m) {
     m.def("sg2_upload_weights", &sg2_upload_weights);
     m.def("sg2_sort", &sg2_sort);
     m.def("sg2_layout", &sg2_layout);
+    m.def("sg2_pack", &sg2_pack);
+    m.def("sg2_fold_backward", &sg2_fold_backward);
+    m.def("sg2_unit_vectors", &sg2_unit_vectors);
     m.def("sg2_scan_resident_items", []() { return sg::sg2_scan_resident_items(); });
     m.def("sg2_recycle", &sg2_recycle_b, py::arg("counts"), py::arg("W1"), py::arg("b1"), py::arg("W2"), py::arg("b2"), py::arg("keys_a"),
           py::arg("keys_b"), py::arg("threshold"), py::arg("seed"), py::arg("call"), py::arg("info"));

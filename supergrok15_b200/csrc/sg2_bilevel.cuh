@@ -15,7 +15,7 @@
 //
 // Because x, z, dt, B and C are affine in (g, s) (SG2Pack::AFF* tables), their weight gradients are gradients of the
 // TABLES:  dU[j][k] += d value_j[t] * (g_t, s_t, 1)[k].  The chain rule from the tables to input_proj / in_proj / dt_proj /
-// B_proj / C_proj is a handful of tiny matrix products done by autograd on the host.  This formulation contains the
+// B_proj / C_proj is a handful of tiny matrix products (sg2_meta.cu: sg2_fold_bwd_kernel).  This formulation contains the
 // cross-column terms exactly (every column's dependence on B_s and C_s goes through the shared tables).
 // Per direction the kernel produces NG = 138 + 128 gradient values:
 //   [0,256)    d A_log [16][16]          [256,384)  d rope_freq [16][8]      [384,400)  d D [16]

@@ -98,12 +98,27 @@ def supports_native(meta_net) -> bool:
             meta_net.expert_hidden <= 16)
 
 
+def scan_leaves(mn) -> List[torch.Tensor]:
+    """Parameters that the scan's inputs and outputs depend on, in ``SG2Pack`` order: input_proj, then nine tensors per direction."""
+    out = [mn.input_proj.weight, mn.input_proj.bias]
+    for b in (mn.mamba_fwd, mn.mamba_bwd):
+        out += [b.in_proj.weight, b.dt_proj.weight, b.dt_proj.bias, b.B_proj.weight, b.C_proj.weight, b.A_log, b.D, b.rope_freq, b.out_proj.weight]
+    return out
+
+
 @torch.no_grad()
 def pack_metanet(meta_net) -> torch.Tensor:
-    """Meta-net weights as one fp32 vector in ``SG2Pack`` order (experts zero-padded to 16 hidden units)."""
+    """Meta-net weights as one fp32 vector in ``SG2Pack`` order (experts zero-padded to 16 hidden units).  On CUDA one kernel copies
+    and folds everything (``csrc/sg2_meta.cu``); the statement below is what it computes."""
     if not supports_native(meta_net):
         raise ValueError("the fused v2 kernels support d_model 8, d_state 16, expand 2, gru 4, 4 heads, 144 experts, "
                          "expert_hidden <= 16")
+    if meta_net.input_proj.weight.is_cuda:
+        g = meta_net.gru
+        ts = scan_leaves(meta_net) + [g.W_z.weight, g.W_r.weight, g.W_h.weight, g.W_z.bias, g.W_r.bias, g.W_h.bias]
+        ts += [q.weight for q in meta_net.peer_queries] + list(meta_net.product_keys_A) + list(meta_net.product_keys_B)
+        ts += [meta_net.expert_W1, meta_net.expert_b1, meta_net.expert_W2, meta_net.expert_b2]
+        return _build.require().sg2_pack([t.detach().float().contiguous() for t in ts], meta_net.expert_hidden)
     L = layout()
     dev = meta_net.input_proj.weight.device
     out = torch.zeros(L["TOTAL"], dtype=torch.float32, device=dev)

@@ -4,7 +4,7 @@ All parameter tensors are processed in ONE batched call: sort -> gather -> forwa
 copies of the persistent states) -> contexts ``ctx [total, 16]``.  The part after the scan (GRU, soft top-4 product-key
 routing, experts) is element-wise and runs through autograd in slices, producing d(meta_loss)/d ctx.  The scan adjoint
 kernels turn that into gradients of A_log, rope_freq, D, out_proj and of the folded affine tables; autograd through
-``scan_params`` (a few 16x16 matrix products) carries the table gradients to input_proj / in_proj / dt_proj / B_proj / C_proj.
+one small kernel (``csrc/sg2_meta.cu``) carries the table gradients to input_proj / in_proj / dt_proj / B_proj / C_proj.
 The result equals autograd of ``Mamba3PEERMetaNet.forward_for_bilevel`` (tested), including the cross-column terms that
 the reference kernel drops.
 
@@ -114,25 +114,13 @@ def gru(x, h, W, b):
     return _Gru.apply(x, h, W, b)
 
 
-def scan_params(meta_net) -> List[torch.Tensor]:
-    """Differentiable tensors the adjoint kernel reports gradients for, per direction:
-    A_log [16,16], rope [16,8], D [16], U_x, U_z, U_dt, U_B, U_C [16,3] each, out_proj [8,16]."""
-    Wi, bi = meta_net.input_proj.weight.double(), meta_net.input_proj.bias.double()
-    inp = torch.cat([Wi, bi.unsqueeze(1)], 1)                                   # [8,3]
-    out = []
-    for blk in (meta_net.mamba_fwd, meta_net.mamba_bwd):
-        xz = blk.in_proj.weight.double() @ inp
-        x_t, z_t = xz[:16], xz[16:]
-        dt_t = blk.dt_proj.weight.double() @ x_t
-        dt_t = torch.cat([dt_t[:, :2], (dt_t[:, 2] + blk.dt_proj.bias.double()).unsqueeze(1)], 1)
-        b_t = blk.B_proj.weight.double() @ x_t
-        c_t = blk.C_proj.weight.double() @ x_t
-        out += [blk.A_log, blk.rope_freq, blk.D, x_t, z_t, dt_t, b_t, c_t, blk.out_proj.weight]
-    return out
-
-
-_SLICES = [(0, 256, (16, 16)), (256, 384, (16, 8)), (384, 400, (16,)), (400, 448, (16, 3)), (448, 496, (16, 3)), (496, 544, (16, 3)),
-           (544, 592, (16, 3)), (592, 640, (16, 3)), (640, 768, (8, 16))]
+# (offset, shape) of the scan's parameters in the packed layout, in the order of ``ops/sg2.py: scan_leaves``
+def _leaf_views(flat: torch.Tensor, leaves) -> List[torch.Tensor]:
+    L = sg2_ops.layout()
+    offs = [L["IN_W"], L["IN_B"]]
+    for base in (L["DIR0"], L["DIR1"]):
+        offs += [base + L[k] for k in ("D_INPROJ", "D_DTW", "D_DTB", "D_BW", "D_CW", "D_ALOG", "D_D", "D_ROPE", "D_OUT")]
+    return [flat[o:o + t.numel()].view(t.shape) for o, t in zip(offs, leaves)]
 
 
 class _Workspace:
@@ -161,17 +149,16 @@ class _Workspace:
 
 
 class _ScanCtx(torch.autograd.Function):
+    """Contexts of every element; differentiable with respect to ``leaves`` (fp32, ``ops/sg2.py: scan_leaves``), whose packed copy is ``w``."""
+
     @staticmethod
-    def forward(ctx, wsp, grads_list, sharps, fwd_states, bwd_states, *params):
+    def forward(ctx, wsp, w, grads_list, sharps, fwd_states, bwd_states, *leaves):
         C = _build.require()
         p = wsp.plan
-        for dst, src in zip(wsp.h_fwd, fwd_states):
-            dst.copy_(src)
-        for dst, src in zip(wsp.h_bwd, bwd_states):
-            dst.copy_(src)
+        torch._foreach_copy_(wsp.h_fwd + wsp.h_bwd, list(fwd_states) + list(bwd_states))
         buf = C.sg2_prepare(grads_list, sharps, p.offsets[:-1], p.total, p.seg_off, 1e30, p.ws)      # no clipping: raw gradients
         C.sg2_scan(p.items, p.n_items, p.dir1_start, p.tds, p.n_td, p.any_multi, buf, p.ws)
-        ctx.wsp, ctx.buf = wsp, buf
+        ctx.wsp, ctx.buf, ctx.w, ctx.leaves = wsp, buf, w, leaves
         return p.ws["ctx"][: 16 * p.total].view(p.total, 16).clone()
 
     @staticmethod
@@ -180,13 +167,8 @@ class _ScanCtx(torch.autograd.Function):
         wsp, p = ctx.wsp, ctx.wsp.plan
         C.sg2_scan_backward(p.items, p.n_items, p.dir1_start, p.tds, p.n_td, wsp.snap_base, ctx.buf, dctx.contiguous().float(), p.ws,
                             wsp.snaps, wsp.partial, wsp.grads, snap_every=wsp.snap_every)
-        g = wsp.grads.view(2, wsp.ng)
-        outs = []
-        for d in range(2):
-            for a, b, shape in _SLICES:
-                t = g[d, a:b].reshape(shape).clone()
-                outs.append(t.double() if shape == (16, 3) else t)
-        return (None, None, None, None, None, *outs)
+        flat = C.sg2_fold_backward(ctx.w, wsp.grads, wsp.ng)          # a tensor of this call: its views may become the parameters' .grad
+        return (None, None, None, None, None, None, *_leaf_views(flat, ctx.leaves))
 
 
 def snapshot_tiles(checkpoint_interval: int) -> int:
@@ -216,18 +198,10 @@ def bilevel_backward_cuda(opt, named, train_grads: Dict[str, torch.Tensor], val_
         i = opt._param_to_idx.get(id(p))
         if i is None:
             continue
-        vg = val_grads[name].detach().reshape(-1).float()
-        sel.append((i, train_grads[name].detach().reshape(-1).float().contiguous(), vg))
+        sel.append((i, train_grads[name].detach().reshape(-1).float().contiguous(), val_grads[name].detach().reshape(-1).contiguous()))
     if not sel:
         return 0
     dev = sel[0][1].device
-    # tensors with non-finite validation gradients are skipped (decided on the device, applied as a zero weight)
-    vus = []
-    for _, _, vg in sel:
-        ok = torch.isfinite(vg).all()
-        n = torch.where(torch.isfinite(vg), vg, torch.zeros_like(vg)).norm()
-        vus.append(torch.where(ok & (n > 1e-12), 1.0 / n.clamp_min(1e-30), torch.where(ok, torch.ones_like(n), torch.zeros_like(n)))
-                   * torch.where(torch.isfinite(vg), vg, torch.zeros_like(vg)))
     numels = tuple(g.numel() for _, g, _ in sel)
     g_snap = snapshot_tiles(checkpoint_interval)
     key = (numels, str(dev), g_snap)
@@ -239,16 +213,20 @@ def bilevel_backward_cuda(opt, named, train_grads: Dict[str, torch.Tensor], val_
     C.sg2_upload_weights(w)
     sg2_ops._resident["owner"] = None                      # the optimizer step must re-upload its own copy afterwards
     idxs = [i for i, _, _ in sel]
-    params = scan_params(mn)
     with torch.enable_grad():
-        ctx_all = _ScanCtx.apply(wsp, [g for _, g, _ in sel], [opt._flat_sharpness[i] for i in idxs],
-                                 [opt._flat_mamba_fwd_states[i] for i in idxs], [opt._flat_mamba_bwd_states[i] for i in idxs], *params)
+        leaves = [t.float().contiguous() for t in sg2_ops.scan_leaves(mn)]
+        ctx_all = _ScanCtx.apply(wsp, w, [g for _, g, _ in sel], [opt._flat_sharpness[i] for i in idxs],
+                                 [opt._flat_mamba_fwd_states[i] for i in idxs], [opt._flat_mamba_bwd_states[i] for i in idxs], *leaves)
     p = wsp.plan
     g_all = p.ws["g"][: p.total]
     s_all = p.ws["s"][: p.total]
     gru_all = torch.cat([opt._flat_gru_states[i] for i in idxs], 0)
-    vu_all = torch.cat(vus)
-    dctx = torch.zeros(p.total, 16, device=dev)
+    # unit validation gradients; tensors with non-finite entries are skipped (decided on the device, applied as zeros)
+    vgs = [v for _, _, v in sel]
+    if any(v.dtype != vgs[0].dtype or v.dtype not in (torch.float32, torch.bfloat16, torch.float16) for v in vgs):
+        vgs = [v.float() for v in vgs]
+    vu_all = C.sg2_unit_vectors(vgs, p.offsets[:-1], p.total)
+    dctx = torch.empty(p.total, 16, device=dev)
     for a in range(0, p.total, slice_elems):                # element-wise tail of the meta-net, slice by slice
         b = min(p.total, a + slice_elems)
         c = ctx_all[a:b].detach().requires_grad_(True)

@@ -150,15 +150,17 @@ class SuperGrok2(SuperGrok15):
         (reference supergrok2.py:516-1330); tensors with non-finite validation gradients are skipped."""
         self._ensure_state()
         named = list(model.named_parameters())
-        saved = {n: p.grad.detach().clone() for n, p in named if p.grad is not None}
+        # the training gradients step aside (and come back as the same tensors) while the validation gradients take their place: no copies
+        saved = {n: p.grad for n, p in named if p.grad is not None}
         if not saved:
             return 0.0
         try:
-            model.zero_grad()
+            for _, p in named:
+                p.grad = None
             with torch.enable_grad():
                 val_loss = criterion(model(val_x), val_y)
                 val_loss.backward()
-            vgs = {n: p.grad.detach().clone() for n, p in named if p.grad is not None}
+            vgs = {n: p.grad.detach() for n, p in named if p.grad is not None}
             meta_optimizer.zero_grad()
             n_used = sg2_ops.bilevel_backward(self, named, saved, vgs, self.bilevel_checkpoint_interval)
             if n_used:
