@@ -1,0 +1,43 @@
+"""Which calls of ``nn_ops.linear`` take the column-sum bias gradient, and what they return."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from supergrok15_b200.ops import nn_ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape,out", [((4096, 64), 8), ((1025, 4, 40), 99), ((4097, 136), 520)])
+def test_gradients_match_fp64(shape, out, dtype):
+    g = torch.Generator(device="cuda").manual_seed(out)
+    x, w, b = (torch.randn(s, generator=g, device="cuda").to(dtype).requires_grad_() for s in (shape, (out, shape[-1]), (out,)))
+    dy = torch.randn(*shape[:-1], out, generator=g, device="cuda").to(dtype)
+    assert nn_ops._col_sum_bias(x, w, b)
+    y = nn_ops.linear(x, w, b)
+    got = torch.autograd.grad(y, (x, w, b), dy)
+    ref = [t.detach().double().requires_grad_() for t in (x, w, b)]
+    want = torch.autograd.grad(F.linear(*ref), ref, dy.double())
+    for a, c in zip(got, want):
+        # fp32 sums of 4,097 terms, one rounding to the 16-bit types (2^-9, 2^-12 relative)
+        assert a.shape == c.shape and float((a.double() - c).norm() / c.norm()) < (2e-5 if dtype == torch.float32 else 4e-3)
+
+
+def test_other_calls_stay_with_the_library():
+    x, w, b = (torch.randn(s, device="cuda", requires_grad=True) for s in ((4096, 16), (8, 16), (8,)))
+    assert nn_ops._col_sum_bias(x, w, b)
+    assert not nn_ops._col_sum_bias(x[:100], w, b) and not nn_ops._col_sum_bias(x, w, None) and not nn_ops._col_sum_bias(x, w, b.detach())
+    with torch.no_grad():
+        assert not nn_ops._col_sum_bias(x, w, b)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert nn_ops.linear(x, w, b).dtype == torch.bfloat16
+    per_sample = torch.func.vmap(lambda t: nn_ops.linear(t, w, b))(x.detach().view(2, 2048, 16))
+    assert torch.allclose(per_sample.view(4096, 8), F.linear(x, w, b), atol=1e-5)
+    _, jvp = torch.func.jvp(lambda t: nn_ops.linear(t, w, b), (x.detach(),), (torch.ones_like(x),))
+    assert torch.allclose(jvp, torch.ones_like(x) @ w.t(), atol=1e-5)
+    (gx,) = torch.autograd.grad(nn_ops.linear(x, w, b).square().sum(), x, create_graph=True)
+    got = torch.autograd.grad(gx.square().sum(), (w, b))
+    (gr,) = torch.autograd.grad(F.linear(x, w, b).square().sum(), x, create_graph=True)
+    for a, c in zip(got, torch.autograd.grad(gr.square().sum(), (w, b))):
+        assert torch.allclose(a, c, rtol=1e-4, atol=1e-3 * float(c.abs().max()))
