@@ -17,7 +17,7 @@ void sg2_pull_sqnorm(int dtype, const MTArgs& a, const PeerPtrs& bases, int worl
                      float* partials, cudaStream_t s);
 void sg2_gather(const uint32_t* vals_sorted, const float* g_packed, const float* s_packed, float* gs_sorted, int64_t total, cudaStream_t s);
 void sg2_scan(const void* items_dev, int n_items, int dir1_start, const void* tds_dev, int n_td, bool any_multi, const float* gs_sorted,
-              const uint32_t* vals_sorted, float* agg, float* carry, float* ctx, const int* status, cudaStream_t s);
+              const uint32_t* vals_sorted, float* agg, float* carry, float* ctx, const int* status, const ScanSnaps& snaps, cudaStream_t s);
 void sg2_elem(int dtype, const MTArgs& a, float beta2, float eps, float rescale, const float* dyn, const float* w_global, const int* status,
               const float* g_packed,
               const float* s_packed, const float* ctx, int* expert_counts, int n_peers, void* local_base, void* const* peer_base,
@@ -41,10 +41,11 @@ namespace sg {
 bool routed_experts_supported(int heads, int E, int hidden, int topk);
 int routed_experts_bwd_ctas(int64_t n, int heads);
 int routed_experts_fwd(const float* g, const int* ia, const int* ib, const float* wa, const float* wb, const float* W1, const float* b1,
-                       const float* W2, const float* b2, int64_t n, int heads, int E, int pk, float* total, cudaStream_t s);
+                       const float* W2, const float* b2, int64_t n, int heads, int E, int pk, float* table, float* total, cudaStream_t s);
+int routed_experts_table_floats(int E);
 int routed_experts_bwd(const float* g, const int* ia, const int* ib, const float* wa, const float* wb, const float* W1, const float* b1,
                        const float* W2, const float* b2, const float* dtotal, int64_t n, int heads, int E, int pk, float* dwa, float* dwb,
-                       float* partial, float* dparams, cudaStream_t s);
+                       float* table, float* partial, float* dparams, cudaStream_t s);
 }
 
 namespace sg {
@@ -129,14 +130,19 @@ const int* status_ptr(const c10::optional<Tensor>& st) {
     return st->data_ptr<int>();
 }
 
+// snaps / snap_base (bilevel): the state at the start of every snap_every-th 16-step tile of item i goes to snaps[snap_base[i] + k]
 void sg2_scan(Tensor items, int64_t n_items, int64_t dir1_start, Tensor tds, int64_t n_td, bool any_multi, int64_t sorted_buf, py::dict ws,
-              c10::optional<Tensor> status) {
+              c10::optional<Tensor> status, c10::optional<Tensor> snaps, c10::optional<Tensor> snap_base, int64_t snap_every) {
+    TORCH_CHECK(!snaps.has_value() || (snaps->is_cuda() && snaps->scalar_type() == at::kFloat && snap_base.has_value() && snap_base->is_cuda() &&
+                                       snap_base->scalar_type() == at::kLong && snap_base->numel() >= n_items), "snaps: fp32, snap_base: int64 per item");
     c10::cuda::CUDAGuard guard(items.device());
     cudaStream_t st = at::cuda::getCurrentCUDAStream();
     auto W = [&](const char* k) { return ws[k].cast<Tensor>(); };
     const uint32_t* vs = sorted_buf ? u32(W("vals1")) : u32(W("vals0"));
     sg::sg2_scan(items.data_ptr(), (int)n_items, (int)dir1_start, tds.data_ptr(), (int)n_td, any_multi, W("gs").data_ptr<float>(), vs,
-                 W("agg").data_ptr<float>(), W("carry").data_ptr<float>(), W("ctx").data_ptr<float>(), status_ptr(status), st);
+                 W("agg").data_ptr<float>(), W("carry").data_ptr<float>(), W("ctx").data_ptr<float>(), status_ptr(status),
+                 sg::ScanSnaps{snaps.has_value() ? snaps->data_ptr<float>() : nullptr, snaps.has_value() ? snap_base->data_ptr<int64_t>() : nullptr,
+                               (int)std::max<int64_t>(snap_every, 1)}, st);
 }
 
 // masters: empty, or one fp32 tensor per parameter.  peer_ptrs: base addresses of the peers' parameter buffers (same layout as
@@ -311,10 +317,10 @@ Tensor routed_experts_fwd(const Tensor& g, const Tensor& ia, const Tensor& ib, c
                           const Tensor& W2, const Tensor& b2, int64_t pk) {
     const XShape s = routed_check(g, ia, ib, wa, wb, W1, b1, W2, b2);
     c10::cuda::CUDAGuard guard(g.device());
-    Tensor total = at::empty({s.n}, g.options());
+    Tensor total = at::empty({s.n}, g.options()), table = at::empty({sg::routed_experts_table_floats(s.E)}, g.options());
     const int rc = sg::routed_experts_fwd(g.data_ptr<float>(), ia.data_ptr<int>(), ib.data_ptr<int>(), wa.data_ptr<float>(), wb.data_ptr<float>(),
                                           W1.data_ptr<float>(), b1.data_ptr<float>(), W2.data_ptr<float>(), b2.data_ptr<float>(), s.n, s.heads, s.E,
-                                          (int)pk, total.data_ptr<float>(), at::cuda::getCurrentCUDAStream());
+                                          (int)pk, table.data_ptr<float>(), total.data_ptr<float>(), at::cuda::getCurrentCUDAStream());
     TORCH_CHECK(rc == 0, "routed_experts_fwd launch failed (code ", rc, ")");
     return total;
 }
@@ -328,11 +334,11 @@ std::vector<Tensor> routed_experts_bwd(const Tensor& g, const Tensor& ia, const 
     const int64_t ng = 3 * (int64_t)s.E * s.hidden + s.E;
     Tensor dwa = at::empty_like(wa), dwb = at::empty_like(wb);
     Tensor partial = at::empty({(int64_t)sg::routed_experts_bwd_ctas(s.n, s.heads), ng}, g.options());
-    Tensor dparams = at::empty({ng}, g.options());
+    Tensor dparams = at::empty({ng}, g.options()), table = at::empty({sg::routed_experts_table_floats(s.E)}, g.options());
     const int rc = sg::routed_experts_bwd(g.data_ptr<float>(), ia.data_ptr<int>(), ib.data_ptr<int>(), wa.data_ptr<float>(), wb.data_ptr<float>(),
                                           W1.data_ptr<float>(), b1.data_ptr<float>(), W2.data_ptr<float>(), b2.data_ptr<float>(),
                                           dtotal.data_ptr<float>(), s.n, s.heads, s.E, (int)pk, dwa.data_ptr<float>(), dwb.data_ptr<float>(),
-                                          partial.data_ptr<float>(), dparams.data_ptr<float>(), at::cuda::getCurrentCUDAStream());
+                                          table.data_ptr<float>(), partial.data_ptr<float>(), dparams.data_ptr<float>(), at::cuda::getCurrentCUDAStream());
     TORCH_CHECK(rc == 0, "routed_experts_bwd launch failed (code ", rc, ")");
     return {dwa, dwb, dparams};
 }
@@ -508,7 +514,8 @@ void register_sg2(pybind11::module_& m) {
     m.attr("DYN_TS") = (int)sg::DYN_TS; m.attr("DYN_LR") = (int)sg::DYN_LR; m.attr("DYN_WD") = (int)sg::DYN_WD;
     m.attr("DYN_LAMB") = (int)sg::DYN_LAMB; m.attr("DYN_EPOCH") = (int)sg::DYN_EPOCH;
     m.def("sg2_scan", &sg2_scan, py::arg("items"), py::arg("n_items"), py::arg("dir1_start"), py::arg("tds"), py::arg("n_td"), py::arg("any_multi"),
-          py::arg("sorted_buf"), py::arg("ws"), py::arg("status") = c10::optional<Tensor>());
+          py::arg("sorted_buf"), py::arg("ws"), py::arg("status") = c10::optional<Tensor>(), py::arg("snaps") = c10::optional<Tensor>(),
+          py::arg("snap_base") = c10::optional<Tensor>(), py::arg("snap_every") = 1);
     m.def("sg2_elem", &sg2_elem, py::arg("params"), py::arg("ms"), py::arg("vs"), py::arg("mus"), py::arg("grus"), py::arg("masters"),
           py::arg("dyn"), py::arg("packed"), py::arg("offsets"), py::arg("beta2"), py::arg("eps"), py::arg("rescale"),
           py::arg("expert_counts"), py::arg("ws"), py::arg("local_base") = 0, py::arg("peer_ptrs") = std::vector<int64_t>(),

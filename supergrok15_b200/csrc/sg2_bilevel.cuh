@@ -8,8 +8,7 @@
 //   adj 1   per chunk: aggregate of the reverse recurrence  dh[t-1] = M_t^T (dh[t] + dy_t C_t)   (prefix product walked
 //           forwards from the chunk start, with the same 2^-100 early exit as the forward aggregates)
 //   adj 2   carry: dh arriving at the end of every chunk (chunks in reverse order; the last chunk receives zero)
-//   adj 3   per chunk: re-run the chunk forwards storing the state at every 16-step tile boundary (global scratch), then
-//           walk the tiles backwards: recompute the 16 states of the tile into shared memory, run the exact adjoint of
+//   adj 3   per chunk: walk the tiles backwards from the states that the forward scan has left at their boundaries (global scratch): recompute the 16 states of the tile into shared memory, run the exact adjoint of
 //           each timestep, accumulate parameter gradients privately per lane
 //   adj 4   fixed-order reduction of the per-item partial gradients
 //
@@ -27,7 +26,7 @@ namespace sg {
 namespace {
 
 constexpr int BL_TILE = 16;                    // timesteps per backward tile
-constexpr int BL_ITEMS = 4;                    // items per CTA (64 threads)
+constexpr int BL_ITEMS = 2;                    // items per CTA (one warp: 39.7 KB of shared memory, five CTAs per SM)
 constexpr int BL_THREADS = BL_ITEMS * 16;
 constexpr int BL_NG = 768;                     // gradient values per direction (layout above)
 constexpr int BL_LANE_ACC = 16 + 8 + 1 + 9 + 8;   // register-resident accumulators per lane: dah, df, dD, dUx/Uz/Udt, dWout column
@@ -150,24 +149,34 @@ __global__ void __launch_bounds__(128) sg2_adj2_kernel(const TensorDir* __restri
     }
 }
 
-// forward recurrence through the cnt timesteps of one tile whose rows stage_a has parked in `tile` (state only: no outputs)
+// forward recurrence through the cnt timesteps of one tile whose rows stage_a has parked in `tile` (state only: no outputs), in the
+// arithmetic of the forward scan (sg2_kernels.cu: scan_phase3): a state recomputed from a snapshot is bit for bit the one that
+// a snapshot at that place would have held
 template <int DIR>
 __device__ __forceinline__ void bl_advance_tile(const ColConst<DIR>& cc, const float* __restrict__ tile, int cnt, float (&h)[16]) {
+    f2 he[4], ho[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) { he[q] = pk(h[4 * q], h[4 * q + 2]); ho[q] = pk(h[4 * q + 1], h[4 * q + 3]); }
+#pragma unroll 1
     for (int l = 0; l < cnt; ++l) {
         const float* row = tile + l * ROW;
         const float2 v = *reinterpret_cast<const float2*>(row + 32);
         const float x = fmaf(cc.ux[0], v.x, fmaf(cc.ux[1], v.y, cc.ux[2]));
         const float dt = softplus20(fmaf(cc.ud[0], v.x, fmaf(cc.ud[1], v.y, cc.ud[2])));
-        const float dtx = dt * x;
+        const float ndtc = -fminf(dt, DT_CAP), dtx = dt * x;
+        const f2 ndt2 = pk(ndtc, ndtc), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
 #pragma unroll
-        for (int p = 0; p < 8; ++p) {
-            float abe, abo, cs, sn;
-            pair_coeffs(dt, cc.ah[2 * p], cc.ah[2 * p + 1], cc.f[p], abe, abo, cs, sn);
-            const float he = h[2 * p], ho = h[2 * p + 1];
-            h[2 * p] = fmaf(abe, he * cs - ho * sn, dtx * row[row_pos(2 * p)]);
-            h[2 * p + 1] = fmaf(abo, ho * cs + he * sn, dtx * row[row_pos(2 * p + 1)]);
+        for (int q = 0; q < 4; ++q) {
+            const ulonglong2 B = reinterpret_cast<const ulonglong2*>(row)[q];
+            f2 abe, abo, cs, sn;
+            quad_coeffs(ndt2, dt2, pk(cc.ah[4 * q], cc.ah[4 * q + 2]), pk(cc.ah[4 * q + 1], cc.ah[4 * q + 3]), pk(cc.f[2 * q], cc.f[2 * q + 1]), abe, abo, cs, sn);
+            const f2 re = fma2(ho[q], mul2(sn, mone), mul2(he[q], cs)), ro = fma2(he[q], sn, mul2(ho[q], cs));
+            he[q] = fma2(abe, re, mul2(dtx2, B.x));
+            ho[q] = fma2(abo, ro, mul2(dtx2, B.y));
         }
     }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) { upk(he[q], h[4 * q], h[4 * q + 2]); upk(ho[q], h[4 * q + 1], h[4 * q + 3]); }
 }
 
 // ---- adj 3: the adjoint proper ----
@@ -176,34 +185,14 @@ __device__ __forceinline__ void bl_advance_tile(const ColConst<DIR>& cc, const f
 // (snap_every - 1) / 2 extra tile passes on average for 1 / snap_every of the snapshot memory.  The gradients do not depend on it.
 template <int DIR>
 __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uint32_t* __restrict__ vals_sorted, const float* __restrict__ dctx,
-                        const float* __restrict__ carry, const float* __restrict__ dcarry, float* __restrict__ snaps, int64_t snap_base,
-                        float* __restrict__ partial, float* __restrict__ tile, float* __restrict__ hist, float* __restrict__ sacc,
+                        const float* __restrict__ dcarry, const float* __restrict__ snaps, int64_t snap_base,
+                        float* __restrict__ partial, float* __restrict__ tile, float* __restrict__ hist,
                         int item_idx, int j, unsigned hmask, int snap_every) {
     ColConst<DIR> cc;
     cc.load(j);
     const int len = it.ue - it.ub;
     const int ntile = (len + BL_TILE - 1) / BL_TILE;
     float h[16];
-    // ---- forward re-run of the chunk: state snapshot at every tile start
-    {
-        const float* cin = carry + ((int64_t)item_idx * 16 + j) * 16;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) { const float4 t = reinterpret_cast<const float4*>(cin)[q]; h[4 * q] = t.x; h[4 * q + 1] = t.y; h[4 * q + 2] = t.z; h[4 * q + 3] = t.w; }
-    }
-    for (int tI = 0; tI < ntile; ++tI) {
-        const int u0 = it.ub + tI * BL_TILE;
-        const int cnt = (it.ue - u0 < BL_TILE) ? (it.ue - u0) : BL_TILE;
-        if (tI % snap_every == 0) {
-            float* sp = snaps + ((snap_base + tI / snap_every) * 16 + j) * 16;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) reinterpret_cast<float4*>(sp)[q] = make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
-        }
-        if (tI == ntile - 1) break;                        // the last tile is recomputed by the backward loop anyway
-        stage_a<DIR>(tile, gs, it.off, it.n, u0 + j, j < cnt, j);      // rows of the forward layout (ROW floats)
-        __syncwarp(hmask);
-        bl_advance_tile<DIR>(cc, tile, cnt, h);
-        __syncwarp(hmask);
-    }
     // ---- backward over the tiles
     float dh[16], dah[16], df[8], dux[3] = {0.f, 0.f, 0.f}, duz[3] = {0.f, 0.f, 0.f}, dud[3] = {0.f, 0.f, 0.f}, dwo[8], dD = 0.f;
     {
@@ -215,9 +204,7 @@ __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uin
     for (int s = 0; s < 16; ++s) dah[s] = 0.f;
 #pragma unroll
     for (int p = 0; p < 8; ++p) { df[p] = 0.f; dwo[p] = 0.f; }
-    // lane-private accumulators of dU_B / dU_C in shared memory: sacc[a * BL_THREADS + tid], a in [0, 96)
-    float* my = sacc + threadIdx.x;
-    for (int a = 0; a < 96; ++a) my[a * BL_THREADS] = 0.f;
+    float dbc[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};     // dU rows 2 j and 2 j + 1 of the 32 rows (B 0..15, C 16..31), summed over the columns
     for (int tI = ntile - 1; tI >= 0; --tI) {
         const int u0 = it.ub + tI * BL_TILE;
         const int cnt = (it.ue - u0 < BL_TILE) ? (it.ue - u0) : BL_TILE;
@@ -266,7 +253,7 @@ __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uin
             const float gout = row[36 + j];
             const float sz = sigmoidf(z), sl = z * sz;
             const float dy = gout * sl;
-            float y = 0.f, ddt = 0.f, ddtx = 0.f;
+            float y = 0.f, ddt = 0.f, ddtx = 0.f, v32[32];
 #pragma unroll
             for (int p = 0; p < 8; ++p) {
                 const int e = 2 * p, o = 2 * p + 1;
@@ -278,14 +265,7 @@ __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uin
                 const float hce = fmaf(abe, re, dtx * Be), hco = fmaf(abo, ro, dtx * Bo);     // state AFTER this step
                 y = fmaf(hce, Ce, fmaf(hco, Co, y));
                 const float de = fmaf(dy, Ce, dh[e]), dd = fmaf(dy, Co, dh[o]);
-                const float dCe = dy * hce, dCo = dy * hco, dBe = de * dtx, dBo = dd * dtx;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    my[(e * 3 + k) * BL_THREADS] = fmaf(dBe, in3[k], my[(e * 3 + k) * BL_THREADS]);
-                    my[(o * 3 + k) * BL_THREADS] = fmaf(dBo, in3[k], my[(o * 3 + k) * BL_THREADS]);
-                    my[(48 + e * 3 + k) * BL_THREADS] = fmaf(dCe, in3[k], my[(48 + e * 3 + k) * BL_THREADS]);
-                    my[(48 + o * 3 + k) * BL_THREADS] = fmaf(dCo, in3[k], my[(48 + o * 3 + k) * BL_THREADS]);
-                }
+                v32[e] = de * dtx; v32[o] = dd * dtx; v32[16 + e] = dy * hce; v32[16 + o] = dy * hco;      // d B, d C of this column
                 ddtx = fmaf(de, Be, fmaf(dd, Bo, ddtx));
                 const float dabe = de * re, dabo = dd * ro, dre = de * abe, dro = dd * abo;
                 const float dcs = fmaf(dre, he, dro * ho), dsn = fmaf(dro, he, -dre * ho);
@@ -297,6 +277,21 @@ __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uin
                 dah[e] = fmaf(gae, dt, dah[e]); dah[o] = fmaf(gao, dt, dah[o]);
                 dh[e] = fmaf(dre, cs, dro * sn);
                 dh[o] = fmaf(dro, cs, -dre * sn);
+            }
+            {   // d B and d C are shared by the sixteen columns: halve the 32 values four times over the lanes, lane j ends with the sums of two
+                float r16[16], r8[8], r4[4];
+                const bool b3 = j & 8, b2 = j & 4, b1 = j & 2, b0 = j & 1;
+#pragma unroll
+                for (int k = 0; k < 16; ++k) r16[k] = (b3 ? v32[16 + k] : v32[k]) + __shfl_xor_sync(hmask, b3 ? v32[k] : v32[16 + k], 8);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) r8[k] = (b2 ? r16[8 + k] : r16[k]) + __shfl_xor_sync(hmask, b2 ? r16[k] : r16[8 + k], 4);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) r4[k] = (b1 ? r8[4 + k] : r8[k]) + __shfl_xor_sync(hmask, b1 ? r8[k] : r8[4 + k], 2);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    const float t = (b0 ? r4[2 + k] : r4[k]) + __shfl_xor_sync(hmask, b0 ? r4[k] : r4[2 + k], 1);
+                    dbc[k][0] = fmaf(t, in3[0], dbc[k][0]); dbc[k][1] = fmaf(t, in3[1], dbc[k][1]); dbc[k][2] += t;
+                }
             }
             const float outj = fmaf(y, sl, cc.Dj * x);
             const float dz = gout * y * sz * (1.f + z * (1.f - sz));
@@ -322,29 +317,21 @@ __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uin
     for (int k = 0; k < 3; ++k) { out[400 + j * 3 + k] = dux[k]; out[448 + j * 3 + k] = duz[k]; out[496 + j * 3 + k] = dud[k]; }
 #pragma unroll
     for (int d = 0; d < 8; ++d) out[640 + d * 16 + j] = dwo[d];
-    // dU_B / dU_C: sum over the 16 lanes of this item (fixed order), lane s writes row s
-    __syncwarp(hmask);
-    const int base = threadIdx.x & ~15;
-    for (int k = 0; k < 3; ++k) {
-        float sb = 0.f, sc = 0.f;
-        for (int jj = 0; jj < 16; ++jj) {
-            sb += sacc[(j * 3 + k) * BL_THREADS + base + jj];
-            sc += sacc[(48 + j * 3 + k) * BL_THREADS + base + jj];
-        }
-        out[544 + j * 3 + k] = sb;
-        out[592 + j * 3 + k] = sc;
-    }
+    // rows 2 j, 2 j + 1 of [dU_B | dU_C]
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) out[544 + (2 * j + k) * 3 + c] = dbc[k][c];
 }
 
 __global__ void __launch_bounds__(BL_THREADS) sg2_adj3_kernel(const Item* __restrict__ items, int n_items, int dir1_start,
                                                               const int64_t* __restrict__ snap_base, const float2* __restrict__ gs,
                                                               const uint32_t* __restrict__ vals_sorted, const float* __restrict__ dctx,
-                                                              const float* __restrict__ carry, const float* __restrict__ dcarry,
-                                                              float* __restrict__ snaps, float* __restrict__ partial, int snap_every) {
+                                                              const float* __restrict__ dcarry, const float* __restrict__ snaps,
+                                                              float* __restrict__ partial, int snap_every) {
     extern __shared__ __align__(16) float bl_smem[];
     float* tiles = bl_smem;                                             // [BL_ITEMS][BL_TILE*BL_ROW]  (BL_ROW >= ROW)
     float* hist = tiles + BL_ITEMS * BL_TILE * BL_ROW;                  // [BL_ITEMS][BL_TILE*16*16]
-    float* sacc = hist + BL_ITEMS * BL_TILE * 256;                      // [96][BL_THREADS]
     const int slot = threadIdx.x >> 4, j = threadIdx.x & 15;
     const int item_idx = blockIdx.x * BL_ITEMS + slot;
     const unsigned hmask = 0xffffu << (16 * ((threadIdx.x >> 4) & 1));
@@ -356,18 +343,15 @@ __global__ void __launch_bounds__(BL_THREADS) sg2_adj3_kernel(const Item* __rest
     }
     float* tile = tiles + slot * BL_TILE * BL_ROW;
     float* hs = hist + slot * BL_TILE * 256;
-    if (item_idx < dir1_start) bl_adj3<0>(it, gs, vals_sorted, dctx, carry, dcarry, snaps, snap_base[item_idx], partial, tile, hs, sacc, item_idx, j, hmask, snap_every);
-    else                       bl_adj3<1>(it, gs, vals_sorted, dctx, carry, dcarry, snaps, snap_base[item_idx], partial, tile, hs, sacc, item_idx, j, hmask, snap_every);
+    if (item_idx < dir1_start) bl_adj3<0>(it, gs, vals_sorted, dctx, dcarry, snaps, snap_base[item_idx], partial, tile, hs, item_idx, j, hmask, snap_every);
+    else                       bl_adj3<1>(it, gs, vals_sorted, dctx, dcarry, snaps, snap_base[item_idx], partial, tile, hs, item_idx, j, hmask, snap_every);
 }
 
 // ---- adj 4: fixed-order sum over the items of each direction; d(A/2) -> d A_log ----
-__global__ void __launch_bounds__(256) sg2_adj4_kernel(const float* __restrict__ partial, int n_items, int dir1_start, float* __restrict__ grads) {
-    const int dir = blockIdx.y;
-    const int k = blockIdx.x * 256 + threadIdx.x;
-    if (k >= BL_NG) return;
-    const int i0 = dir == 0 ? 0 : dir1_start, i1 = dir == 0 ? dir1_start : n_items;
-    float s = 0.f;
-    for (int i = i0; i < i1; ++i) s += partial[(int64_t)i * BL_NG + k];
+__global__ void __launch_bounds__(1024) sg2_adj4_kernel(const float* __restrict__ partial, int n_items, int dir1_start, float* __restrict__ grads) {
+    const int dir = blockIdx.y, k = blockIdx.x * 32 + (threadIdx.x & 31);
+    float s = column_parts_sum(partial, dir == 0 ? 0 : dir1_start, dir == 0 ? dir1_start : n_items, BL_NG, k);
+    if (threadIdx.x >= 32 || k >= BL_NG) return;
     if (k < 256) {                                                      // ah = -0.5*exp(A_log)  =>  d A_log = d ah * ah
         const int W = (dir == 0) ? P::DIR0 : P::DIR1;
         s *= -0.5f * __expf(c_w[W + P::D_ALOG + k]);
@@ -377,7 +361,7 @@ __global__ void __launch_bounds__(256) sg2_adj4_kernel(const float* __restrict__
 
 }  // namespace
 
-size_t sg2_bilevel_smem_bytes() { return (size_t)(BL_ITEMS * BL_TILE * BL_ROW + BL_ITEMS * BL_TILE * 256 + 96 * BL_THREADS) * sizeof(float); }
+size_t sg2_bilevel_smem_bytes() { return (size_t)(BL_ITEMS * BL_TILE * BL_ROW + BL_ITEMS * BL_TILE * 256) * sizeof(float); }
 int sg2_bilevel_ng() { return BL_NG; }
 int sg2_bilevel_tile() { return BL_TILE; }
 
@@ -399,8 +383,8 @@ void sg2_scan_backward(const void* items_dev, int n_items, int dir1_start, const
     count_launch(4);
     sg2_adj1_kernel<<<blocks, BL_THREADS, 0, s>>>(items, n_items, dir1_start, gs, vals_sorted, dctx, agg);
     sg2_adj2_kernel<<<n_td, 128, 0, s>>>(tds, agg, dcarry);
-    sg2_adj3_kernel<<<blocks, BL_THREADS, smem, s>>>(items, n_items, dir1_start, snap_base_dev, gs, vals_sorted, dctx, carry, dcarry, snaps, partial, snap_every);
-    sg2_adj4_kernel<<<dim3((BL_NG + 255) / 256, 2), 256, 0, s>>>(partial, n_items, dir1_start, grads);
+    sg2_adj3_kernel<<<blocks, BL_THREADS, smem, s>>>(items, n_items, dir1_start, snap_base_dev, gs, vals_sorted, dctx, dcarry, snaps, partial, snap_every);
+    sg2_adj4_kernel<<<dim3((BL_NG + 31) / 32, 2), 1024, 0, s>>>(partial, n_items, dir1_start, grads);
 }
 
 }  // namespace sg

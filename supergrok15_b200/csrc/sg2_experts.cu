@@ -12,6 +12,7 @@
 // order of additions is fixed), then every thread owns up to nine fixed (expert, hidden unit) pairs - their weights in
 // registers - and walks the tile's elements; per-CTA sums go to a partial buffer that a second kernel adds in CTA order.
 #include "sg_native.h"
+#include "column_parts.cuh"
 
 namespace sg {
 namespace {
@@ -20,43 +21,69 @@ constexpr int XH = 16;            // expert hidden width
 constexpr int XK = 4;             // keys kept per sub-key (top-4 x top-4 = 16 experts per head)
 constexpr int XTHREADS = 256;
 constexpr int XMAXQ = 9;          // (expert, hidden) pairs per thread in the backward pass: experts <= 16 * XMAXQ = 144
-constexpr int XPAD = XH + 1;      // shared-memory row pitch of the expert tables (different experts fall into different banks)
+constexpr int XSEG = XH + 1;      // linear pieces of an expert = row pitch of its tables (odd: different experts fall into different banks)
 
-struct XParams {                  // shared-memory copy of the expert tables
-    float* w1; float* b1; float* w2; float* b2;
-};
+// An expert is a piecewise linear function of the scalar g: hidden unit j switches at t_j = -b1_j / W1_j.  The tables hold the sorted
+// switching points and, per piece, slope and intercept (summed in fp64), so that a value takes five comparisons and one FMA instead of
+// 16 hidden units with three table words each; both forms were bound by the shared-memory reads (54 against 6 per value).
+// The indicator of a unit (for the parameter gradients) is still evaluated from its own weights: at a switching point the value does
+// not care on which side it is taken, a derivative would.
+struct XTable { const float* t; const float2* ab; };
+size_t __host__ __device__ constexpr x_table_floats(int E) { return (size_t)E * XSEG * 3 + ((E * XSEG) & 1); }      // t padded to a float2 boundary
 
-__device__ __forceinline__ XParams load_params(float* sm, const float* __restrict__ W1, const float* __restrict__ b1,
-                                               const float* __restrict__ W2, const float* __restrict__ b2, int E) {
-    XParams p{sm, sm + E * XPAD, sm + 2 * E * XPAD, sm + 3 * E * XPAD};
-    for (int i = threadIdx.x; i < E * XH; i += XTHREADS) {
-        const int e = i / XH, j = i % XH;
-        p.w1[e * XPAD + j] = W1[i];
-        p.b1[e * XPAD + j] = b1[i];
-        p.w2[e * XPAD + j] = W2[i];
+// sixteen lanes per expert: lane j ranks its switching point, lane s sums piece s (lane 0 also piece 16)
+__global__ void __launch_bounds__(128) experts_table_kernel(const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
+                                                            const float* __restrict__ b2, int E, float* __restrict__ table) {
+    const int e_raw = blockIdx.x * 8 + (threadIdx.x >> 4), j = threadIdx.x & 15;
+    const int e = e_raw < E ? e_raw : E - 1;                          // whole warps take part in the shuffles
+    const float w1 = W1[e * XH + j], b = b1[e * XH + j], w2 = W2[e * XH + j];
+    const float t = w1 != 0.f ? -b / w1 : INFINITY;
+    int rank = 0;
+    for (int k = 0; k < XH; ++k) {
+        const float tk = __shfl_sync(0xffffffffu, t, k, 16);
+        rank += (tk < t || (tk == t && k < j)) ? 1 : 0;
     }
-    for (int i = threadIdx.x; i < E; i += XTHREADS) p.b2[i] = b2[i];
-    return p;
+    float* th = table + (size_t)e * XSEG;
+    float2* ab = reinterpret_cast<float2*>(table + E * XSEG + ((E * XSEG) & 1)) + (size_t)e * XSEG;
+    if (e_raw < E) th[rank] = t;
+    const double base = (double)b2[e];
+    for (int rep = 0; rep < 2; ++rep) {
+        const int s = rep == 0 ? j : XH;                               // piece s: the s lowest switching points lie below g
+        double slope = 0.0, icept = base;
+        for (int k = 0; k < XH; ++k) {
+            const float kw1 = __shfl_sync(0xffffffffu, w1, k, 16), kb = __shfl_sync(0xffffffffu, b, k, 16), kw2 = __shfl_sync(0xffffffffu, w2, k, 16);
+            const int kr = __shfl_sync(0xffffffffu, rank, k, 16);
+            const bool on = kw1 > 0.f ? kr < s : kw1 < 0.f ? kr >= s : kb > 0.f;
+            if (on) { slope += (double)kw2 * kw1; icept += (double)kw2 * kb; }
+        }
+        if (e_raw < E && (rep == 0 || j == 0)) ab[s] = make_float2((float)slope, (float)icept);
+    }
 }
 
-__device__ __forceinline__ float expert_eval(const XParams& p, int e, float g) {
-    float o = p.b2[e];
-    const float* w1 = p.w1 + e * XPAD; const float* bb = p.b1 + e * XPAD; const float* w2 = p.w2 + e * XPAD;
-#pragma unroll
-    for (int j = 0; j < XH; ++j) o = fmaf(fmaxf(fmaf(g, w1[j], bb[j]), 0.f), w2[j], o);
-    return o;
+__device__ __forceinline__ XTable load_table(float* sm, const float* __restrict__ table, int E) {
+    for (int i = threadIdx.x; i < (int)x_table_floats(E); i += XTHREADS) sm[i] = table[i];
+    return XTable{sm, reinterpret_cast<const float2*>(sm + E * XSEG + ((E * XSEG) & 1))};
+}
+
+__device__ __forceinline__ float expert_eval(const XTable& p, int e, float g) {
+    const float* t = p.t + e * XSEG;
+    int s = g > t[7] ? 8 : 0;
+    s += g > t[s + 3] ? 4 : 0;
+    s += g > t[s + 1] ? 2 : 0;
+    s += g > t[s] ? 1 : 0;
+    s += g > t[s] ? 1 : 0;
+    const float2 ab = p.ab[e * XSEG + s];
+    return fmaf(ab.x, g, ab.y);
 }
 
 // one thread per (element, head); the heads of an element are added in head order by the thread of head 0
 __global__ void __launch_bounds__(XTHREADS) routed_experts_fwd_kernel(const float* __restrict__ g, const int4* __restrict__ ia,
                                                                       const int4* __restrict__ ib, const float4* __restrict__ wa,
-                                                                      const float4* __restrict__ wb, const float* __restrict__ W1,
-                                                                      const float* __restrict__ b1, const float* __restrict__ W2,
-                                                                      const float* __restrict__ b2, int64_t n, int heads, int E, int pk,
-                                                                      float* __restrict__ total) {
-    extern __shared__ float sm[];
-    const XParams p = load_params(sm, W1, b1, W2, b2, E);
-    float* s_tot = sm + 3 * E * XPAD + E;
+                                                                      const float4* __restrict__ wb, const float* __restrict__ table,
+                                                                      int64_t n, int heads, int E, int pk, float* __restrict__ total) {
+    extern __shared__ __align__(8) float sm[];
+    const XTable p = load_table(sm, table, E);
+    float* s_tot = sm + x_table_floats(E);
     __syncthreads();
     const int epc = XTHREADS / heads;                                   // elements per CTA
     const int le = threadIdx.x / heads, h = threadIdx.x % heads;
@@ -92,13 +119,13 @@ __global__ void __launch_bounds__(XTHREADS) routed_experts_bwd_kernel(const floa
                                                                       const int4* __restrict__ ib, const float4* __restrict__ wa,
                                                                       const float4* __restrict__ wb, const float* __restrict__ W1,
                                                                       const float* __restrict__ b1, const float* __restrict__ W2,
-                                                                      const float* __restrict__ b2, const float* __restrict__ dtotal,
+                                                                      const float* __restrict__ table, const float* __restrict__ dtotal,
                                                                       int64_t n, int heads, int E, int pk, float4* __restrict__ dwa,
                                                                       float4* __restrict__ dwb, float* __restrict__ partial) {
-    extern __shared__ float sm[];
-    const XParams p = load_params(sm, W1, b1, W2, b2, E);
+    extern __shared__ __align__(8) float sm[];
+    const XTable p = load_table(sm, table, E);
     const int epc = XTHREADS / heads;
-    float* s_g = sm + 3 * E * XPAD + E;                                 // [epc]
+    float* s_g = sm + x_table_floats(E);                                // [epc]
     float* s_route = s_g + XTHREADS;                                    // [epc][E]
     __syncthreads();
     const int le = threadIdx.x / heads, h = threadIdx.x % heads;
@@ -109,9 +136,9 @@ __global__ void __launch_bounds__(XTHREADS) routed_experts_bwd_kernel(const floa
     for (int q = 0; q < XMAXQ; ++q) {
         const int e = e0 + (XTHREADS / XH) * q;
         const bool in = e < E;
-        w1r[q] = in ? p.w1[e * XPAD + j] : 0.f;
-        b1r[q] = in ? p.b1[e * XPAD + j] : 0.f;
-        w2r[q] = in ? p.w2[e * XPAD + j] : 0.f;
+        w1r[q] = in ? W1[e * XH + j] : 0.f;
+        b1r[q] = in ? b1[e * XH + j] : 0.f;
+        w2r[q] = in ? W2[e * XH + j] : 0.f;
         aw1[q] = ab1[q] = aw2[q] = ab2[q] = 0.f;
     }
     const int64_t tiles = (n + epc - 1) / epc;
@@ -196,16 +223,8 @@ __global__ void __launch_bounds__(XTHREADS) routed_experts_bwd_kernel(const floa
     }
 }
 
-__global__ void __launch_bounds__(256) routed_experts_reduce_kernel(const float* __restrict__ partial, int parts, int ng, float* __restrict__ out) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= ng) return;
-    float t = 0.f;
-    for (int p = 0; p < parts; ++p) t += partial[(int64_t)p * ng + i];
-    out[i] = t;
-}
-
-size_t fwd_smem(int E) { return (size_t)(3 * E * XPAD + E + XTHREADS) * sizeof(float); }
-size_t bwd_smem(int E, int heads) { return (size_t)(3 * E * XPAD + E + XTHREADS + (XTHREADS / heads) * E) * sizeof(float); }
+size_t fwd_smem(int E) { return (size_t)(x_table_floats(E) + XTHREADS) * sizeof(float); }
+size_t bwd_smem(int E, int heads) { return (size_t)(x_table_floats(E) + XTHREADS + (XTHREADS / heads) * E) * sizeof(float); }
 
 }  // namespace
 
@@ -221,30 +240,35 @@ int routed_experts_bwd_ctas(int64_t n, int heads) {
     return (int)(tiles < cap ? (tiles < 1 ? 1 : tiles) : cap);
 }
 
+// floats of scratch for the value tables of E experts
+int routed_experts_table_floats(int E) { return (int)x_table_floats(E); }
+
 int routed_experts_fwd(const float* g, const int* ia, const int* ib, const float* wa, const float* wb, const float* W1, const float* b1,
-                       const float* W2, const float* b2, int64_t n, int heads, int E, int pk, float* total, cudaStream_t s) {
+                       const float* W2, const float* b2, int64_t n, int heads, int E, int pk, float* table, float* total, cudaStream_t s) {
     if (n <= 0) return 0;
     const size_t smem = fwd_smem(E);
     if (cudaFuncSetAttribute(routed_experts_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 2;
     const int epc = XTHREADS / heads;
-    count_launch();
+    count_launch(2);
+    experts_table_kernel<<<(E + 7) / 8, 128, 0, s>>>(W1, b1, W2, b2, E, table);
     routed_experts_fwd_kernel<<<(unsigned)((n + epc - 1) / epc), XTHREADS, smem, s>>>(
-        g, (const int4*)ia, (const int4*)ib, (const float4*)wa, (const float4*)wb, W1, b1, W2, b2, n, heads, E, pk, total);
+        g, (const int4*)ia, (const int4*)ib, (const float4*)wa, (const float4*)wb, table, n, heads, E, pk, total);
     return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
 int routed_experts_bwd(const float* g, const int* ia, const int* ib, const float* wa, const float* wb, const float* W1, const float* b1,
                        const float* W2, const float* b2, const float* dtotal, int64_t n, int heads, int E, int pk, float* dwa, float* dwb,
-                       float* partial, float* dparams, cudaStream_t s) {
+                       float* table, float* partial, float* dparams, cudaStream_t s) {
     const int ng = 3 * E * XH + E;
     if (n <= 0) return cudaMemsetAsync(dparams, 0, (size_t)ng * sizeof(float), s) == cudaSuccess ? 0 : 3;
     const size_t smem = bwd_smem(E, heads);
     if (cudaFuncSetAttribute(routed_experts_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 2;
     const int ctas = routed_experts_bwd_ctas(n, heads);
-    count_launch(2);
-    routed_experts_bwd_kernel<<<ctas, XTHREADS, smem, s>>>(g, (const int4*)ia, (const int4*)ib, (const float4*)wa, (const float4*)wb, W1, b1, W2, b2,
-                                                          dtotal, n, heads, E, pk, (float4*)dwa, (float4*)dwb, partial);
-    routed_experts_reduce_kernel<<<(ng + 255) / 256, 256, 0, s>>>(partial, ctas, ng, dparams);
+    count_launch(3);
+    experts_table_kernel<<<(E + 7) / 8, 128, 0, s>>>(W1, b1, W2, b2, E, table);
+    routed_experts_bwd_kernel<<<ctas, XTHREADS, smem, s>>>(g, (const int4*)ia, (const int4*)ib, (const float4*)wa, (const float4*)wb, W1, b1, W2,
+                                                          table, dtotal, n, heads, E, pk, (float4*)dwa, (float4*)dwb, partial);
+    column_parts_kernel<<<(ng + 31) / 32, 1024, 0, s>>>(partial, ctas, ng, dparams);
     return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 

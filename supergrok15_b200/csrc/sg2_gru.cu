@@ -4,6 +4,7 @@
 // order, sums stay in registers across tiles, one partial row per CTA, a second kernel adds the rows in CTA order (no atomics).
 #include "sg_native.h"
 #include "sg2_gru_math.h"
+#include "column_parts.cuh"
 
 namespace sg {
 namespace {
@@ -100,13 +101,6 @@ __global__ void __launch_bounds__(GT) gru_bwd_kernel(const float* __restrict__ x
     for (int u = 0; u < GMAXO; ++u) { const int id = threadIdx.x + u * GT; if (id < ng) out[id] = acc[u]; }
 }
 
-__global__ void __launch_bounds__(256) gru_reduce_kernel(const float* __restrict__ partial, int parts, int ng, float* __restrict__ out) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= ng) return;
-    float t = 0.f;
-    for (int p = 0; p < parts; ++p) t += partial[(int64_t)p * ng + i];
-    out[i] = t;
-}
 }  // namespace
 
 int gru_ng(int IN) { return 3 * gru::GH * (IN + gru::GH) + 3 * gru::GH; }
@@ -136,7 +130,7 @@ int gru_bwd(const float* x, const float* h, const float* W, const float* b, cons
     const int ctas = gru_bwd_ctas(n);
     count_launch(2);
     gru_bwd_kernel<0><<<ctas, GT, smem, s>>>(x, h, W, b, dhn, n, IN, dx, partial);
-    gru_reduce_kernel<<<(ng + 255) / 256, 256, 0, s>>>(partial, ctas, ng, dparams);
+    column_parts_kernel<<<(ng + 31) / 32, 1024, 0, s>>>(partial, ctas, ng, dparams);
     return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 

@@ -23,6 +23,7 @@
 #include "sg_native.h"
 #include "optim_math.cuh"
 #include "peer_fetch.cuh"
+#include "column_parts.cuh"
 
 namespace sg {
 
@@ -316,10 +317,10 @@ struct ColConst {
 constexpr int T3 = 32, R3 = 36;                         // tile rows: B[16] / out[16], C[16], (g, s, -, -): 9 float4, conflict free
 constexpr int PRE3 = 16 * 48;                            // dt[16] x[16] gate[16] of 16 timesteps
 constexpr int SM3 = T3 * R3 + PRE3;
-template <int DIR>
+template <int DIR, bool SNAP>
 __device__ void scan_phase3(const Item& it, const TensorDir* __restrict__ tds, const float2* __restrict__ gs,
                             const uint32_t* __restrict__ vals_sorted, const float* __restrict__ carry, float* __restrict__ ctx,
-                            float* __restrict__ tile, const float* __restrict__ ucol, int item_idx, int lane) {
+                            float* __restrict__ tile, const float* __restrict__ ucol, const ScanSnaps& sn, int item_idx, int lane) {
     constexpr int W = (DIR == 0) ? P::DIR0 : P::DIR1;
     constexpr int AF = (DIR == 0) ? P::AFF0 : P::AFF1;
     const int j = lane & 15, half = lane >> 4;
@@ -367,6 +368,14 @@ __device__ void scan_phase3(const Item& it, const TensorDir* __restrict__ tds, c
         __syncwarp();
 #pragma unroll 1
         for (int l0 = 0; l0 < cnt; l0 += 16) {
+            if constexpr (SNAP) {
+                const int tI = (u0 - it.ub + l0) >> 4;
+                if (tI % sn.every == 0) {
+                    float4* dst = reinterpret_cast<float4*>(sn.out + ((sn.base[item_idx] + tI / sn.every) * 16 + j) * 16 + 8 * half);
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) { float4 t; upk(he[q], t.x, t.z); upk(ho[q], t.y, t.w); dst[q] = t; }
+                }
+            }
             {   // lane = column, the halves take every other timestep
                 const float4 ua = reinterpret_cast<const float4*>(ucol)[0], ub = reinterpret_cast<const float4*>(ucol)[1];
                 const float uc = ucol[8];
@@ -443,10 +452,10 @@ __device__ void scan_phase3(const Item& it, const TensorDir* __restrict__ tds, c
 
 // PHASE 3, sixteen lanes per item (a lane carries a whole column, eight RoPE pairs): the form for steps with more chunks than the
 // warp-per-item form holds at once, where the column's own work (dt, x, gate, loads) should not be split over two lanes.
-template <int DIR>
+template <int DIR, bool SNAP>
 __device__ void scan_phase3_col(const Item& it, const TensorDir* __restrict__ tds, const float2* __restrict__ gs,
                             const uint32_t* __restrict__ vals_sorted, const float* __restrict__ carry, float* __restrict__ ctx,
-                            float* __restrict__ tile, int item_idx, int j, unsigned hmask) {
+                            float* __restrict__ tile, const ScanSnaps& sn, int item_idx, int j, unsigned hmask) {
     constexpr int W = (DIR == 0) ? P::DIR0 : P::DIR1;
     ColPacked<DIR> cc;
     cc.load(j);
@@ -457,6 +466,14 @@ __device__ void scan_phase3_col(const Item& it, const TensorDir* __restrict__ td
         for (int q = 0; q < 4; ++q) { const float4 t = reinterpret_cast<const float4*>(cin)[q]; he[q] = pk(t.x, t.z); ho[q] = pk(t.y, t.w); }
     }
     for (int u0 = it.ub; u0 < it.ue; u0 += TILE_T) {
+        if constexpr (SNAP) {
+            const int tI = (u0 - it.ub) / TILE_T;
+            if (tI % sn.every == 0) {
+                float4* dst = reinterpret_cast<float4*>(sn.out + ((sn.base[item_idx] + tI / sn.every) * 16 + j) * 16);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) { float4 t; upk(he[q], t.x, t.z); upk(ho[q], t.y, t.w); dst[q] = t; }
+            }
+        }
         const int cnt = (it.ue - u0 < TILE_T) ? (it.ue - u0) : TILE_T;
         stage_a<DIR>(tile, gs, it.off, it.n, u0 + j, j < cnt, j);
         __syncwarp(hmask);
@@ -610,10 +627,11 @@ __global__ void __launch_bounds__(SCAN_THREADS, 3) sg2_scan1_kernel(const Item* 
     else                       scan_phase1<1>(it, gs, agg, tiles[slot], item_idx, j, hmask);
 }
 
+template <bool SNAP>
 __global__ void __launch_bounds__(SCAN_THREADS, COL_MINB) sg2_scan3_col_kernel(const Item* __restrict__ items, int n_items, int dir1_start,
                                                                    const TensorDir* __restrict__ tds, const float2* __restrict__ gs,
                                                                    const uint32_t* __restrict__ vals_sorted, const float* __restrict__ carry,
-                                                                   float* __restrict__ ctx, const int* __restrict__ status) {
+                                                                   float* __restrict__ ctx, const int* __restrict__ status, ScanSnaps sn) {
     __shared__ __align__(16) float tiles[ITEMS_PER_CTA][TILE_T * ROW];
     if (status && (*status & 0xff) != STATUS_OK) return;              // a wait on a peer timed out earlier in this step: the persistent scan states stay
     const int slot = threadIdx.x >> 4, j = threadIdx.x & 15;
@@ -622,14 +640,15 @@ __global__ void __launch_bounds__(SCAN_THREADS, COL_MINB) sg2_scan3_col_kernel(c
     if (item_idx >= n_items) return;
     const Item it = items[item_idx];
     if (it.tensor < 0) return;
-    if (item_idx < dir1_start) scan_phase3_col<0>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], item_idx, j, hmask);
-    else                       scan_phase3_col<1>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], item_idx, j, hmask);
+    if (item_idx < dir1_start) scan_phase3_col<0, SNAP>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], sn, item_idx, j, hmask);
+    else                       scan_phase3_col<1, SNAP>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], sn, item_idx, j, hmask);
 }
 
+template <bool SNAP>
 __global__ void __launch_bounds__(SCAN3_THREADS, WARP_MINB) sg2_scan3_kernel(const Item* __restrict__ items, int n_items, int dir1_start,
                                                                    const TensorDir* __restrict__ tds, const float2* __restrict__ gs,
                                                                    const uint32_t* __restrict__ vals_sorted, const float* __restrict__ carry,
-                                                                   float* __restrict__ ctx, const int* __restrict__ status) {
+                                                                   float* __restrict__ ctx, const int* __restrict__ status, ScanSnaps sn) {
     __shared__ __align__(16) float tiles[ITEMS3][SM3];
     __shared__ __align__(16) float ucols[16][12];                     // affine tables of x, z, dt per column (a CTA never mixes directions)
     if (status && (*status & 0xff) != STATUS_OK) return;              // a wait on a peer timed out earlier in this step: the persistent scan states stay
@@ -643,8 +662,8 @@ __global__ void __launch_bounds__(SCAN3_THREADS, WARP_MINB) sg2_scan3_kernel(con
     if (item_idx >= n_items) return;
     const Item it = items[item_idx];
     if (it.tensor < 0) return;
-    if (item_idx < dir1_start) scan_phase3<0>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], ucols[lane & 15], item_idx, lane);
-    else                       scan_phase3<1>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], ucols[lane & 15], item_idx, lane);
+    if (item_idx < dir1_start) scan_phase3<0, SNAP>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], ucols[lane & 15], sn, item_idx, lane);
+    else                       scan_phase3<1, SNAP>(it, tds, gs, vals_sorted, carry, ctx, tiles[slot], ucols[lane & 15], sn, item_idx, lane);
 }
 
 // Phase 2: carry-in of every chunk.  One CTA of 128 threads (column j, pair p) per (tensor, direction).  The recurrence over the
@@ -921,7 +940,8 @@ void sg2_gather(const uint32_t* vals_sorted, const float* g_packed, const float*
 constexpr int SCAN_WARP_ITEMS = 148 * WARP_MINB * ITEMS3;
 
 void sg2_scan(const void* items_dev, int n_items, int dir1_start, const void* tds_dev, int n_td, bool any_multi,
-              const float* gs_sorted, const uint32_t* vals_sorted, float* agg, float* carry, float* ctx, const int* status, cudaStream_t s) {
+              const float* gs_sorted, const uint32_t* vals_sorted, float* agg, float* carry, float* ctx, const int* status, const ScanSnaps& snaps,
+              cudaStream_t s) {
     if (n_items <= 0) return;
     const int blocks = (n_items + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA;
     const Item* items = reinterpret_cast<const Item*>(items_dev);
@@ -930,8 +950,14 @@ void sg2_scan(const void* items_dev, int n_items, int dir1_start, const void* td
     count_launch(any_multi ? 3 : 2);
     if (any_multi) sg2_scan1_kernel<<<blocks, SCAN_THREADS, 0, s>>>(items, n_items, dir1_start, gs, agg, status);
     sg2_carry_kernel<<<n_td, 128, 0, s>>>(tds, agg, carry);
-    if (n_items <= SCAN_WARP_ITEMS) sg2_scan3_kernel<<<(n_items + ITEMS3 - 1) / ITEMS3, SCAN3_THREADS, 0, s>>>(items, n_items, dir1_start, tds, gs, vals_sorted, carry, ctx, status);
-    else sg2_scan3_col_kernel<<<blocks, SCAN_THREADS, 0, s>>>(items, n_items, dir1_start, tds, gs, vals_sorted, carry, ctx, status);
+    const int grid_w = (n_items + ITEMS3 - 1) / ITEMS3;
+    if (n_items <= SCAN_WARP_ITEMS) {
+        if (snaps.out) sg2_scan3_kernel<true><<<grid_w, SCAN3_THREADS, 0, s>>>(items, n_items, dir1_start, tds, gs, vals_sorted, carry, ctx, status, snaps);
+        else sg2_scan3_kernel<false><<<grid_w, SCAN3_THREADS, 0, s>>>(items, n_items, dir1_start, tds, gs, vals_sorted, carry, ctx, status, snaps);
+    } else {
+        if (snaps.out) sg2_scan3_col_kernel<true><<<blocks, SCAN_THREADS, 0, s>>>(items, n_items, dir1_start, tds, gs, vals_sorted, carry, ctx, status, snaps);
+        else sg2_scan3_col_kernel<false><<<blocks, SCAN_THREADS, 0, s>>>(items, n_items, dir1_start, tds, gs, vals_sorted, carry, ctx, status, snaps);
+    }
 }
 
 int sg2_scan_resident_items() { return COL_MINB * ITEMS_PER_CTA; }

@@ -9,6 +9,7 @@
 // autograd graph) of the PyTorch statement in optim/metanet.py: soft_head.
 #include "sg_native.h"
 #include "sg2_routing_math.h"
+#include "column_parts.cuh"
 
 namespace sg {
 namespace {
@@ -147,12 +148,154 @@ __global__ void __launch_bounds__(RT) routing_bwd_kernel(const float* __restrict
     for (int u = 0; u < RMAXK; ++u) { const int id = threadIdx.x + u * RT; if (id < 2 * n_k) out[n_wq + id] = acc_k[u]; }
 }
 
-__global__ void __launch_bounds__(256) routing_reduce_kernel(const float* __restrict__ partial, int parts, int ng, float* __restrict__ out) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= ng) return;
-    float t = 0.f;
-    for (int p = 0; p < parts; ++p) t += partial[(int64_t)p * ng + i];
-    out[i] = t;
+// The same for the default meta-net (4 heads, 22 inputs, 12 key rows), with the operands of every product in registers.  A thread of
+// (element, head) reads a row of Wq once, as six 16-byte loads, for both the query and d pin; the heads' d pin meet by shuffles.  The parameter
+// gradients are outer products summed over the tile: a warp takes every eighth element, a lane a 4 x 6 block of d Wq and a 3 x 4 block
+// of one key table (whose score gradients stand in a dense row of 12), so that five loads feed 36 FMAs; the eight warps are added in order
+// at the end.  Bound by instruction issue; 422,755 elements: 818 -> ROUTE_US us (two shared-memory loads per FMA before).
+namespace fixed {
+constexpr int H = 4, P = 22, PP = 24, PK = 12, TILE = RT / H;
+constexpr int WHEAD = 8 * PP + 4;                              // row pitch 24, heads 4 floats apart in the banks
+constexpr int QP = 36, SP = 100;                                // pitches of [32] query rows and [96] dense score gradients: odd in float4
+constexpr int N_WQ = H * 8 * P, N_K = H * PK * 4, NG = N_WQ + 2 * N_K;
+constexpr int F_W = 0, F_K = F_W + H * WHEAD, F_X = F_K + 2 * N_K, F_Q = F_X + TILE * PP, F_DQ = F_Q + TILE * QP, F_DS = F_DQ + TILE * QP,
+              FLOATS = F_DS + TILE * SP;
+static_assert(8 * NG <= FLOATS - F_X, "the warps' sums fit where the tile was");
+}  // namespace fixed
+
+__global__ void __launch_bounds__(RT, 2) routing_bwd_default_kernel(const float* __restrict__ pin, const float* __restrict__ Wq, const float* __restrict__ KA,
+                                                                    const float* __restrict__ KB, const int4* __restrict__ ia, const int4* __restrict__ ib,
+                                                                    const float4* __restrict__ wa, const float4* __restrict__ wb,
+                                                                    const float4* __restrict__ dwa, const float4* __restrict__ dwb, int64_t n,
+                                                                    float* __restrict__ dpin, float* __restrict__ partial) {
+    using namespace fixed;
+    extern __shared__ __align__(16) float sm[];
+    float *s_w = sm + F_W, *s_k = sm + F_K, *s_x = sm + F_X, *s_q = sm + F_Q, *s_dq = sm + F_DQ, *s_ds = sm + F_DS;
+    for (int i = threadIdx.x; i < H * 8 * PP; i += RT) {
+        const int r = i / PP, j = i % PP;
+        s_w[(r / 8) * WHEAD + (r % 8) * PP + j] = j < P ? Wq[r * P + j] : 0.f;
+    }
+    for (int i = threadIdx.x; i < N_K; i += RT) { s_k[i] = KA[i]; s_k[N_K + i] = KB[i]; }
+    for (int i = threadIdx.x; i < TILE * (PP - P); i += RT) s_x[(i / (PP - P)) * PP + P + i % (PP - P)] = 0.f;
+    const int le = threadIdx.x / H, h = threadIdx.x % H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rg = lane >> 2, cg = lane & 3;                    // d Wq rows 4 rg .. + 3, columns 6 cg .. + 5; key table rg & 1 of head rg >> 1, rows 3 cg .. + 2
+    float aw[4][6], ak[3][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 6; ++v) aw[u][v] = 0.f;
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) ak[u][v] = 0.f;
+    const int64_t tiles = (n + TILE - 1) / TILE;
+    for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int64_t left = n - tile * TILE;
+        const int cnt = left < TILE ? (int)left : TILE;
+        __syncthreads();                                        // the previous tile's sums have been taken
+        for (int i = threadIdx.x; i < cnt * P; i += RT) s_x[(i / P) * PP + i % P] = pin[tile * TILE * P + i];
+        __syncthreads();
+        const bool live = le < cnt;
+        float dt[8], dq[8], q[8], dp[PP];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) dq[k] = 0.f;
+#pragma unroll
+        for (int j = 0; j < PP; ++j) dp[j] = 0.f;
+        if (live) {
+            const int64_t r = (tile * TILE + le) * H + h;
+            const int4 a4 = ia[r], b4 = ib[r];
+            const float4 wa4 = wa[r], wb4 = wb[r], da4 = dwa[r], db4 = dwb[r];
+            const int a_i[RK] = {a4.x, a4.y, a4.z, a4.w}, b_i[RK] = {b4.x, b4.y, b4.z, b4.w};
+            const float a_w[RK] = {wa4.x, wa4.y, wa4.z, wa4.w}, b_w[RK] = {wb4.x, wb4.y, wb4.z, wb4.w};
+            const float a_d[RK] = {da4.x, da4.y, da4.z, da4.w}, b_d[RK] = {db4.x, db4.y, db4.z, db4.w};
+            route_bwd(a_i, b_i, a_w, b_w, a_d, b_d, s_k + h * PK * RH, s_k + N_K + h * PK * RH, dt, dq);
+            float4* ds = reinterpret_cast<float4*>(s_ds + le * SP + h * 2 * PK);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) ds[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            float* dsf = s_ds + le * SP + h * 2 * PK;
+#pragma unroll
+            for (int k = 0; k < RK; ++k) { dsf[a_i[k]] += dt[k]; dsf[PK + b_i[k]] += dt[RK + k]; }
+            float x[PP];
+#pragma unroll
+            for (int j = 0; j < PP / 4; ++j) {
+                const float4 v = reinterpret_cast<const float4*>(s_x + le * PP)[j];
+                x[4 * j] = v.x; x[4 * j + 1] = v.y; x[4 * j + 2] = v.z; x[4 * j + 3] = v.w;
+            }
+#pragma unroll
+            for (int o = 0; o < 8; ++o) {
+                float acc = 0.f;
+#pragma unroll
+                for (int j = 0; j < PP / 4; ++j) {
+                    const float4 v = reinterpret_cast<const float4*>(s_w + h * WHEAD + o * PP)[j];
+                    acc = fmaf(v.x, x[4 * j], acc); acc = fmaf(v.y, x[4 * j + 1], acc); acc = fmaf(v.z, x[4 * j + 2], acc); acc = fmaf(v.w, x[4 * j + 3], acc);
+                    dp[4 * j] = fmaf(v.x, dq[o], dp[4 * j]); dp[4 * j + 1] = fmaf(v.y, dq[o], dp[4 * j + 1]);
+                    dp[4 * j + 2] = fmaf(v.z, dq[o], dp[4 * j + 2]); dp[4 * j + 3] = fmaf(v.w, dq[o], dp[4 * j + 3]);
+                }
+                q[o] = acc;
+            }
+            float4* qo = reinterpret_cast<float4*>(s_q + le * QP + h * 8);
+            qo[0] = make_float4(q[0], q[1], q[2], q[3]); qo[1] = make_float4(q[4], q[5], q[6], q[7]);
+            float4* dqo = reinterpret_cast<float4*>(s_dq + le * QP + h * 8);
+            dqo[0] = make_float4(dq[0], dq[1], dq[2], dq[3]); dqo[1] = make_float4(dq[4], dq[5], dq[6], dq[7]);
+        }
+        {   // sum of d pin over the four heads (four neighbouring lanes); each keeps six columns
+            const bool hi = (h & 2) != 0, odd = (h & 1) != 0;
+            float a[12], c[6];
+#pragma unroll
+            for (int j = 0; j < 12; ++j) {
+                const float got = __shfl_xor_sync(0xffffffffu, hi ? dp[j] : dp[12 + j], 2);
+                a[j] = (hi ? dp[12 + j] : dp[j]) + got;
+            }
+#pragma unroll
+            for (int j = 0; j < 6; ++j) {
+                const float got = __shfl_xor_sync(0xffffffffu, odd ? a[j] : a[6 + j], 1);
+                c[j] = (odd ? a[6 + j] : a[j]) + got;
+            }
+            const int base = (hi ? 12 : 0) + (odd ? 6 : 0);
+            if (live)
+#pragma unroll
+                for (int j = 0; j < 6; ++j)
+                    if (base + j < P) dpin[(tile * TILE + le) * P + base + j] = c[j];
+        }
+        __syncthreads();
+        for (int m = warp; m < cnt; m += RT / 32) {
+            const float4 d = *reinterpret_cast<const float4*>(s_dq + m * QP + 4 * rg), qv = *reinterpret_cast<const float4*>(s_q + m * QP + 4 * rg);
+            float x[6];
+#pragma unroll
+            for (int v = 0; v < 3; ++v) {
+                const float2 t = reinterpret_cast<const float2*>(s_x + m * PP + 6 * cg)[v];
+                x[2 * v] = t.x; x[2 * v + 1] = t.y;
+            }
+            const float dr[4] = {d.x, d.y, d.z, d.w}, qr[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int v = 0; v < 6; ++v) aw[u][v] = fmaf(dr[u], x[v], aw[u][v]);
+            const float* ds = s_ds + m * SP + rg * PK + 3 * cg;   // [head][A, B][12]: rg = 2 head + table
+#pragma unroll
+            for (int u = 0; u < 3; ++u)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) ak[u][v] = fmaf(ds[u], qr[v], ak[u][v]);
+        }
+    }
+    __syncthreads();
+    float* red = s_x + warp * NG;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 6; ++v)
+            if (6 * cg + v < P) red[(4 * rg + u) * P + 6 * cg + v] = aw[u][v];
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) red[N_WQ + (rg & 1) * N_K + ((rg >> 1) * PK + 3 * cg + u) * 4 + v] = ak[u][v];
+    __syncthreads();
+    for (int i = threadIdx.x; i < NG; i += RT) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < RT / 32; ++w) t += s_x[w * NG + i];
+        partial[(int64_t)blockIdx.x * NG + i] = t;
+    }
 }
 
 size_t fwd_smem(int heads, int P, int pk) { return (size_t)weights_floats(heads, P, pk) * sizeof(float); }
@@ -196,11 +339,18 @@ int routing_bwd(const float* pin, const float* Wq, const float* KA, const float*
     if (n <= 0) return cudaMemsetAsync(dparams, 0, (size_t)ng * sizeof(float), s) == cudaSuccess ? 0 : 3;
     const size_t smem = bwd_smem(heads, P, pk);
     if (cudaFuncSetAttribute(routing_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 2;
-    const int ctas = routing_bwd_ctas(n, heads);
+    int ctas = routing_bwd_ctas(n, heads);
     count_launch(2);
-    routing_bwd_kernel<<<ctas, RT, smem, s>>>(pin, Wq, KA, KB, (const int4*)ia, (const int4*)ib, (const float4*)wa, (const float4*)wb,
-                                              (const float4*)dwa, (const float4*)dwb, n, heads, P, pk, dpin, partial);
-    routing_reduce_kernel<<<(ng + 255) / 256, 256, 0, s>>>(partial, ctas, ng, dparams);
+    if (heads == fixed::H && P == fixed::P && pk == fixed::PK) {
+        const size_t fsm = (size_t)fixed::FLOATS * sizeof(float);
+        if (cudaFuncSetAttribute(routing_bwd_default_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm) != cudaSuccess) return 2;
+        ctas = ctas < 2 * 148 ? ctas : 2 * 148;
+        routing_bwd_default_kernel<<<ctas, RT, fsm, s>>>(pin, Wq, KA, KB, (const int4*)ia, (const int4*)ib, (const float4*)wa, (const float4*)wb,
+                                                         (const float4*)dwa, (const float4*)dwb, n, dpin, partial);
+    } else
+        routing_bwd_kernel<<<ctas, RT, smem, s>>>(pin, Wq, KA, KB, (const int4*)ia, (const int4*)ib, (const float4*)wa, (const float4*)wb,
+                                                  (const float4*)dwa, (const float4*)dwb, n, heads, P, pk, dpin, partial);
+    column_parts_kernel<<<(ng + 31) / 32, 1024, 0, s>>>(partial, ctas, ng, dparams);
     return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 

@@ -199,6 +199,8 @@ constexpr int MAX_RANKS = 8;
 constexpr int STATUS_OK = 0;
 constexpr int STATUS_TIMEOUT = 1;     // status word = STATUS_TIMEOUT | (peer << 8) | (site << 16)
 struct PeerPtrs { void* p[MAX_RANKS]; };
+// Optional state snapshots of the scan (bilevel): the state before every `every`-th 16-step tile of item i goes to out[base[i] + k] ([16][16] floats).
+struct ScanSnaps { float* out; const int64_t* base; int every; };
 int sg2_scan_resident_items();       // scan items an SM holds at once (the host sizes its chunks in whole waves)
 void write_words(uint32_t* dst, const uint32_t* host_words, int n, cudaStream_t s);
 }  // namespace sg

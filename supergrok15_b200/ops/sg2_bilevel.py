@@ -157,7 +157,7 @@ class _ScanCtx(torch.autograd.Function):
         p = wsp.plan
         torch._foreach_copy_(wsp.h_fwd + wsp.h_bwd, list(fwd_states) + list(bwd_states))
         buf = C.sg2_prepare(grads_list, sharps, p.offsets[:-1], p.total, p.seg_off, 1e30, p.ws)      # no clipping: raw gradients
-        C.sg2_scan(p.items, p.n_items, p.dir1_start, p.tds, p.n_td, p.any_multi, buf, p.ws)
+        C.sg2_scan(p.items, p.n_items, p.dir1_start, p.tds, p.n_td, p.any_multi, buf, p.ws, snaps=wsp.snaps, snap_base=wsp.snap_base, snap_every=wsp.snap_every)
         ctx.wsp, ctx.buf, ctx.w, ctx.leaves = wsp, buf, w, leaves
         return p.ws["ctx"][: 16 * p.total].view(p.total, 16).clone()
 
