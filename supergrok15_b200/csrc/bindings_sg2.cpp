@@ -24,7 +24,6 @@ void sg2_elem(int dtype, const MTArgs& a, float beta2, float eps, float rescale,
               cudaStream_t s);
 size_t sg2_item_bytes();
 size_t sg2_td_bytes();
-size_t sg2_bilevel_smem_bytes();
 int sg2_bilevel_ng();
 int sg2_bilevel_tile();
 void sg2_scan_backward(const void* items_dev, int n_items, int dir1_start, const void* tds_dev, int n_td, const int64_t* snap_base_dev,
@@ -533,7 +532,7 @@ void register_sg2(pybind11::module_& m) {
           py::arg("snap_base"), py::arg("sorted_buf"), py::arg("dctx"), py::arg("ws"), py::arg("snaps"), py::arg("partial"), py::arg("grads"),
           py::arg("snap_every") = 1);
     m.def("sg2_bilevel_info", []() { py::dict d; d["ng"] = sg::sg2_bilevel_ng(); d["tile"] = sg::sg2_bilevel_tile();
-                                     d["smem"] = (int64_t)sg::sg2_bilevel_smem_bytes(); return d; });
+                                      return d; });
     m.def("sg2_sort_blocks", [](int64_t total) { return (int64_t)sg::sg2_sort_blocks(total); });
 }
 }  // namespace sgb

@@ -21,15 +21,18 @@ constexpr int XH = 16;            // expert hidden width
 constexpr int XK = 4;             // keys kept per sub-key (top-4 x top-4 = 16 experts per head)
 constexpr int XTHREADS = 256;
 constexpr int XMAXQ = 9;          // (expert, hidden) pairs per thread in the backward pass: experts <= 16 * XMAXQ = 144
+constexpr int XE = 16 * XMAXQ;    // row pitch of the dense routing table (columns from E on stay zero)
 constexpr int XSEG = XH + 1;      // linear pieces of an expert = row pitch of its tables (odd: different experts fall into different banks)
 
 // An expert is a piecewise linear function of the scalar g: hidden unit j switches at t_j = -b1_j / W1_j.  The tables hold the sorted
-// switching points and, per piece, slope and intercept (summed in fp64), so that a value takes five comparisons and one FMA instead of
-// 16 hidden units with three table words each; both forms were bound by the shared-memory reads (54 against 6 per value).
+// switching points and, per piece, slope and intercept (summed in fp64), so that a value takes five comparisons, an FMA and an addition
+// instead of 16 hidden units with three table words each; both forms were bound by the shared-memory reads (54 against 7 per value).
+// The intercept is kept as a rounded value and its remainder: its rounding error would be the same for all elements of a piece and would
+// not average out of the sums over them (gradients of the keys, which live on differences of expert values).
 // The indicator of a unit (for the parameter gradients) is still evaluated from its own weights: at a switching point the value does
 // not care on which side it is taken, a derivative would.
-struct XTable { const float* t; const float2* ab; };
-size_t __host__ __device__ constexpr x_table_floats(int E) { return (size_t)E * XSEG * 3 + ((E * XSEG) & 1); }      // t padded to a float2 boundary
+struct XTable { const float* t; const float* hi; const float2* ab; };                                    // ab: slope, remainder of the intercept
+size_t __host__ __device__ constexpr x_table_floats(int E) { return (size_t)E * XSEG * 4; }
 
 // sixteen lanes per expert: lane j ranks its switching point, lane s sums piece s (lane 0 also piece 16)
 __global__ void __launch_bounds__(128) experts_table_kernel(const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
@@ -44,7 +47,8 @@ __global__ void __launch_bounds__(128) experts_table_kernel(const float* __restr
         rank += (tk < t || (tk == t && k < j)) ? 1 : 0;
     }
     float* th = table + (size_t)e * XSEG;
-    float2* ab = reinterpret_cast<float2*>(table + E * XSEG + ((E * XSEG) & 1)) + (size_t)e * XSEG;
+    float* hi = table + ((size_t)E + e) * XSEG;
+    float2* ab = reinterpret_cast<float2*>(table + 2 * (size_t)E * XSEG) + (size_t)e * XSEG;
     if (e_raw < E) th[rank] = t;
     const double base = (double)b2[e];
     for (int rep = 0; rep < 2; ++rep) {
@@ -56,13 +60,13 @@ __global__ void __launch_bounds__(128) experts_table_kernel(const float* __restr
             const bool on = kw1 > 0.f ? kr < s : kw1 < 0.f ? kr >= s : kb > 0.f;
             if (on) { slope += (double)kw2 * kw1; icept += (double)kw2 * kb; }
         }
-        if (e_raw < E && (rep == 0 || j == 0)) ab[s] = make_float2((float)slope, (float)icept);
+        if (e_raw < E && (rep == 0 || j == 0)) { hi[s] = (float)icept; ab[s] = make_float2((float)slope, (float)(icept - (double)(float)icept)); }
     }
 }
 
 __device__ __forceinline__ XTable load_table(float* sm, const float* __restrict__ table, int E) {
     for (int i = threadIdx.x; i < (int)x_table_floats(E); i += XTHREADS) sm[i] = table[i];
-    return XTable{sm, reinterpret_cast<const float2*>(sm + E * XSEG + ((E * XSEG) & 1))};
+    return XTable{sm, sm + E * XSEG, reinterpret_cast<const float2*>(sm + 2 * E * XSEG)};
 }
 
 __device__ __forceinline__ float expert_eval(const XTable& p, int e, float g) {
@@ -73,7 +77,12 @@ __device__ __forceinline__ float expert_eval(const XTable& p, int e, float g) {
     s += g > t[s] ? 1 : 0;
     s += g > t[s] ? 1 : 0;
     const float2 ab = p.ab[e * XSEG + s];
-    return fmaf(ab.x, g, ab.y);
+    return fmaf(ab.x, g, ab.y) + p.hi[e * XSEG + s];
+}
+
+__device__ __forceinline__ int expert_of(int a, int b, int pk, int E) {
+    const int e = a * pk + b;
+    return e < 0 ? 0 : (e >= E ? E - 1 : e);
 }
 
 // one thread per (element, head); the heads of an element are added in head order by the thread of head 0
@@ -100,9 +109,7 @@ __global__ void __launch_bounds__(XTHREADS) routed_experts_fwd_kernel(const floa
         for (int a = 0; a < XK; ++a)
 #pragma unroll
             for (int b = 0; b < XK; ++b) {
-                int e = av[a] * pk + bv[b];
-                e = e < 0 ? 0 : (e >= E ? E - 1 : e);
-                t = fmaf(wav[a] * wbv[b], expert_eval(p, e, gv), t);
+                t = fmaf(wav[a] * wbv[b], expert_eval(p, expert_of(av[a], bv[b], pk, E), gv), t);
             }
     }
     s_tot[threadIdx.x] = t;
@@ -115,7 +122,7 @@ __global__ void __launch_bounds__(XTHREADS) routed_experts_fwd_kernel(const floa
 }
 
 // Persistent CTAs over tiles of XTHREADS / heads elements.  partial: [gridDim.x, 3*E*XH + E] (dW1, db1, dW2, db2).
-__global__ void __launch_bounds__(XTHREADS) routed_experts_bwd_kernel(const float* __restrict__ g, const int4* __restrict__ ia,
+__global__ void __launch_bounds__(XTHREADS, 2) routed_experts_bwd_kernel(const float* __restrict__ g, const int4* __restrict__ ia,
                                                                       const int4* __restrict__ ib, const float4* __restrict__ wa,
                                                                       const float4* __restrict__ wb, const float* __restrict__ W1,
                                                                       const float* __restrict__ b1, const float* __restrict__ W2,
@@ -126,48 +133,43 @@ __global__ void __launch_bounds__(XTHREADS) routed_experts_bwd_kernel(const floa
     const XTable p = load_table(sm, table, E);
     const int epc = XTHREADS / heads;
     float* s_g = sm + x_table_floats(E);                                // [epc]
-    float* s_route = s_g + XTHREADS;                                    // [epc][E]
+    float* s_route = s_g + XTHREADS;                                    // [epc][XE]
     __syncthreads();
     const int le = threadIdx.x / heads, h = threadIdx.x % heads;
     // the (expert, hidden unit) pairs of this thread: hidden unit j is fixed, experts e0 + 16 q
     const int j = threadIdx.x & (XH - 1), e0 = threadIdx.x / XH;
-    float w1r[XMAXQ], b1r[XMAXQ], w2r[XMAXQ], aw1[XMAXQ], ab1[XMAXQ], aw2[XMAXQ], ab2[XMAXQ];
+    // per pair: sums of c * g, c and c * z over the elements whose unit is on (c: the element's routing weight times its gradient)
+    float w1r[XMAXQ], b1r[XMAXQ], cg[XMAXQ], c0[XMAXQ], cz[XMAXQ], csum = 0.f;
 #pragma unroll
     for (int q = 0; q < XMAXQ; ++q) {
         const int e = e0 + (XTHREADS / XH) * q;
         const bool in = e < E;
         w1r[q] = in ? W1[e * XH + j] : 0.f;
         b1r[q] = in ? b1[e * XH + j] : 0.f;
-        w2r[q] = in ? W2[e * XH + j] : 0.f;
-        aw1[q] = ab1[q] = aw2[q] = ab2[q] = 0.f;
+        cg[q] = c0[q] = cz[q] = 0.f;
     }
     const int64_t tiles = (n + epc - 1) / epc;
     for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int64_t elem = tile * epc + le;
         const bool live = le < epc && elem < n;
-        int ev[XK * XK];
-        float cv[XK * XK];
-        float dt = 0.f;
+        int av[XK] = {0, 0, 0, 0}, bv[XK] = {0, 0, 0, 0};
+        float wav[XK], wbv[XK], dt = 0.f;
         if (live) {
             const float gv = g[elem];
             dt = dtotal[elem];
             const int64_t r = elem * heads + h;
             const int4 a4 = ia[r], b4 = ib[r];
             const float4 wa4 = wa[r], wb4 = wb[r];
-            const int av[XK] = {a4.x, a4.y, a4.z, a4.w}, bv[XK] = {b4.x, b4.y, b4.z, b4.w};
-            const float wav[XK] = {wa4.x, wa4.y, wa4.z, wa4.w}, wbv[XK] = {wb4.x, wb4.y, wb4.z, wb4.w};
+            av[0] = a4.x; av[1] = a4.y; av[2] = a4.z; av[3] = a4.w; bv[0] = b4.x; bv[1] = b4.y; bv[2] = b4.z; bv[3] = b4.w;
+            wav[0] = wa4.x; wav[1] = wa4.y; wav[2] = wa4.z; wav[3] = wa4.w; wbv[0] = wb4.x; wbv[1] = wb4.y; wbv[2] = wb4.z; wbv[3] = wb4.w;
             float da[XK] = {0.f, 0.f, 0.f, 0.f}, db[XK] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int a = 0; a < XK; ++a)
 #pragma unroll
                 for (int b = 0; b < XK; ++b) {
-                    int e = av[a] * pk + bv[b];
-                    e = e < 0 ? 0 : (e >= E ? E - 1 : e);
-                    const float dw = dt * expert_eval(p, e, gv);       // d total / d (wa*wb) times the incoming gradient
+                    const float dw = dt * expert_eval(p, expert_of(av[a], bv[b], pk, E), gv);       // d total / d (wa*wb) times the incoming gradient
                     da[a] = fmaf(dw, wbv[b], da[a]);
                     db[b] = fmaf(dw, wav[a], db[b]);
-                    ev[a * XK + b] = e;
-                    cv[a * XK + b] = dt * wav[a] * wbv[b];
                 }
             dwa[r] = make_float4(da[0], da[1], da[2], da[3]);
             dwb[r] = make_float4(db[0], db[1], db[2], db[3]);
@@ -175,14 +177,14 @@ __global__ void __launch_bounds__(XTHREADS) routed_experts_bwd_kernel(const floa
         } else if (h == 0 && le < epc) {
             s_g[le] = 0.f;
         }
-        for (int i = threadIdx.x; i < epc * E; i += XTHREADS) s_route[i] = 0.f;
+        for (int i = threadIdx.x; i < epc * XE; i += XTHREADS) s_route[i] = 0.f;
         __syncthreads();
         // head after head: within one head the 16 experts of an element are distinct when its keys are (top-k indices are);
         // repeated keys would still be added by one thread, in a fixed order
         for (int hh = 0; hh < heads; ++hh) {
             if (live && h == hh) {
 #pragma unroll
-                for (int k = 0; k < XK * XK; ++k) s_route[le * E + ev[k]] += cv[k];
+                for (int k = 0; k < XK * XK; ++k) s_route[le * XE + expert_of(av[k / XK], bv[k % XK], pk, E)] += dt * wav[k / XK] * wbv[k % XK];
             }
             __syncthreads();
         }
@@ -190,24 +192,16 @@ __global__ void __launch_bounds__(XTHREADS) routed_experts_bwd_kernel(const floa
         const int cnt = left < epc ? (int)left : epc;
         for (int m = 0; m < cnt; ++m) {
             const float gm = s_g[m];
-            const float* rt = s_route + m * E;
+            const float* rt = s_route + m * XE + e0;
 #pragma unroll
-            for (int q = 0; q < XMAXQ; ++q) {
-                const int e = e0 + (XTHREADS / XH) * q;
-                if (e < E) {
-                    const float c = rt[e];
-                    if (c != 0.f) {
-                        const float z = fmaf(gm, w1r[q], b1r[q]);
-                        const float on = z > 0.f ? 1.f : 0.f;
-                        aw2[q] = fmaf(c, z * on, aw2[q]);
-                        const float dz = c * w2r[q] * on;
-                        aw1[q] = fmaf(dz, gm, aw1[q]);
-                        ab1[q] += dz;
-                        ab2[q] += c;
-                    }
-                }
+            for (int q = 0; q < XMAXQ; ++q) {                         // without branches: about half of the entries are zero, but never a whole warp's
+                const float z = fmaf(gm, w1r[q], b1r[q]);
+                const float c = z > 0.f ? rt[(XTHREADS / XH) * q] : 0.f;
+                cz[q] = fmaf(c, z, cz[q]); cg[q] = fmaf(c, gm, cg[q]); c0[q] += c;
             }
         }
+        if (threadIdx.x < E)
+            for (int m = 0; m < cnt; ++m) csum += s_route[m * XE + threadIdx.x];
         __syncthreads();                                               // the tables are rewritten by the next tile
     }
     float* out = partial + (int64_t)blockIdx.x * (3 * E * XH + E);
@@ -215,16 +209,17 @@ __global__ void __launch_bounds__(XTHREADS) routed_experts_bwd_kernel(const floa
     for (int q = 0; q < XMAXQ; ++q) {
         const int e = e0 + (XTHREADS / XH) * q;
         if (e < E) {
-            out[e * XH + j] = aw1[q];
-            out[E * XH + e * XH + j] = ab1[q];
-            out[2 * E * XH + e * XH + j] = aw2[q];
-            if (j == 0) out[3 * E * XH + e] = ab2[q];
+            const float w2 = W2[e * XH + j];
+            out[e * XH + j] = w2 * cg[q];
+            out[E * XH + e * XH + j] = w2 * c0[q];
+            out[2 * E * XH + e * XH + j] = cz[q];
         }
     }
+    if (threadIdx.x < E) out[3 * E * XH + threadIdx.x] = csum;
 }
 
 size_t fwd_smem(int E) { return (size_t)(x_table_floats(E) + XTHREADS) * sizeof(float); }
-size_t bwd_smem(int E, int heads) { return (size_t)(x_table_floats(E) + XTHREADS + (XTHREADS / heads) * E) * sizeof(float); }
+size_t bwd_smem(int E, int heads) { return (size_t)(x_table_floats(E) + XTHREADS + (XTHREADS / heads) * XE) * sizeof(float); }
 
 }  // namespace
 
