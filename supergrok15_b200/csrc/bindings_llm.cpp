@@ -210,9 +210,80 @@ std::vector<Tensor> flash_bwd(const Tensor& q, const Tensor& k, const Tensor& v,
                 " HD ", HD);
     return {dq, dk, dv};
 }
+
+// ---- autograd nodes in C++ (see bindings_nn.cpp)
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+
+struct CrossEntropyNode : Function<CrossEntropyNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& logits_, const Tensor& target_, int64_t ignore_index) {
+        Tensor logits = logits_.contiguous(), target = target_.contiguous();
+        auto r = ce_fwd(logits, target, ignore_index);
+        ctx->save_for_backward({logits, target, r[1], r[2]});
+        ctx->saved_data["ignore"] = ignore_index;
+        return r[0];
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list dy) {
+        const auto s = ctx->get_saved_variables();
+        return {ce_bwd(s[0], s[1], s[2], s[3], dy[0].reshape({1}), ctx->saved_data["ignore"].toInt()), Tensor(), Tensor()};
+    }
+};
+
+struct GeluNode : Function<GeluNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x_) {
+        Tensor x = x_.contiguous();
+        ctx->save_for_backward({x});
+        return gelu_fwd(x);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list dy) { return {gelu_bwd(ctx->get_saved_variables()[0], dy[0])}; }
+};
+
+struct SwigluNode : Function<SwigluNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& g_, const Tensor& u_) {
+        Tensor g = g_.contiguous(), u = u_.contiguous();
+        ctx->save_for_backward({g, u});
+        return swiglu_fwd(g, u);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list dy) {
+        const auto s = ctx->get_saved_variables();
+        auto r = swiglu_bwd(s[0], s[1], dy[0]);
+        return {r[0], r[1]};
+    }
+};
+
+struct RopeNode : Function<RopeNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& c, const Tensor& s) {
+        ctx->save_for_backward({c, s});
+        return rope(x.contiguous(), c, s, false);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list dy) {
+        const auto t = ctx->get_saved_variables();
+        return {rope(dy[0].contiguous(), t[0], t[1], true), Tensor(), Tensor()};
+    }
+};
+
+struct FlashNode : Function<FlashNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, bool causal, const Tensor& err) {
+        auto r = flash_fwd(q, k, v, causal, err, 3);
+        ctx->save_for_backward({q, k, v, r[0], r[1], err});
+        ctx->saved_data["causal"] = causal;
+        return r[0];
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list dy) {
+        const auto s = ctx->get_saved_variables();
+        auto r = flash_bwd(s[0], s[1], s[2], s[3], s[4], dy[0], ctx->saved_data["causal"].toBool(), s[5]);
+        return {r[0], r[1], r[2], Tensor(), Tensor()};
+    }
+};
 }  // namespace
 
 void register_llm(pybind11::module_& m) {
+    m.def("cross_entropy_node", [](const Tensor& logits, const Tensor& target, int64_t ignore_index) { return CrossEntropyNode::apply(logits, target, ignore_index); });
+    m.def("gelu_node", [](const Tensor& x) { return GeluNode::apply(x); });
+    m.def("swiglu_node", [](const Tensor& g, const Tensor& u) { return SwigluNode::apply(g, u); });
+    m.def("rope_node", [](const Tensor& x, const Tensor& c, const Tensor& s) { return RopeNode::apply(x, c, s); });
+    m.def("flash_node", [](const Tensor& q, const Tensor& k, const Tensor& v, bool causal, const Tensor& err) { return FlashNode::apply(q, k, v, causal, err); });
     m.def("rope", &rope, py::arg("x"), py::arg("cos"), py::arg("sin"), py::arg("backward") = false);
     m.def("swiglu_fwd", &swiglu_fwd);
     m.def("swiglu_bwd", &swiglu_bwd);

@@ -25,6 +25,17 @@ import torch.nn.functional as F
 from .. import _build
 
 
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def _cpp_node(*tensors: Optional[torch.Tensor]) -> bool:
+    """Whether a call may use the C++ autograd node of its operation (``csrc/bindings_nn.cpp``, ``csrc/bindings_llm.cpp``): plain eager tensors.
+    Inside a gradient sink, under functorch transforms and forward-mode AD, while tracing or compiling and for tensor subclasses the
+    Python functions below take the call, as they define what happens there."""
+    return not (_SINK.on or torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0 or
+                torch.jit.is_tracing() or torch.compiler.is_compiling()) and all(t is None or type(t) in _PLAIN for t in tensors)
+
+
 def attention_small_reference(qkv: torch.Tensor, n_heads: int, causal: bool = True) -> torch.Tensor:
     B, S, D3 = qkv.shape
     D = D3 // 3
@@ -56,6 +67,8 @@ def attention_small_supported(qkv: torch.Tensor, n_heads: int) -> bool:
 def attention_small(qkv: torch.Tensor, n_heads: int, causal: bool = True) -> torch.Tensor:
     if not attention_small_supported(qkv, n_heads):
         return attention_small_reference(qkv, n_heads, causal)
+    if _cpp_node(qkv):
+        return _build.require().attn_small_node(qkv, n_heads, causal)
     return _AttnSmall.apply(qkv, n_heads, causal)
 
 
@@ -219,10 +232,7 @@ def _col_sum_bias(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Te
         return False
     if x.dtype not in (torch.float32, torch.bfloat16, torch.float16) or x.dtype != weight.dtype or x.dtype != bias.dtype or x.numel() < _COL_SUM_ROWS * x.shape[-1]:
         return False
-    if x.shape[-1] == 0 or type(x) not in (torch.Tensor, torch.nn.Parameter) or type(weight) not in (torch.Tensor, torch.nn.Parameter) or type(bias) not in (torch.Tensor, torch.nn.Parameter):
-        return False
-    return not (torch.is_autocast_enabled("cuda") or torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0 or
-                torch.jit.is_tracing() or torch.compiler.is_compiling())
+    return x.shape[-1] > 0 and not torch.is_autocast_enabled("cuda") and _cpp_node(x, weight, bias)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -244,6 +254,8 @@ def layer_norm(x: torch.Tensor, residual: Optional[torch.Tensor], weight: torch.
     if not x.is_cuda or x.dtype not in (torch.bfloat16, torch.float32) or x.shape[-1] % 4 or x.shape[-1] > 3072:
         z = x if residual is None else x + residual
         return F.layer_norm(z, (x.shape[-1],), weight, bias, eps)
+    if _cpp_node(x, residual, weight, bias):
+        return _build.require().norm_node(x, residual, weight, bias, eps, False)
     return _LayerNorm.apply(x, residual, weight, bias, eps)
 
 
@@ -276,6 +288,8 @@ def norm_residual(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor,
         z = x + residual
         y = F.rms_norm(z, (x.shape[-1],), weight, eps) if rms else F.layer_norm(z, (x.shape[-1],), weight, bias, eps)
         return y, z
+    if _cpp_node(x, residual, weight, bias):
+        return _build.require().norm_residual_node(x, residual, weight, bias, eps, rms)
     return _NormResidual.apply(x, residual, weight, bias, eps, rms)
 
 
@@ -327,6 +341,9 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = 
     import os
     impl = impl or os.environ.get("SG_ATTN", "sdpa")
     if impl == "tcgen05" and flash_supported(q, k, v):
+        if _cpp_node(q, k, v):
+            from . import gemm as _gemm
+            return _build.require().flash_node(q, k, v, causal, _gemm._err_flag(q.device))
         return _FlashAttention.apply(q, k, v, causal)
     return attention_reference(q, k, v, causal)
 
@@ -340,6 +357,8 @@ def rms_norm(x: torch.Tensor, residual: Optional[torch.Tensor], weight: torch.Te
     if not x.is_cuda or x.dtype not in (torch.bfloat16, torch.float32) or x.shape[-1] % 4 or x.shape[-1] > 3072 or weight.dtype != x.dtype:
         z = x if residual is None else x + residual
         return F.rms_norm(z, (x.shape[-1],), weight, eps)
+    if _cpp_node(x, residual, weight):
+        return _build.require().norm_node(x, residual, weight, None, eps, True)
     return _LayerNorm.apply(x, residual, weight, None, eps, True)
 
 
@@ -365,7 +384,8 @@ class _Rope(torch.autograd.Function):
 def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
     if not _native_ok(x) or x.shape[-1] % 8:
         return rope_reference(x, cos, sin)
-    return _Rope.apply(x, cos.float().contiguous(), sin.float().contiguous())
+    cos, sin = cos.float().contiguous(), sin.float().contiguous()
+    return _build.require().rope_node(x, cos, sin) if _cpp_node(x, cos, sin) else _Rope.apply(x, cos, sin)
 
 
 class _SwiGLU(torch.autograd.Function):
@@ -385,7 +405,7 @@ class _SwiGLU(torch.autograd.Function):
 def swiglu(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     if not _native_ok(gate) or gate.numel() % 8 or gate.dtype != up.dtype:
         return F.silu(gate) * up
-    return _SwiGLU.apply(gate, up)
+    return _build.require().swiglu_node(gate, up) if _cpp_node(gate, up) else _SwiGLU.apply(gate, up)
 
 
 class _Gelu(torch.autograd.Function):
@@ -404,7 +424,7 @@ class _Gelu(torch.autograd.Function):
 def gelu(x: torch.Tensor) -> torch.Tensor:
     if not _native_ok(x) or x.numel() % 8:
         return F.gelu(x)
-    return _Gelu.apply(x)
+    return _build.require().gelu_node(x) if _cpp_node(x) else _Gelu.apply(x)
 
 
 class _Embedding(torch.autograd.Function):
@@ -451,4 +471,6 @@ def cross_entropy(logits: torch.Tensor, target: torch.Tensor, ignore_index: int 
     """Mean cross-entropy of logits [rows, V] against int64 targets [rows]; the result is an fp32 scalar."""
     if not _native_ok(logits) or logits.dim() != 2 or logits.shape[1] % 8:
         return F.cross_entropy(logits.float(), target, ignore_index=ignore_index)
+    if _cpp_node(logits, target):
+        return _build.require().cross_entropy_node(logits, target, ignore_index)
     return _CrossEntropy.apply(logits, target, ignore_index)
