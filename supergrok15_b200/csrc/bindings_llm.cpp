@@ -156,7 +156,7 @@ std::vector<Tensor> ce_fwd(const Tensor& logits, const Tensor& target, int64_t i
     c10::cuda::CUDAGuard guard(logits.device());
     const int64_t rows = logits.size(0);
     auto fo = logits.options().dtype(at::kFloat);
-    Tensor lse = at::empty({rows}, fo), loss = at::empty({rows}, fo), mean_out = at::zeros({2}, fo);
+    Tensor lse = at::empty({rows}, fo), loss = at::empty({rows}, fo), mean_out = rows > 0 ? at::empty({2}, fo) : at::zeros({2}, fo);
     sg::ce_fwd(dtype_code(logits), logits.data_ptr(), target.data_ptr<int64_t>(), lse.data_ptr<float>(), loss.data_ptr<float>(),
                mean_out.data_ptr<float>(), rows, (int)logits.size(1), ignore_index, at::cuda::getCurrentCUDAStream());
     return {mean_out.narrow(0, 0, 1).reshape({}), lse, mean_out};
