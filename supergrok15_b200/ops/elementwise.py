@@ -98,8 +98,9 @@ def clip_coef_device(grads: Tensors, max_norm: float) -> torch.Tensor:
     dev = grads[0].device
     pt = sqnorm_per_tensor(grads)
     out = workspace(dev, "clip", 4)
-    tot = _global_totals(pt, len(grads), dev)
-    _build.require().scalar_finalize(_op("SC_CLIP"), tot, 1, out, float(max_norm), 0.0, 0.0)
+    # the coefficient's kernel sums the tensors itself; only totals that other ranks add to need a launch of their own
+    tot, n = (pt, len(grads)) if _reducer is None else (_global_totals(pt, len(grads), dev), 1)
+    _build.require().scalar_finalize(_op("SC_CLIP"), tot, n, out, float(max_norm), 0.0, 0.0)
     return out
 
 
