@@ -25,6 +25,7 @@ using namespace tc;
 
 constexpr int FA_THREADS = 192;
 constexpr int FB_THREADS = 320;                          // backward: TMA warp, MMA warp, two groups of four warps
+constexpr int FB_GRID = 148;                             // and one persistent CTA per SM
 constexpr uint32_t TILE_HALF_BYTES = 128 * 128;          // [128 rows x 64 bf16] = 16 KB
 
 __device__ __forceinline__ float ex2f(float x) {
@@ -751,14 +752,36 @@ struct FbBars {
 //    [64g, 64g+32) of the same block, which only it has read, so the groups need not wait for each other;
 //  - the next tile's X is issued as soon as all threads have taken this tile's scores out (pa_full), its Y as soon as dS is stored
 //    (pb_full): the tensor cores work on dV and X while the threads form dS, and on dK and Y while they form the next P.
-// B4 S2048 H16 hd128 causal: kernel A 212 -> 175 us, kernel B 153 -> 129 us against four warps and products issued tile by tile.
+// The kernel is persistent: one CTA per SM walks over its tiles with the barriers and the TMEM kept, and the loads and the first
+// products of its next tile run while the threads finish this one.
+// B4 S2048 H16 hd128 causal, kernel A / kernel B: 212 / 153 us with four warps and products issued tile by tile, 175 / 129 with the two
+// points above, 166 / 124 persistent (tensor pipe 41 % busy before the last step).
+struct FbItem { int h, b, tile, first, n_it; };
+
+// Work item k of a CTA.  Items are ordered by decreasing work (kernel A: key tile 0 is visited by every query tile; kernel B: the
+// last query tile visits every key tile; the (batch, head) pairs of one tile index are adjacent) and dealt out back and forth, so
+// that under the causal mask a CTA which got a long item in one round gets a short one in the next.
+template <bool KV>
+__device__ __forceinline__ bool fb_item(int k, int n_hb, int nt, int H, int causal, FbItem& w) {
+    const int G = (int)gridDim.x, item = (k & 1) ? (k + 1) * G - 1 - (int)blockIdx.x : k * G + (int)blockIdx.x;
+    if (item >= n_hb * nt) return false;
+    const int hb = item % n_hb, ord = item / n_hb;
+    w.h = hb % H; w.b = hb / H;
+    w.tile = KV ? ord : nt - 1 - ord;
+    w.first = KV && causal ? w.tile : 0;                                 // tiles of the other sequence axis that interact with this one
+    w.n_it = KV ? nt - w.first : (causal ? w.tile + 1 : nt);
+    return true;
+}
+constexpr int FB_STAGE_PITCH = 80;                                       // 64 bytes of a row and a pad: conflict-free 16-byte accesses
+constexpr int FB_STAGE_BYTES = 8 * 32 * FB_STAGE_PITCH;
+
 template <int HD, bool KV>
 __global__ void __launch_bounds__(FB_THREADS, 1) flash_bwd_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                   const __grid_constant__ CUtensorMap map_k,
                                                                   const __grid_constant__ CUtensorMap map_v,
                                                                   const __grid_constant__ CUtensorMap map_do, const float* __restrict__ lse,
                                                                   const float* __restrict__ delta, __nv_bfloat16* __restrict__ out0,
-                                                                  __nv_bfloat16* __restrict__ out1, int S, int H, int64_t ld_out, float scale,
+                                                                  __nv_bfloat16* __restrict__ out1, int S, int H, int n_hb, int64_t ld_out, float scale,
                                                                   int causal, int* __restrict__ err) {
     constexpr int HALVES = HD / 64;
     constexpr uint32_t QKV_BYTES = HALVES * TILE_HALF_BYTES;
@@ -770,19 +793,12 @@ __global__ void __launch_bounds__(FB_THREADS, 1) flash_bwd_kernel(const __grid_c
     uint8_t* sT1 = sT0 + 2 * QKV_BYTES;                  // ring [2]: dO_i (A) or V_j (B)
     float* s_lse = reinterpret_cast<float*>(sT1 + 2 * QKV_BYTES);       // [2][128] (kernel A: per-query vectors of the current tile)
     float* s_del = s_lse + 256;                                          // [2][128]
-    FbBars* bars = reinterpret_cast<FbBars*>(s_del + 256);
+    uint8_t* s_stage = reinterpret_cast<uint8_t*>(s_del + 256);          // [8 warps][32 rows] of the epilogue
+    FbBars* bars = reinterpret_cast<FbBars*>(s_stage + FB_STAGE_BYTES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nt = S / 128;
-    // 1-D grid ordered by decreasing work: kernel A starts with key tile 0 (visited by every query tile), kernel B with the last
-    // query tile; all (batch, head) pairs of one tile index are adjacent
-    const int n_hb = (int)gridDim.x / nt, hb = (int)blockIdx.x % n_hb, ord = (int)blockIdx.x / n_hb;
-    const int tile = KV ? ord : nt - 1 - ord;
-    const int h = hb % H, b = hb / H;
-    // tiles of the other sequence axis that interact with this one
-    const int first = KV ? (causal ? tile : 0) : 0;
-    const int n_it = KV ? nt - first : (causal ? tile + 1 : nt);
-    const int row_res = b * S + tile * 128, col0 = h * HD;
+    FbItem w;
 
     if (threadIdx.x == 0) {
         mbar_init(&bars->res_full, 1);
@@ -804,18 +820,26 @@ __global__ void __launch_bounds__(FB_THREADS, 1) flash_bwd_kernel(const __grid_c
 
     if (warp == 0) {
         if (lane == 0) {
-            mbar_expect_tx(&bars->res_full, 2 * QKV_BYTES);
-            for (int hf = 0; hf < HALVES; ++hf) {
-                tma_load_2d(sR0 + hf * TILE_HALF_BYTES, KV ? &map_k : &map_q, col0 + hf * 64, row_res, &bars->res_full);
-                tma_load_2d(sR1 + hf * TILE_HALF_BYTES, KV ? &map_v : &map_do, col0 + hf * 64, row_res, &bars->res_full);
-            }
-            for (int it = 0; it < n_it; ++it) {
-                const int s = it & 1, row_t = b * S + (first + it) * 128;
-                if (it >= 2 && !mbar_wait(&bars->ring_empty[s], ((it >> 1) & 1) ^ 1)) { atomicExch(err, 31); break; }
-                mbar_expect_tx(&bars->ring_full[s], 2 * QKV_BYTES);
-                for (int hf = 0; hf < HALVES; ++hf) {
-                    tma_load_2d(sT0 + s * QKV_BYTES + hf * TILE_HALF_BYTES, KV ? &map_q : &map_k, col0 + hf * 64, row_t, &bars->ring_full[s]);
-                    tma_load_2d(sT1 + s * QKV_BYTES + hf * TILE_HALF_BYTES, KV ? &map_do : &map_v, col0 + hf * 64, row_t, &bars->ring_full[s]);
+            bool ok = true;
+            for (int k = 0, n = 0; ok && fb_item<KV>(k, n_hb, nt, H, causal, w); ++k) {
+                const int col0 = w.h * HD;
+                for (int it = 0; it < w.n_it; ++it, ++n) {
+                    const int s = n & 1, row_t = w.b * S + (w.first + it) * 128;
+                    if (n >= 2 && !mbar_wait(&bars->ring_empty[s], ((n >> 1) & 1) ^ 1)) { atomicExch(err, 31); ok = false; break; }
+                    mbar_expect_tx(&bars->ring_full[s], 2 * QKV_BYTES);
+                    for (int hf = 0; hf < HALVES; ++hf) {
+                        tma_load_2d(sT0 + s * QKV_BYTES + hf * TILE_HALF_BYTES, KV ? &map_q : &map_k, col0 + hf * 64, row_t, &bars->ring_full[s]);
+                        tma_load_2d(sT1 + s * QKV_BYTES + hf * TILE_HALF_BYTES, KV ? &map_do : &map_v, col0 + hf * 64, row_t, &bars->ring_full[s]);
+                    }
+                    if (it == 0) {                                        // the resident tiles are free once the last Y before this item is done
+                        if (n > 0 && !mbar_wait(&bars->b_full, (n - 1) & 1)) { atomicExch(err, 30); ok = false; break; }
+                        const int row_res = w.b * S + w.tile * 128;
+                        mbar_expect_tx(&bars->res_full, 2 * QKV_BYTES);
+                        for (int hf = 0; hf < HALVES; ++hf) {
+                            tma_load_2d(sR0 + hf * TILE_HALF_BYTES, KV ? &map_k : &map_q, col0 + hf * 64, row_res, &bars->res_full);
+                            tma_load_2d(sR1 + hf * TILE_HALF_BYTES, KV ? &map_v : &map_do, col0 + hf * 64, row_res, &bars->res_full);
+                        }
+                    }
                 }
             }
         }
@@ -840,66 +864,83 @@ __global__ void __launch_bounds__(FB_THREADS, 1) flash_bwd_kernel(const __grid_c
                     tc_mma_bf16_ta(acc, tm + (kk >> 2) * 64 + (kk & 3) * 8, make_desc_sw128_mn(t0 + kk * 2048, TILE_HALF_BYTES, 1024), idesc_acc,
                                    (add || kk > 0) ? 1u : 0u);
             };
-            bool ok = mbar_wait(&bars->res_full, 0);
-            if (!ok) atomicExch(err, 32);
-            if (ok && !mbar_wait(&bars->ring_full[0], 0)) { atomicExch(err, 33); ok = false; }
-            if (ok) {
+            // the tiles of iteration n (of the item that is the k-th of this CTA) are in shared memory
+            auto tiles_ready = [&](int n, int k, bool first_it) {
+                if (first_it && !mbar_wait(&bars->res_full, k & 1)) { atomicExch(err, 32); return false; }
+                if (!mbar_wait(&bars->ring_full[n & 1], (n >> 1) & 1)) { atomicExch(err, 33); return false; }
                 tc_fence_after();
+                return true;
+            };
+            bool more = fb_item<KV>(0, n_hb, nt, H, causal, w), ok = more && tiles_ready(0, 0, true);
+            if (ok) {
                 first_product(tm_x, sR0, sT0);
                 tc_commit(&bars->a_full);
                 first_product(tm_y, sR1, sT1);
                 tc_commit(&bars->b_full);
             }
-            for (int it = 0; it < n_it && ok; ++it) {
-                const int s = it & 1, ns = s ^ 1;
-                const bool more = it + 1 < n_it;
-                if (!mbar_wait(&bars->pa_full, it & 1)) { atomicExch(err, 34); ok = false; break; }
-                tc_fence_after();
-                if (KV) acc_product(tm_acc0, tm_x, sT1 + s * QKV_BYTES, it > 0);                     // dV += P^T . dO_i
-                if (more) {
-                    if (!mbar_wait(&bars->ring_full[ns], ((it + 1) >> 1) & 1)) { atomicExch(err, 33); ok = false; break; }
+            for (int k = 0, n = 0; ok && more; ++k) {
+                const int n_it = w.n_it;
+                more = fb_item<KV>(k + 1, n_hb, nt, H, causal, w);
+                for (int it = 0; it < n_it; ++it, ++n) {
+                    const int s = n & 1, ns = s ^ 1;
+                    const bool last = it + 1 == n_it, next = !last || more;
+                    if (!mbar_wait(&bars->pa_full, n & 1)) { atomicExch(err, 34); ok = false; break; }
                     tc_fence_after();
-                    first_product(tm_x, sR0, sT0 + ns * QKV_BYTES);
-                    tc_commit(&bars->a_full);
-                }
-                if (!mbar_wait(&bars->pb_full, it & 1)) { atomicExch(err, 35); ok = false; break; }
-                tc_fence_after();
-                acc_product(KV ? tm_acc1 : tm_acc0, tm_y, sT0 + s * QKV_BYTES, it > 0);              // dK += dS^T . Q_i / dQ += dS . K_j
-                tc_commit(&bars->ring_empty[s]);
-                if (more) {
-                    first_product(tm_y, sR1, sT1 + ns * QKV_BYTES);
-                    tc_commit(&bars->b_full);
+                    if (KV) acc_product(tm_acc0, tm_x, sT1 + s * QKV_BYTES, it > 0);                     // dV += P^T . dO_i
+                    if (next) {
+                        if (!tiles_ready(n + 1, k + 1, last)) { ok = false; break; }
+                        first_product(tm_x, sR0, sT0 + ns * QKV_BYTES);
+                        tc_commit(&bars->a_full);
+                    }
+                    if (!mbar_wait(&bars->pb_full, n & 1)) { atomicExch(err, 35); ok = false; break; }
+                    tc_fence_after();
+                    acc_product(KV ? tm_acc1 : tm_acc0, tm_y, sT0 + s * QKV_BYTES, it > 0);              // dK += dS^T . Q_i / dQ += dS . K_j
+                    tc_commit(&bars->ring_empty[s]);
+                    if (last) tc_commit(&bars->done);
+                    if (next) {
+                        first_product(tm_y, sR1, sT1 + ns * QKV_BYTES);
+                        tc_commit(&bars->b_full);
+                    }
                 }
             }
-            tc_commit(&bars->done);
         }
     } else {
         const int q = warp & 3, g = (warp - 2) >> 2, row = q * 32 + lane, tl = (int)threadIdx.x - 64;
         const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
         const uint32_t my_x = tm_x + lane_addr + g * 64, my_y = tm_y + lane_addr + g * 64;
         const float c2 = scale * 1.4426950408889634f;
-        const int64_t vec0 = ((int64_t)b * H + h) * S;
-        float lse_row = 0.f, del_row = 0.f;
-        if (!KV) { lse_row = lse[vec0 + tile * 128 + row] * 1.4426950408889634f; del_row = delta[vec0 + tile * 128 + row]; }
-        // kernel A: the per-query vectors of a tile; threads 0..127 fetch -lse * log2(e), threads 128..255 delta
-        const float* vsrc = (tl < 128 ? lse : delta) + vec0 + (tl & 127);
+        // kernel A: the per-query vectors of a tile; threads 0..127 fetch -lse * log2(e), threads 128..255 delta.
+        // kernel B: both values of the thread's own query.
         float* vdst = (tl < 128 ? s_lse : s_del) + (tl & 127);
+        const float* vbase = (tl < 128 ? lse : delta) + (tl & 127);
         const float vmul = tl < 128 ? -1.4426950408889634f : 1.f;
-        bool ok = true;
+        float v0 = 0.f, v1 = 0.f;
+        int vo = 0;
+        auto fetch_first = [&](const FbItem& x) {
+            const int o = (x.b * H + x.h) * S;
+            if (KV) { vo = o + x.first * 128; v0 = vbase[vo]; }
+            else { v0 = lse[o + x.tile * 128 + row]; v1 = delta[o + x.tile * 128 + row]; }
+        };
+        bool ok = true, more = fb_item<KV>(0, n_hb, nt, H, causal, w);
+        if (more) fetch_first(w);
+        for (int k = 0, n = 0; ok && more; ++k) {
+        const int n_it = w.n_it, orow0 = w.b * S + w.tile * 128 + q * 32, ocol0 = w.h * HD;
+        const int diag_it = causal ? (KV ? 0 : n_it - 1) : -1;            // the iteration whose tile holds the diagonal
+        const float lse_row = v0 * 1.4426950408889634f, del_row = v1;
         if (KV) {
-            vdst[0] = vsrc[first * 128] * vmul;
+            vdst[(n & 1) * 128] = v0 * vmul;                              // buffer n & 1: every thread has left iteration n-2
             mbar_arrive_(&bars->vec_full);
         }
-        for (int it = 0; it < n_it && ok; ++it) {
-            const int other = first + it, bs = it & 1;
+        for (int it = 0; it < n_it && ok; ++it, ++n) {
+            const int bs = n & 1;
             // kernel A: the per-query vectors of the NEXT tile are fetched now and parked in the other buffer at the end of this
             // iteration, so their global-memory latency hides behind the work on this tile
             float nx = 0.f;
-            if (KV && it + 1 < n_it) nx = vsrc[(other + 1) * 128];
-            if (KV && !mbar_wait(&bars->vec_full, it & 1)) { atomicExch(err, 39); ok = false; break; }
-            if (!mbar_wait(&bars->a_full, it & 1)) { atomicExch(err, 36); ok = false; break; }
+            if (KV && it + 1 < n_it) { vo += 128; nx = vbase[vo]; }
+            if (KV && !mbar_wait(&bars->vec_full, n & 1)) { atomicExch(err, 39); ok = false; break; }
+            if (!mbar_wait(&bars->a_full, n & 1)) { atomicExch(err, 36); ok = false; break; }
             tc_fence_after();
-            const bool diag = causal && other == tile;
+            const bool diag = it == diag_it;
             uint32_t r[2][32];
 #pragma unroll
             for (int c = 0; c < 2; ++c) tc_ld32(my_x + c * 32, r[c]);
@@ -926,21 +967,20 @@ __global__ void __launch_bounds__(FB_THREADS, 1) flash_bwd_kernel(const __grid_c
 #pragma unroll
                     for (int i = 0; i < 32; ++i) if (KV ? c * 32 + i < rel : c * 32 + i > rel) r[c][i] = 0u;
             }
-            uint32_t pk[32];
+            uint32_t d[2][32];                                           // dP; d[0] also takes the packed bf16 operands, in place
             if (KV) {
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
                     const __nv_bfloat162 hh = __floats2bfloat162_rn(__uint_as_float(r[i >> 4][(2 * i) & 31]), __uint_as_float(r[i >> 4][(2 * i + 1) & 31]));
-                    pk[i] = *reinterpret_cast<const uint32_t*>(&hh);
+                    d[0][i] = *reinterpret_cast<const uint32_t*>(&hh);
                 }
-                tc_st32(my_x, pk);
+                tc_st32(my_x, d[0]);
                 tc_wait_st();
                 tc_fence_before();
                 mbar_arrive_(&bars->pa_full);
             }
-            if (!mbar_wait(&bars->b_full, it & 1)) { atomicExch(err, 37); ok = false; break; }
+            if (!mbar_wait(&bars->b_full, n & 1)) { atomicExch(err, 37); ok = false; break; }
             tc_fence_after();
-            uint32_t d[2][32];
 #pragma unroll
             for (int c = 0; c < 2; ++c) tc_ld32(my_y + c * 32, d[c]);
             tc_wait_ld();
@@ -955,10 +995,10 @@ __global__ void __launch_bounds__(FB_THREADS, 1) flash_bwd_kernel(const __grid_c
                     fma2g(u ? de.z : de.x, u ? de.w : de.y, -1.f, -1.f, __uint_as_float(d[c][k0]), __uint_as_float(d[c][k0 + 1]), t0, t1);   // dP - delta
                     fma2g(__uint_as_float(r[c][k0]), __uint_as_float(r[c][k0 + 1]), t0, t1, 0.f, 0.f, ds0, ds1);
                     const __nv_bfloat162 hh = __floats2bfloat162_rn(ds0, ds1);
-                    pk[i + u] = *reinterpret_cast<const uint32_t*>(&hh);
+                    d[0][i + u] = *reinterpret_cast<const uint32_t*>(&hh);   // its own columns or ones already used
                 }
             }
-            tc_st32(my_y, pk);                                            // this group alone has read these columns
+            tc_st32(my_y, d[0]);                                            // this group alone has read these columns
             tc_wait_st();
             tc_fence_before();
             mbar_arrive_(&bars->pb_full);
@@ -966,29 +1006,42 @@ __global__ void __launch_bounds__(FB_THREADS, 1) flash_bwd_kernel(const __grid_c
                 if (it + 1 < n_it) { vdst[(bs ^ 1) * 128] = nx * vmul; mbar_arrive_(&bars->vec_full); }
             }
         }
-        if (ok && !mbar_wait(&bars->done, 0)) { atomicExch(err, 38); ok = false; }
+        more = fb_item<KV>(k + 1, n_hb, nt, H, causal, w);
+        if (more) fetch_first(w);
+        if (ok && !mbar_wait(&bars->done, k & 1)) { atomicExch(err, 38); ok = false; }
+        ok = __all_sync(0xffffffffu, ok);                                // the epilogue synchronises the warp
         if (ok) {
             tc_fence_after();
-            const int64_t grow = (int64_t)row_res + row;
-            // kernel A: group 0 writes dV, group 1 dK; kernel B: each group writes half of the columns of dQ
-            __nv_bfloat16* orow = (KV && g == 1 ? out1 : out0) + grow * ld_out + col0;
+            // kernel A: group 0 writes dV, group 1 dK; kernel B: each group writes half of the columns of dQ.  A warp's 32 rows x 32
+            // columns go through shared memory, so that four lanes store 64 consecutive bytes of a row (a lane per row stored
+            // isolated 16-byte pieces)
+            __nv_bfloat16* obase = (KV && g == 1 ? out1 : out0) + (int64_t)orow0 * ld_out + ocol0;
             const float f = (KV && g == 0) ? 1.f : scale;                 // dV needs no scale; dK and dQ carry the softmax scale
             const uint32_t acc = (KV && g == 1 ? tm_acc1 : tm_acc0) + lane_addr;
             const int c0 = KV ? 0 : g * (HD / 64), c1 = KV ? HD / 32 : c0 + HD / 64;
+            uint8_t* stg = s_stage + (warp - 2) * 32 * FB_STAGE_PITCH;
 #pragma unroll 1
             for (int c = c0; c < c1; ++c) {
                 uint32_t t[32];
                 tc_ld32(acc + c * 32, t);
                 tc_wait_ld();
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
+                for (int u = 0; u < 4; ++u) {
                     uint4 pk;
                     __nv_bfloat162* hh = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) hh[u] = __floats2bfloat162_rn(__uint_as_float(t[8 * k + 2 * u]) * f, __uint_as_float(t[8 * k + 2 * u + 1]) * f);
-                    reinterpret_cast<uint4*>(orow)[c * 4 + k] = pk;
+                    for (int e = 0; e < 4; ++e) hh[e] = __floats2bfloat162_rn(__uint_as_float(t[8 * u + 2 * e]) * f, __uint_as_float(t[8 * u + 2 * e + 1]) * f);
+                    *reinterpret_cast<uint4*>(stg + lane * FB_STAGE_PITCH + u * 16) = pk;
                 }
+                __syncwarp();
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int rr = u * 8 + (lane >> 2), piece = lane & 3;
+                    *reinterpret_cast<uint4*>(obase + rr * ld_out + c * 32 + piece * 8) = *reinterpret_cast<const uint4*>(stg + rr * FB_STAGE_PITCH + piece * 16);
+                }
+                __syncwarp();
             }
+        }
         }
     }
     tc_fence_before();
@@ -1008,7 +1061,7 @@ int launch_bwd(const void* q, const void* k, const void* v, int64_t ld, const vo
     if (!make_map(&mk, k, rows, (int64_t)H * HD, ld, 128, 64, true)) return 12;
     if (!make_map(&mv, v, rows, (int64_t)H * HD, ld, 128, 64, true)) return 13;
     if (!make_map(&md, dout, rows, (int64_t)H * HD, ld_o, 128, 64, true)) return 14;
-    constexpr size_t smem = (size_t)(6 * (HD / 64)) * TILE_HALF_BYTES + 2048 + sizeof(FbBars) + 1024;
+    constexpr size_t smem = (size_t)(6 * (HD / 64)) * TILE_HALF_BYTES + 2048 + FB_STAGE_BYTES + sizeof(FbBars) + 1024;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(flash_bwd_kernel<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 2;
@@ -1018,9 +1071,10 @@ int launch_bwd(const void* q, const void* k, const void* v, int64_t ld, const vo
     count_launch(3);
     flash_delta_kernel<<<(unsigned)((rows * H * (HD / 8) + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, rows, S, H, HD, ld_o, ld_o);
     const int64_t ld_out = (int64_t)H * HD;
-    flash_bwd_kernel<HD, true><<<dim3((S / 128) * H * B), FB_THREADS, smem, st>>>(mq, mk, mv, md, lse, delta, (__nv_bfloat16*)dv, (__nv_bfloat16*)dk, S, H,
+    const int items = (S / 128) * H * B, grid = items < FB_GRID ? items : FB_GRID;
+    flash_bwd_kernel<HD, true><<<grid, FB_THREADS, smem, st>>>(mq, mk, mv, md, lse, delta, (__nv_bfloat16*)dv, (__nv_bfloat16*)dk, S, H, H * B,
                                                                              ld_out, scale, causal ? 1 : 0, err);
-    flash_bwd_kernel<HD, false><<<dim3((S / 128) * H * B), FB_THREADS, smem, st>>>(mq, mk, mv, md, lse, delta, (__nv_bfloat16*)dq, nullptr, S, H, ld_out,
+    flash_bwd_kernel<HD, false><<<grid, FB_THREADS, smem, st>>>(mq, mk, mv, md, lse, delta, (__nv_bfloat16*)dq, nullptr, S, H, H * B, ld_out,
                                                                               scale, causal ? 1 : 0, err);
     return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
