@@ -1,5 +1,5 @@
 // Model-side kernels for the small-sequence transformers of the grokking tasks (sm_100a):
-//   * causal multi-head attention for very short sequences (S <= 8) - one warp per (batch, head), the whole
+//   * causal multi-head attention for very short sequences (S <= 8) - a group of lanes per (batch, head), the whole
 //     S x S score matrix lives in registers; forward and backward (scores recomputed, nothing saved but q,k,v);
 //   * LayerNorm with fused residual add, forward and backward (deterministic two-stage column reduction for
 //     the weight / bias gradients, no atomics).
