@@ -27,37 +27,52 @@ constexpr int SORT_WARPS = SORT_THREADS / 32;
 #endif
 constexpr int SORT_IPT = SG_SORT_IPT;                  // items per thread
 constexpr int SORT_TILE = SORT_THREADS * SORT_IPT;    // 4096 keys per CTA
-constexpr int MAX_SEG = 4096;
+constexpr int MAX_SEG = SORT_TILE;                     // segment offsets that a CTA holds in shared memory
 
-__device__ __forceinline__ int seg_of(uint32_t gidx, const int64_t* __restrict__ seg_off, int n_seg) {
-    int lo = 0, hi = n_seg;                           // seg_off[lo] <= gidx < seg_off[lo+1]
+// Every element of a segment pass looks its segment up: in shared memory, in 32 bits (offsets are below 2^32), as long as the
+// offsets fit there, else in global memory.
+template <typename O>
+__device__ __forceinline__ uint32_t seg_search(uint32_t gidx, const O* tab, int n_seg) {
+    int lo = 0, hi = n_seg;                           // tab[lo] <= gidx < tab[lo+1]
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (seg_off[mid] <= (int64_t)gidx) lo = mid; else hi = mid;
+        if (tab[mid] <= (O)gidx) lo = mid; else hi = mid;
     }
-    return lo;
+    return (uint32_t)lo;
+}
+__device__ __forceinline__ void stage_segs(uint32_t* tab, const int64_t* __restrict__ seg_off, int n_seg) {
+    if (n_seg <= MAX_SEG)
+        for (int i = threadIdx.x; i < n_seg; i += SORT_THREADS) tab[i] = (uint32_t)seg_off[i];
+}
+__device__ __forceinline__ uint32_t seg_of(uint32_t gidx, const uint32_t* tab, const int64_t* __restrict__ seg_off, int n_seg) {
+    return n_seg <= MAX_SEG ? seg_search(gidx, tab, n_seg) : seg_search(gidx, seg_off, n_seg);
 }
 
-// digit of element for this pass: key byte (pass < 4) or segment-id byte (pass >= 4)
-__device__ __forceinline__ uint32_t digit_of(uint32_t key, uint32_t val, int pass, const int64_t* seg_off, int n_seg) {
-    if (pass < 4) return (key >> (8 * pass)) & 0xffu;
-    return ((uint32_t)seg_of(val, seg_off, n_seg) >> (8 * (pass - 4))) & 0xffu;
-}
-
-// warp w of the CTA owns the contiguous range [tile + w*32*IPT, tile + (w+1)*32*IPT); item r of lane l is
-// tile + w*32*IPT + r*32 + l, so (warp, round, lane) order equals index order: ranking in that order is stable.
-__global__ void __launch_bounds__(SORT_THREADS) sort_hist_kernel(const uint32_t* __restrict__ keys,
-                                                                 const uint32_t* __restrict__ vals, uint32_t* __restrict__ hist,
+// Digit counts of one tile.  A key pass reads the keys alone, a segment pass (SEG) the payloads alone; the sixteen loads of a
+// thread are issued before the first count, which would otherwise hold each of them up
+// (18.9 M keys, five passes: 250 -> 144 us; 422,755 keys: 37 -> 17).
+template <bool SEG>
+__global__ void __launch_bounds__(SORT_THREADS) sort_hist_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ hist,
                                                                  const int64_t* __restrict__ seg_off, int n_seg, int64_t total,
-                                                                 int pass, int n_blocks) {
+                                                                 int shift, int n_blocks) {
     __shared__ uint32_t cnt[256];
+    __shared__ uint32_t segs[SEG ? MAX_SEG : 1];
     cnt[threadIdx.x] = 0;
+    if constexpr (SEG) stage_segs(segs, seg_off, n_seg);
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * SORT_TILE;
-    for (int r = 0; r < SORT_IPT; ++r) {
-        const int64_t i = base + (int64_t)r * SORT_THREADS + threadIdx.x;
-        if (i < total) atomicAdd(&cnt[digit_of(keys[i], vals[i], pass, seg_off, n_seg)], 1u);   // integer smem atomics: exact
+    const int64_t base = (int64_t)blockIdx.x * SORT_TILE + threadIdx.x;
+    const int64_t rounds = (total - base + SORT_THREADS - 1) / SORT_THREADS;
+    const int n = (int)(rounds < SORT_IPT ? rounds : SORT_IPT);
+    uint32_t x[SORT_IPT];
+#pragma unroll
+    for (int r = 0; r < SORT_IPT; ++r) x[r] = r < n ? in[base + r * SORT_THREADS] : 0u;
+    if constexpr (SEG) {
+#pragma unroll
+        for (int r = 0; r < SORT_IPT; ++r) x[r] = seg_of(x[r], segs, seg_off, n_seg);
     }
+#pragma unroll
+    for (int r = 0; r < SORT_IPT; ++r)
+        if (r < n) atomicAdd(&cnt[(x[r] >> shift) & 0xffu], 1u);                               // integer smem atomics: exact
     __syncthreads();
     hist[(int64_t)threadIdx.x * n_blocks + blockIdx.x] = cnt[threadIdx.x];
 }
@@ -97,13 +112,20 @@ __global__ void __launch_bounds__(256) sort_scan_rows_kernel(uint32_t* __restric
 // shared memory in their digit order inside the tile; the tile is then written out entry by entry, so that the entries of one
 // digit - which go to consecutive global positions - are stored by consecutive lanes (runs of ~16 keys = 64 bytes instead of
 // isolated 4-byte writes).
+// Warp w of the CTA owns the contiguous range [tile + w*32*IPT, tile + (w+1)*32*IPT); item r of lane l is tile + w*32*IPT + r*32 + l,
+// so (warp, round, lane) order equals index order: ranking in that order is stable.
+// The lanes with an equal digit are found by eight ballots: match_any takes a turn per distinct value (its unit was busy 82 % of the
+// time).  18.9 M keys, a pass over a low key byte 168 -> 126 us, over the segment ids 216 -> 195.  The top key byte holds few values per
+// warp, and match_any stays: 94 us.  The segment search stays inside the ranking loop: all sixteen ahead of it spilled (234 us).
+enum { SORT_KEY_LOW = 0, SORT_KEY_TOP = 1, SORT_SEG = 2 };
+template <int MODE>
 __global__ void __launch_bounds__(SORT_THREADS, SG_SORT_MINB) sort_scatter_kernel(const uint32_t* __restrict__ keys_in,
                                                                     const uint32_t* __restrict__ vals_in,
                                                                     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
                                                                     const uint32_t* __restrict__ hist,
                                                                     const uint32_t* __restrict__ tot,
                                                                     const int64_t* __restrict__ seg_off, int n_seg, int64_t total,
-                                                                    int pass, int n_blocks) {
+                                                                    int shift, int n_blocks) {
     __shared__ uint32_t wcnt[SORT_WARPS][256];        // per-warp running digit counts -> warp bases inside the tile's digit run
     __shared__ uint32_t gbase[256];                   // global position of this tile's first key of digit d
     __shared__ uint32_t tstart[256];                  // position of digit d inside the tile (exclusive scan of the tile's digit counts)
@@ -112,6 +134,7 @@ __global__ void __launch_bounds__(SORT_THREADS, SG_SORT_MINB) sort_scatter_kerne
     __shared__ uint8_t s_dig[SORT_TILE];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < SORT_WARPS * 256; i += SORT_THREADS) (&wcnt[0][0])[i] = 0;
+    if constexpr (MODE == SORT_SEG) stage_segs(s_key, seg_off, n_seg);          // s_key is free until the ranking is done
     {   // digit base = exclusive scan of the 256 digit totals (thread d owns digit d)
         const uint32_t t = tot[threadIdx.x];
         uint32_t inc = t;
@@ -141,9 +164,21 @@ __global__ void __launch_bounds__(SORT_THREADS, SG_SORT_MINB) sort_scatter_kerne
 #pragma unroll
     for (int r = 0; r < SORT_IPT; ++r) {
         const bool ok = wbase + r * 32 + lane < total;
-        d[r] = ok ? digit_of(k[r], v[r], pass, seg_off, n_seg) : 0xffffffffu;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d[r]);
-        const int leader = __ffs(peers) - 1;
+        if constexpr (MODE == SORT_SEG) d[r] = (seg_of(v[r], s_key, seg_off, n_seg) >> shift) & 0xffu;
+        else d[r] = (k[r] >> shift) & 0xffu;
+        // the lanes of this round with the same digit (of no interest to a lane past the end)
+        uint32_t peers = __ballot_sync(0xffffffffu, ok);
+        if constexpr (MODE == SORT_KEY_TOP) {
+            peers &= __match_any_sync(0xffffffffu, d[r]);
+        } else {
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                const bool bit = (d[r] >> b) & 1u;
+                const uint32_t set = __ballot_sync(0xffffffffu, bit);
+                peers &= bit ? set : ~set;
+            }
+        }
+        const int leader = (__ffs(peers) - 1) & 31;
         uint32_t prior = 0;
         if (ok && lane == leader) { prior = wcnt[w][d[r]]; wcnt[w][d[r]] = prior + __popc(peers); }
         prior = __shfl_sync(0xffffffffu, prior, leader);
@@ -203,10 +238,11 @@ void sg2_segmented_sort(uint32_t* keys0, uint32_t* keys1, uint32_t* vals0, uint3
         for (int x = n_seg - 1; x > 0; x >>= 8) ++seg_passes;     // bytes needed for the largest segment id
         for (int pass = 0; pass < 4 + seg_passes; ++pass) {
             count_launch(3);
-            sort_hist_kernel<<<nb, SORT_THREADS, 0, s>>>(k[cur], v[cur], hist, seg_offsets_dev, n_seg, total, pass, nb);
+            if (pass < 4) sort_hist_kernel<false><<<nb, SORT_THREADS, 0, s>>>(k[cur], hist, seg_offsets_dev, n_seg, total, 8 * pass, nb);
+            else sort_hist_kernel<true><<<nb, SORT_THREADS, 0, s>>>(v[cur], hist, seg_offsets_dev, n_seg, total, 8 * (pass - 4), nb);
             sort_scan_rows_kernel<<<256, 256, 0, s>>>(hist, tot, nb);
-            sort_scatter_kernel<<<nb, SORT_THREADS, 0, s>>>(k[cur], v[cur], k[cur ^ 1], v[cur ^ 1], hist, tot, seg_offsets_dev,
-                                                            n_seg, total, pass, nb);
+            auto scatter = pass < 3 ? sort_scatter_kernel<SORT_KEY_LOW> : pass == 3 ? sort_scatter_kernel<SORT_KEY_TOP> : sort_scatter_kernel<SORT_SEG>;
+            scatter<<<nb, SORT_THREADS, 0, s>>>(k[cur], v[cur], k[cur ^ 1], v[cur ^ 1], hist, tot, seg_offsets_dev, n_seg, total, 8 * (pass & 3), nb);
             cur ^= 1;
         }
     }
