@@ -25,6 +25,15 @@ from .metanet import Mamba3PEERMetaNet
 from .supergrok15 import SuperGrok15
 
 
+def _copies(named_tensors):
+    """{name: copy}; dense tensors share the launches of one foreach copy."""
+    out = {n: torch.empty_like(t) if t.layout == torch.strided else t.clone() for n, t in named_tensors}
+    dense = [(out[n], t) for n, t in named_tensors if t.layout == torch.strided]
+    if dense:
+        torch._foreach_copy_([d for d, _ in dense], [t for _, t in dense])
+    return out
+
+
 class SuperGrok2(SuperGrok15):
     def __init__(self, params, lr=1e-3, betas=(0.9, 0.999), eps=1e-8, weight_decay=1.0, alpha_init=0.98, lamb=2.0,
                  gamma=0.1, gamma_alpha=0.0, kappa=0.1, warmup_steps=100, warmup_ramp=100, gradient_clipping=1.0,
@@ -150,13 +159,14 @@ class SuperGrok2(SuperGrok15):
         (reference supergrok2.py:516-1330); tensors with non-finite validation gradients are skipped."""
         self._ensure_state()
         named = list(model.named_parameters())
-        # the training gradients step aside (and come back as the same tensors) while the validation gradients take their place: no copies
-        saved = {n: p.grad for n, p in named if p.grad is not None}
-        if not saved:
+        # A backward may fill the storage that .grad already has (buckets of a distributed wrapper, buffers of a captured graph), so the
+        # training gradients are copied before the validation backward: all of them in one foreach call.
+        grads = [(n, p.grad.detach()) for n, p in named if p.grad is not None]
+        if not grads:
             return 0.0
+        saved = _copies(grads)
         try:
-            for _, p in named:
-                p.grad = None
+            model.zero_grad()
             with torch.enable_grad():
                 val_loss = criterion(model(val_x), val_y)
                 val_loss.backward()
