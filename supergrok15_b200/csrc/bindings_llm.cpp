@@ -266,13 +266,16 @@ struct RopeNode : Function<RopeNode> {
 struct FlashNode : Function<FlashNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, bool causal, const Tensor& err) {
         auto r = flash_fwd(q, k, v, causal, err, 3);
-        ctx->save_for_backward({q, k, v, r[0], r[1], err});
+        ctx->save_for_backward({q, k, v, r[0], r[1]});
+        // the process's time-out flag itself, not a saved tensor: hooks that pack those would hand the backward a copy that nobody reads,
+        // and the check that clears the flag would count as an in-place change
+        ctx->saved_data["err"] = err;
         ctx->saved_data["causal"] = causal;
         return r[0];
     }
     static variable_list backward(AutogradContext* ctx, variable_list dy) {
         const auto s = ctx->get_saved_variables();
-        auto r = flash_bwd(s[0], s[1], s[2], s[3], s[4], dy[0], ctx->saved_data["causal"].toBool(), s[5]);
+        auto r = flash_bwd(s[0], s[1], s[2], s[3], s[4], dy[0], ctx->saved_data["causal"].toBool(), ctx->saved_data["err"].toTensor());
         return {r[0], r[1], r[2], Tensor(), Tensor()};
     }
 };

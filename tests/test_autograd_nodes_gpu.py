@@ -99,3 +99,22 @@ def test_in_place_changes_second_backward_and_transforms():
     with nn_ops.grad_sink(True):
         seen.append(nn_ops._cpp_node(x))
     assert seen == [False, False, False]
+
+
+def test_flash_backward_gets_the_time_out_flag_itself():
+    """The flag is no saved tensor: packing hooks do not see it, and a check that clears it between forward and backward is no in-place change."""
+    from supergrok15_b200.ops import gemm
+    fn, args = _ops()["flash"]
+    _, want = _run(fn, args)
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t.dtype) or t, lambda t: t):
+        out = fn(*args)
+    flag = gemm._err_flag(args[0].device)
+    version = flag._version
+    flag.zero_()
+    got = torch.autograd.grad(out, args, torch.full_like(out, 0.5))
+    assert torch.int32 not in packed and flag._version == version + 1
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    out = fn(*args)
+    flag.zero_()                                           # without hooks
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(out, args, torch.full_like(out, 0.5)), want))
