@@ -1,4 +1,6 @@
 // Bindings of the model-side kernels (short-sequence attention, LayerNorm with residual).
+#include <ATen/TensorSubclassLikeUtils.h>
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include "bindings_decl.h"
@@ -151,9 +153,37 @@ struct AttnSmallNode : Function<AttnSmallNode> {
         return {attn_small_bwd(ctx->get_saved_variables()[0], dy[0], ctx->saved_data["heads"].toInt(), ctx->saved_data["causal"].toBool()), Tensor(), Tensor()};
     }
 };
+
+// F.linear whose bias gradient is the two-stage column sum.  Backwards that are differentiated again, batched over gradients, or looked at by
+// a dispatch mode take PyTorch's own sum, as does a gradient whose columns are not adjacent.
+struct LinearNode : Function<LinearNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const Tensor& bias) {
+        ctx->save_for_backward({x, weight});
+        return at::linear(x, weight, bias);
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list dy) {
+        const auto s = ctx->get_saved_variables();
+        const Tensor &x = s[0], &weight = s[1];
+        Tensor dy2 = dy[0].reshape({-1, weight.size(0)}), db;
+        if (ctx->needs_input_grad(2))
+            db = at::GradMode::is_enabled() || at::isTensorSubclassLike(dy2) || dy2.stride(1) != 1 ? dy2.sum(0) : col_sum(dy2, c10::nullopt);
+        return {ctx->needs_input_grad(0) ? dy2.mm(weight).view(x.sizes()) : Tensor(),
+                ctx->needs_input_grad(1) ? dy2.t().mm(x.reshape({-1, x.size(-1)})) : Tensor(), db};
+    }
+};
+
+bool linear_node_takes(const Tensor& x, const Tensor& weight, const Tensor& bias) {
+    for (const Tensor* t : {&x, &weight, &bias})
+        if (t->is_nested() || t->layout() != at::kStrided || t->scalar_type() != x.scalar_type()) return false;
+    const auto dt = x.scalar_type();
+    return (dt == at::kFloat || dt == at::kBFloat16 || dt == at::kHalf) && at::GradMode::is_enabled() && bias.requires_grad() && x.dim() >= 2 && x.size(-1) > 0 &&
+           weight.dim() == 2 && weight.size(0) > 0 && bias.dim() == 1 && bias.size(0) == weight.size(0) && !at::autocast::is_autocast_enabled(at::kCUDA);
+}
 }  // namespace
 
 void register_nn(pybind11::module_& m) {
+    m.def("linear_node_takes", &linear_node_takes);
+    m.def("linear_node", [](const Tensor& x, const Tensor& weight, const Tensor& bias) { return LinearNode::apply(x, weight, bias); });
     m.def("norm_node", [](const Tensor& x, const c10::optional<Tensor>& residual, const Tensor& weight, const c10::optional<Tensor>& bias, double eps, bool rms) {
         return NormNode::apply(x, residual, weight, bias, eps, rms, false)[0];
     });

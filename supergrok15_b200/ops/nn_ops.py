@@ -200,39 +200,18 @@ def _param_grads(gw, gb, dy2, x2, tc=False):
             gb.add_(dy2.sum(0))
 
 
-class _LinearColSum(torch.autograd.Function):
-    """F.linear whose bias gradient is the two-stage column sum of ``csrc/nn_kernels.cu``."""
-
-    @staticmethod
-    def forward(ctx, x, weight, bias):
-        ctx.save_for_backward(x, weight)
-        return F.linear(x, weight, bias)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, weight = ctx.saved_tensors
-        dy2 = dy.reshape(-1, dy.shape[-1])
-        dx = (dy2 @ weight).view(x.shape) if ctx.needs_input_grad[0] else None
-        dw = dy2.t() @ x.reshape(-1, x.shape[-1]) if ctx.needs_input_grad[1] else None
-        if torch.is_grad_enabled() or dy2.stride(-1) != 1:              # create_graph: every step has to be differentiable
-            return dx, dw, dy2.sum(0)
-        return dx, dw, _build.require().col_sum(dy2)
-
-
 # Rows from which the own column sum is used.  PyTorch's reduction over the rows of a [32768, 512 .. 2048] bf16 gradient takes 30 to 60 us
 # (1.1 ms of a 7.2 ms pass of the 6-layer d512 model), the column sum 8 to 25 us; below a few thousand rows both are a few
-# microseconds and the plain call costs the host less.
+# microseconds.
 _COL_SUM_ROWS = 4096
 
 
 def _col_sum_bias(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor]) -> bool:
-    """Whether ``_LinearColSum`` stands in for F.linear: eager CUDA training of a layer whose bias needs a gradient, outside of autocast,
-    of functorch transforms, of forward-mode AD and of tracing, all of which have to see F.linear itself."""
-    if bias is None or not (x.is_cuda and bias.requires_grad and torch.is_grad_enabled()) or x.dim() < 2 or weight.dim() != 2:
-        return False
-    if x.dtype not in (torch.float32, torch.bfloat16, torch.float16) or x.dtype != weight.dtype or x.dtype != bias.dtype or x.numel() < _COL_SUM_ROWS * x.shape[-1]:
-        return False
-    return x.shape[-1] > 0 and not torch.is_autocast_enabled("cuda") and _cpp_node(x, weight, bias)
+    """Whether the C++ node whose bias gradient is the column sum of ``csrc/nn_kernels.cu`` stands in for F.linear: eager CUDA training of a
+    layer with dense [out, in] weights and an [out] bias that needs a gradient, outside of autocast, of functorch transforms, of
+    forward-mode AD and of tracing, all of which have to see F.linear itself."""
+    return (bias is not None and x.is_cuda and not x.is_nested and x.numel() >= _COL_SUM_ROWS * weight.shape[-1] and _cpp_node(x, weight, bias) and
+            _build.require().linear_node_takes(x, weight, bias))
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -244,7 +223,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         from . import gemm
         return gemm.linear(x, weight, bias)
     if _col_sum_bias(x, weight, bias):
-        return _LinearColSum.apply(x, weight, bias)
+        return _build.require().linear_node(x, weight, bias)
     return F.linear(x, weight, bias)
 
 

@@ -41,3 +41,24 @@ def test_other_calls_stay_with_the_library():
     (gr,) = torch.autograd.grad(F.linear(x, w, b).square().sum(), x, create_graph=True)
     for a, c in zip(got, torch.autograd.grad(gr.square().sum(), (w, b))):
         assert torch.allclose(a, c, rtol=1e-4, atol=1e-3 * float(c.abs().max()))
+
+
+def test_forms_that_the_library_takes():
+    """A bias with a leading dimension of one, a layer without outputs, gradients of several output gradients at once, and a frozen bias's
+    neighbours: same results as F.linear."""
+    x, w = (torch.randn(s, device="cuda", requires_grad=True) for s in ((2, 2100, 16), (8, 16)))
+    for b in (torch.randn(1, 8, device="cuda", requires_grad=True), torch.randn(8, device="cuda", requires_grad=True)):
+        dy = torch.randn(3, 2, 2100, 8, device="cuda")
+        y, ref = nn_ops.linear(x, w, b), F.linear(x, w, b)
+        for wanted in ((x, w, b), (b,), (w,)):
+            got = torch.autograd.grad(y, wanted, dy[0], retain_graph=True)
+            for a, c in zip(got, torch.autograd.grad(ref, wanted, dy[0], retain_graph=True)):
+                assert a.shape == c.shape
+                torch.testing.assert_close(a, c, rtol=1e-5, atol=1e-5 * float(c.abs().max()))        # fp32 sums of 4,200 terms in another order
+        got = torch.autograd.grad(y, (x, w, b), dy, is_grads_batched=True)
+        for a, c in zip(got, torch.autograd.grad(ref, (x, w, b), dy, is_grads_batched=True)):
+            torch.testing.assert_close(a, c, rtol=1e-5, atol=1e-5 * float(c.abs().max()))
+    w0, b0 = torch.zeros(0, 16, device="cuda", requires_grad=True), torch.zeros(0, device="cuda", requires_grad=True)
+    gx, gw, gb = torch.autograd.grad(nn_ops.linear(x, w0, b0).sum(), (x, w0, b0))
+    assert gw.shape == w0.shape and gb.shape == b0.shape and not gx.any()
+    assert not nn_ops._col_sum_bias(x, w0, b0) and nn_ops._col_sum_bias(x, w, torch.zeros(8, device="cuda", requires_grad=True))
