@@ -39,7 +39,9 @@ __global__ void __launch_bounds__(128) experts_table_kernel(const float* __restr
                                                             const float* __restrict__ b2, int E, float* __restrict__ table) {
     const int e_raw = blockIdx.x * 8 + (threadIdx.x >> 4), j = threadIdx.x & 15;
     const int e = e_raw < E ? e_raw : E - 1;                          // whole warps take part in the shuffles
-    const float w1 = W1[e * XH + j], b = b1[e * XH + j], w2 = W2[e * XH + j];
+    float w1 = W1[e * XH + j], b = b1[e * XH + j];
+    const float w2 = W2[e * XH + j];
+    if (isnan(w1) || isnan(b)) w1 = b = 0.f;                           // such a unit is off, as fmaxf(NaN, 0) makes it; the ranks below have to be distinct
     const float t = w1 != 0.f ? -b / w1 : INFINITY;
     int rank = 0;
     for (int k = 0; k < XH; ++k) {

@@ -131,6 +131,30 @@ def test_routed_experts_kernel_matches_dense_formulation(n, heads, E, pk):
         assert torch.equal(a, b)                                                                  # fixed summation order
 
 
+def _routing(n, heads, pk, seed):
+    torch.manual_seed(seed)
+    ia, ib = (torch.rand(n, heads, pk, device="cuda").topk(4, dim=-1).indices.int() for _ in range(2))
+    wa, wb = (torch.softmax(torch.randn(n, heads, 4, device="cuda"), -1) for _ in range(2))
+    return ia, ib, wa, wb
+
+
+def test_routed_experts_with_nan_units_read_written_words_only():
+    """A unit whose weight or bias is NaN is off: the values are those of the experts without it, whatever memory the tables are put in."""
+    from supergrok15_b200.ops import sg2_bilevel
+    n, heads, E, pk = 4000, 4, 144, 12
+    ia, ib, wa, wb = _routing(n, heads, pk, 3)
+    g = torch.randn(n, device="cuda")
+    W1, b1, W2 = (torch.randn(E, 16, device="cuda") for _ in range(3))
+    b2 = torch.randn(E, device="cuda")
+    off = torch.rand(E, 16, device="cuda") < 0.3
+    nan_w = off & (torch.rand(E, 16, device="cuda") < 0.5)
+    dirty = [torch.full((1 << 16,), v, device="cuda") for v in (float("-inf"), 0.5, -0.25)]       # what the allocator hands to the tables next
+    del dirty
+    got = sg2_bilevel.routed_experts(g, ia, ib, wa, wb, W1.masked_fill(nan_w, float("nan")), b1.masked_fill(off & ~nan_w, float("nan")), W2, b2, pk)
+    want = sg2_bilevel.routed_experts(g, ia, ib, wa, wb, W1.masked_fill(off, 0.0), b1.masked_fill(off, 0.0), W2, b2, pk)
+    assert torch.equal(got, want)
+
+
 def test_soft_head_expert_kernel_matches_dense_path(monkeypatch):
     opt, named, tg, vg = _setup([(3000,)])
     mn = opt.meta_net
