@@ -25,14 +25,15 @@ constexpr int XE = 16 * XMAXQ;    // row pitch of the dense routing table (colum
 constexpr int XSEG = XH + 1;      // linear pieces of an expert = row pitch of its tables (odd: different experts fall into different banks)
 
 // An expert is a piecewise linear function of the scalar g: hidden unit j switches at t_j = -b1_j / W1_j.  The tables hold the sorted
-// switching points and, per piece, slope and intercept (summed in fp64), so that a value takes five comparisons, an FMA and an addition
-// instead of 16 hidden units with three table words each; both forms were bound by the shared-memory reads (54 against 7 per value).
-// The intercept is kept as a rounded value and its remainder: its rounding error would be the same for all elements of a piece and would
-// not average out of the sums over them (gradients of the keys, which live on differences of expert values).
-// The indicator of a unit (for the parameter gradients) is still evaluated from its own weights: at a switching point the value does
-// not care on which side it is taken, a derivative would.
-struct XTable { const float* t; const float* hi; const float2* ab; };                                    // ab: slope, remainder of the intercept
-size_t __host__ __device__ constexpr x_table_floats(int E) { return (size_t)E * XSEG * 4; }
+// switching points and, per piece, slope and intercept (summed in fp64), so that a value takes five comparisons and a compensated
+// multiply-add instead of 16 hidden units with three table words each; both forms were bound by the shared-memory reads (54 against 9
+// per value).
+// slope * g and the intercept cancel where g lies near the switching points of the units that are on (each unit then has a
+// small value, which 16 separate units would round relative to itself).  So slope and intercept are pairs of floats (value and remainder) and the
+// product and the sum keep their rounding errors: what is lost is 2^-47 of |slope * g|.  The switching points are rounded towards
+// -infinity: for every float g, g > t_j then decides exactly as the sign of g * W1_j + b1_j does.
+struct XTable { const float4* v; const float* t; };                                                     // v: slope, its remainder, intercept, its remainder
+size_t __host__ __device__ constexpr x_table_floats(int E) { return (size_t)E * XSEG * 5; }
 
 // sixteen lanes per expert: lane j ranks its switching point, lane s sums piece s (lane 0 also piece 16)
 __global__ void __launch_bounds__(128) experts_table_kernel(const float* __restrict__ W1, const float* __restrict__ b1, const float* __restrict__ W2,
@@ -42,15 +43,14 @@ __global__ void __launch_bounds__(128) experts_table_kernel(const float* __restr
     float w1 = W1[e * XH + j], b = b1[e * XH + j];
     const float w2 = W2[e * XH + j];
     if (isnan(w1) || isnan(b)) w1 = b = 0.f;                           // such a unit is off, as fmaxf(NaN, 0) makes it; the ranks below have to be distinct
-    const float t = w1 != 0.f ? -b / w1 : INFINITY;
+    const float t = w1 != 0.f ? __fdiv_rd(-b, w1) : INFINITY;
     int rank = 0;
     for (int k = 0; k < XH; ++k) {
         const float tk = __shfl_sync(0xffffffffu, t, k, 16);
         rank += (tk < t || (tk == t && k < j)) ? 1 : 0;
     }
-    float* th = table + (size_t)e * XSEG;
-    float* hi = table + ((size_t)E + e) * XSEG;
-    float2* ab = reinterpret_cast<float2*>(table + 2 * (size_t)E * XSEG) + (size_t)e * XSEG;
+    float4* val = reinterpret_cast<float4*>(table) + (size_t)e * XSEG;
+    float* th = table + 4 * (size_t)E * XSEG + (size_t)e * XSEG;
     if (e_raw < E) th[rank] = t;
     const double base = (double)b2[e];
     for (int rep = 0; rep < 2; ++rep) {
@@ -61,14 +61,17 @@ __global__ void __launch_bounds__(128) experts_table_kernel(const float* __restr
             const int kr = __shfl_sync(0xffffffffu, rank, k, 16);
             const bool on = kw1 > 0.f ? kr < s : kw1 < 0.f ? kr >= s : kb > 0.f;
             if (on) { slope += (double)kw2 * kw1; icept += (double)kw2 * kb; }
+            else icept += 0.0 * kw2;                                   // a non-finite W2 shows, as it does in the sum over the units
         }
-        if (e_raw < E && (rep == 0 || j == 0)) { hi[s] = (float)icept; ab[s] = make_float2((float)slope, (float)(icept - (double)(float)icept)); }
+        const float sh = (float)slope, ih = (float)icept;
+        if (e_raw < E && (rep == 0 || j == 0))
+            val[s] = make_float4(sh, isfinite(sh) ? (float)(slope - sh) : 0.f, ih, isfinite(ih) ? (float)(icept - ih) : 0.f);
     }
 }
 
 __device__ __forceinline__ XTable load_table(float* sm, const float* __restrict__ table, int E) {
     for (int i = threadIdx.x; i < (int)x_table_floats(E); i += XTHREADS) sm[i] = table[i];
-    return XTable{sm, sm + E * XSEG, reinterpret_cast<const float2*>(sm + 2 * E * XSEG)};
+    return XTable{reinterpret_cast<const float4*>(sm), sm + 4 * E * XSEG};
 }
 
 __device__ __forceinline__ float expert_eval(const XTable& p, int e, float g) {
@@ -78,8 +81,12 @@ __device__ __forceinline__ float expert_eval(const XTable& p, int e, float g) {
     s += g > t[s + 1] ? 2 : 0;
     s += g > t[s] ? 1 : 0;
     s += g > t[s] ? 1 : 0;
-    const float2 ab = p.ab[e * XSEG + s];
-    return fmaf(ab.x, g, ab.y) + p.hi[e * XSEG + s];
+    const float4 v = p.v[e * XSEG + s];
+    const float m = __fmul_rn(v.x, g), me = fmaf(v.x, g, -m);                       // m + me = slope * g
+    const float q = __fadd_rn(m, v.z), w = __fsub_rn(q, m);
+    const float qe = __fadd_rn(__fsub_rn(m, __fsub_rn(q, w)), __fsub_rn(v.z, w));    // q + qe = m + intercept
+    const float r = q + ((me + qe) + fmaf(v.y, g, v.w));
+    return r == r ? r : fmaf(v.x, g, v.z);                                          // past the range of floats: no inf - inf of the error terms
 }
 
 __device__ __forceinline__ int expert_of(int a, int b, int pk, int E) {
@@ -92,7 +99,7 @@ __global__ void __launch_bounds__(XTHREADS) routed_experts_fwd_kernel(const floa
                                                                       const int4* __restrict__ ib, const float4* __restrict__ wa,
                                                                       const float4* __restrict__ wb, const float* __restrict__ table,
                                                                       int64_t n, int heads, int E, int pk, float* __restrict__ total) {
-    extern __shared__ __align__(8) float sm[];
+    extern __shared__ __align__(16) float sm[];
     const XTable p = load_table(sm, table, E);
     float* s_tot = sm + x_table_floats(E);
     __syncthreads();
@@ -131,7 +138,7 @@ __global__ void __launch_bounds__(XTHREADS, 2) routed_experts_bwd_kernel(const f
                                                                       const float* __restrict__ table, const float* __restrict__ dtotal,
                                                                       int64_t n, int heads, int E, int pk, float4* __restrict__ dwa,
                                                                       float4* __restrict__ dwb, float* __restrict__ partial) {
-    extern __shared__ __align__(8) float sm[];
+    extern __shared__ __align__(16) float sm[];
     const XTable p = load_table(sm, table, E);
     const int epc = XTHREADS / heads;
     float* s_g = sm + x_table_floats(E);                                // [epc]

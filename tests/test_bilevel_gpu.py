@@ -155,6 +155,43 @@ def test_routed_experts_with_nan_units_read_written_words_only():
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("where", ["spread", "near", "on", "equal", "no_slope"])
+def test_routed_experts_values_at_switching_points(where):
+    """Switching points around, close to and on the gradients, several units with the same one, units without a slope: every value as
+    accurate as the sum over the hidden units, whose terms are each rounded relative to themselves."""
+    from supergrok15_b200.ops import sg2_bilevel
+    n, heads, E, pk = 6000, 4, 144, 12
+    ia, ib, wa, wb = _routing(n, heads, pk, 7)
+    g0 = 0.37
+    g = torch.randn(n, device="cuda") if where == "spread" else g0 * (1 + 1e-3 * torch.randn(n, device="cuda"))
+    W1, b1, W2 = (torch.randn(E, 16, device="cuda") for _ in range(3))
+    b2 = torch.zeros(E, device="cuda")
+    if where != "spread":
+        at = {"near": g0 * (1 + 1e-3 * torch.randn(E, 16, device="cuda")), "on": g[torch.randint(0, n, (E, 16), device="cuda")],
+              "equal": g[torch.randint(0, n, (E, 1), device="cuda")].expand(E, 16), "no_slope": torch.full((E, 16), g0, device="cuda")}[where]
+        if where == "on":                                   # powers of two, so that -b1 / W1 is the gradient itself
+            W1 = torch.sign(W1) * torch.exp2(torch.randint(-3, 4, (E, 16), device="cuda").float())
+        b1 = -W1 * at
+    if where == "no_slope":
+        none = torch.rand(E, 16, device="cuda") < 0.5
+        W1, b1 = W1.masked_fill(none, 0.0), torch.where(none, 1e-3 * torch.randn(E, 16, device="cuda"), b1)
+    d = [t.double() for t in (g, wa, wb, W1, b1, W2, b2)]
+    want = _dense_routed(d[0], ia.long(), ib.long(), *d[1:], pk)
+    size = _dense_routed(d[0], ia.long(), ib.long(), *d[1:5], d[5].abs(), d[6].abs(), pk)              # sum of the magnitudes of all terms
+    parts = _dense_routed(d[0].abs(), ia.long(), ib.long(), d[1], d[2], d[3].abs(), d[4].abs(), d[5].abs(), d[6].abs(), pk)   # |W1 g| and |b1| apart
+    got = sg2_bilevel.routed_experts(g, ia, ib, wa, wb, W1, b1, W2, b2, pk)
+    # a chain of 16 values and one of 4 heads, each term with a few roundings: well below 64 units of the magnitudes; the pairs of floats
+    # hold slope and intercept to 2^-47
+    assert bool(((got.double() - want).abs() <= 64 * 2.0 ** -24 * size + 2.0 ** -44 * parts).all())
+    dt = torch.randn(n, device="cuda")
+    gwa, = torch.autograd.grad(sg2_bilevel.routed_experts(g, ia, ib, wa.requires_grad_(), wb, W1, b1, W2, b2, pk), wa, dt)
+    dwa = d[1].requires_grad_()
+    ref, = torch.autograd.grad(_dense_routed(d[0], ia.long(), ib.long(), dwa, *d[2:], pk), dwa, dt.double())
+    mag, = torch.autograd.grad(_dense_routed(d[0], ia.long(), ib.long(), dwa, *d[2:5], d[5].abs(), d[6].abs(), pk), dwa, dt.double().abs())
+    raw, = torch.autograd.grad(_dense_routed(d[0].abs(), ia.long(), ib.long(), dwa, d[2], d[3].abs(), d[4].abs(), d[5].abs(), d[6].abs(), pk), dwa, dt.double().abs())
+    assert bool(((gwa.double() - ref).abs() <= 64 * 2.0 ** -24 * mag + 2.0 ** -44 * raw).all())
+
+
 def test_soft_head_expert_kernel_matches_dense_path(monkeypatch):
     opt, named, tg, vg = _setup([(3000,)])
     mn = opt.meta_net
