@@ -12,15 +12,22 @@
 namespace sg {
 namespace {
 
-// EPL consecutive head-dim elements owned by one lane, held as loaded (packed) until they are used
-template <typename T, int EPL> struct LaneVec {
+// EPL consecutive head-dim elements owned by one lane, held as loaded (packed) until they are used.  VEC: one access of EPL elements,
+// which has to be aligned to its size; otherwise element by element.
+template <typename T, int EPL, bool VEC> struct LaneVec {
     static constexpr int W = (EPL * (int)sizeof(T) + 3) / 4;           // 32-bit words (one half-filled for a single 16-bit element)
+    static_assert(!VEC || W == 2 || W == 4, "accesses of 8 or 16 bytes");
     uint32_t w[W];
     __device__ __forceinline__ void ld(const T* p) {
-        if constexpr (W == 4) { const uint4 t = *reinterpret_cast<const uint4*>(p); w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w; }
-        else if constexpr (W == 2) { const uint2 t = *reinterpret_cast<const uint2*>(p); w[0] = t.x; w[1] = t.y; }
-        else if constexpr (EPL * sizeof(T) == 4) w[0] = *reinterpret_cast<const uint32_t*>(p);
-        else w[0] = *reinterpret_cast<const uint16_t*>(p);
+        if constexpr (!VEC && sizeof(T) == 4) {
+#pragma unroll
+            for (int e = 0; e < EPL; ++e) w[e] = reinterpret_cast<const uint32_t*>(p)[e];
+        } else if constexpr (!VEC) {
+            const uint16_t* h = reinterpret_cast<const uint16_t*>(p);
+#pragma unroll
+            for (int k = 0; k < W; ++k) w[k] = h[2 * k] | (2 * k + 1 < EPL ? (uint32_t)h[2 * k + 1] << 16 : 0u);
+        } else if constexpr (W == 4) { const uint4 t = *reinterpret_cast<const uint4*>(p); w[0] = t.x; w[1] = t.y; w[2] = t.z; w[3] = t.w; }
+        else { const uint2 t = *reinterpret_cast<const uint2*>(p); w[0] = t.x; w[1] = t.y; }
     }
     __device__ __forceinline__ float get(int e) const {
         if constexpr (sizeof(T) == 4) return __uint_as_float(w[e]);
@@ -30,10 +37,11 @@ template <typename T, int EPL> struct LaneVec {
         T h[EPL];
 #pragma unroll
         for (int e = 0; e < EPL; ++e) h[e] = Cvt<T>::from(v[e]);
-        if constexpr (W == 4) *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(h);
-        else if constexpr (W == 2) *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(h);
-        else if constexpr (EPL * sizeof(T) == 4) *reinterpret_cast<uint32_t*>(p) = *reinterpret_cast<const uint32_t*>(h);
-        else *p = h[0];
+        if constexpr (!VEC) {
+#pragma unroll
+            for (int e = 0; e < EPL; ++e) p[e] = h[e];
+        } else if constexpr (W == 4) *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(h);
+        else *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(h);
     }
 };
 // sum over the LG lanes (aligned group) of one head; every lane gets the result
@@ -46,7 +54,7 @@ template <int LG> __device__ __forceinline__ float group_sum(float x) {
 // qkv [B, S, 3, H, HD], out [B, S, H, HD]; scale = 1/sqrt(HD).  HD / EPL lanes per (b, h): with sixteen bytes per lane a warp holds four heads
 // of 64 bf16, a load instruction moves 512 bytes and one shuffle step of a score serves all four (a warp per head loaded four bytes per
 // lane and spent 50 shuffles on ten scores: 37 us forward and 64 us backward for [8192, 4, 3 x 512] bf16, 134 and 235 MB).
-template <typename T, int S, int EPL, int HD, bool CAUSAL>
+template <typename T, int S, int EPL, int HD, bool CAUSAL, bool VEC>
 __global__ void __launch_bounds__(128) attn_small_fwd_kernel(const T* __restrict__ qkv, T* __restrict__ out, int B, int H, float scale) {
     constexpr int LG = HD / EPL, PER_CTA = 128 / LG;
     const int64_t w0 = (int64_t)blockIdx.x * PER_CTA + threadIdx.x / LG;
@@ -54,7 +62,7 @@ __global__ void __launch_bounds__(128) attn_small_fwd_kernel(const T* __restrict
     const int64_t w = live ? w0 : 0;
     const int b = (int)(w / H), h = (int)(w % H), l = threadIdx.x % LG;
     const int64_t D = (int64_t)H * HD;
-    LaneVec<T, EPL> q[S], k[S], v[S];
+    LaneVec<T, EPL, VEC> q[S], k[S], v[S];
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         const T* base = qkv + ((int64_t)b * S + s) * 3 * D + (int64_t)h * HD + l * EPL;
@@ -89,11 +97,11 @@ __global__ void __launch_bounds__(128) attn_small_fwd_kernel(const T* __restrict
 #pragma unroll
             for (int e = 0; e < EPL; ++e) o[e] = fmaf(sc[i][j] * inv, v[j].get(e), o[e]);
         }
-        if (live) LaneVec<T, EPL>::st(out + ((int64_t)b * S + i) * D + (int64_t)h * HD + l * EPL, o);
+        if (live) LaneVec<T, EPL, VEC>::st(out + ((int64_t)b * S + i) * D + (int64_t)h * HD + l * EPL, o);
     }
 }
 
-template <typename T, int S, int EPL, int HD, bool CAUSAL>
+template <typename T, int S, int EPL, int HD, bool CAUSAL, bool VEC>
 __global__ void __launch_bounds__(128) attn_small_bwd_kernel(const T* __restrict__ qkv, const T* __restrict__ dout, T* __restrict__ dqkv,
                                                              int B, int H, float scale) {
     constexpr int LG = HD / EPL, PER_CTA = 128 / LG;
@@ -102,7 +110,7 @@ __global__ void __launch_bounds__(128) attn_small_bwd_kernel(const T* __restrict
     const int64_t w = live ? w0 : 0;
     const int b = (int)(w / H), h = (int)(w % H), l = threadIdx.x % LG;
     const int64_t D = (int64_t)H * HD;
-    LaneVec<T, EPL> q[S], k[S], v[S], dO[S];
+    LaneVec<T, EPL, VEC> q[S], k[S], v[S], dO[S];
 #pragma unroll
     for (int s = 0; s < S; ++s) {
         const T* base = qkv + ((int64_t)b * S + s) * 3 * D + (int64_t)h * HD + l * EPL;
@@ -155,7 +163,7 @@ __global__ void __launch_bounds__(128) attn_small_bwd_kernel(const T* __restrict
                 for (int e = 0; e < EPL; ++e) { dv[e] = fmaf(p[t][s], dO[t].get(e), dv[e]); dk[e] = fmaf(dp[t][s], q[t].get(e), dk[e]); }
             }
         }
-        if (live) { LaneVec<T, EPL>::st(base, dq); LaneVec<T, EPL>::st(base + D, dk); LaneVec<T, EPL>::st(base + 2 * D, dv); }
+        if (live) { LaneVec<T, EPL, VEC>::st(base, dq); LaneVec<T, EPL, VEC>::st(base + D, dk); LaneVec<T, EPL, VEC>::st(base + 2 * D, dv); }
     }
 }
 
@@ -616,19 +624,19 @@ static void attn_dispatch(bool bwd, const T* qkv, const T* dout, T* out, int B, 
     const float scale = 1.f / sqrtf((float)HD);
     if ((int64_t)B * H == 0) return;
     count_launch();
-#define GO(SV, EV, HV, CV) { \
+#define GO(SV, EV, HV, CV, VV) { \
     const unsigned blocks = (unsigned)(((int64_t)B * H + 128 / (HV / EV) - 1) / (128 / (HV / EV))); \
-    if (bwd) attn_small_bwd_kernel<T, SV, EV, HV, CV><<<blocks, 128, 0, st>>>(qkv, dout, out, B, H, scale); \
-    else attn_small_fwd_kernel<T, SV, EV, HV, CV><<<blocks, 128, 0, st>>>(qkv, out, B, H, scale); }
-#define GO2(SV, EV, HV) { if (causal) GO(SV, EV, HV, true) else GO(SV, EV, HV, false) }
+    if (bwd) attn_small_bwd_kernel<T, SV, EV, HV, CV, VV><<<blocks, 128, 0, st>>>(qkv, dout, out, B, H, scale); \
+    else attn_small_fwd_kernel<T, SV, EV, HV, CV, VV><<<blocks, 128, 0, st>>>(qkv, out, B, H, scale); }
+#define GO2(SV, EV, HV, VV) { if (causal) GO(SV, EV, HV, true, VV) else GO(SV, EV, HV, false, VV) }
     // Sixteen bytes per lane; half of that for eight positions, whose scores and rows need the registers.  A storage offset that breaks
-    // the alignment (a view into a larger buffer) takes a warp per head with the narrowest loads.
+    // the alignment (a view into a larger buffer, at any element) takes a warp per head and loads element by element.
     constexpr int V4 = 16 / (int)sizeof(T), V8 = 8 / (int)sizeof(T);
     const bool al = aligned16(qkv) && aligned16(dout) && aligned16(out);
-    if (al && S == 4) { if (HD == 64) GO2(4, V4, 64) else GO2(4, V4, 32) }
-    else if (al) { if (HD == 64) GO2(8, V8, 64) else GO2(8, V8, 32) }
-    else if (S == 4) { if (HD == 64) GO2(4, 2, 64) else GO2(4, 1, 32) }
-    else { if (HD == 64) GO2(8, 2, 64) else GO2(8, 1, 32) }
+    if (al && S == 4) { if (HD == 64) GO2(4, V4, 64, true) else GO2(4, V4, 32, true) }
+    else if (al) { if (HD == 64) GO2(8, V8, 64, true) else GO2(8, V8, 32, true) }
+    else if (S == 4) { if (HD == 64) GO2(4, 2, 64, false) else GO2(4, 1, 32, false) }
+    else { if (HD == 64) GO2(8, 2, 64, false) else GO2(8, 1, 32, false) }
 #undef GO2
 #undef GO
 }

@@ -63,3 +63,21 @@ def test_short_attention_matches_fp64(B, S, H, hd, off, causal, dtype):
     (want,) = torch.autograd.grad(orf, ref, do.double())
     _close(o.detach(), orf.detach(), dtype)
     _close(got, want, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("S,hd", [(4, 64), (4, 32), (8, 64), (8, 32)])
+@pytest.mark.parametrize("off", [1, 3, 4, 7])
+def test_short_attention_from_any_element_of_a_buffer(S, hd, off, dtype):
+    """Input and output gradient start ``off`` elements into a buffer: every alignment that a contiguous view can have."""
+    B, H = 9, 3
+    g = torch.Generator(device="cuda").manual_seed(off + S)
+    n = B * S * H * hd
+    qkv, do = (torch.randn(m + off, generator=g, device="cuda").to(dtype)[off:].view(B, S, -1) for m in (3 * n, n))
+    o = nn_ops.attention_small(qkv.requires_grad_(), H, True)
+    (got,) = torch.autograd.grad(o, qkv, do)
+    ref = qkv.detach().double().requires_grad_()
+    orf = nn_ops.attention_small_reference(ref, H, True)
+    (want,) = torch.autograd.grad(orf, ref, do.double())
+    _close(o.detach(), orf.detach(), dtype)
+    _close(got, want, dtype)
