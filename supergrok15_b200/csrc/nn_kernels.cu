@@ -169,11 +169,12 @@ __global__ void __launch_bounds__(128) attn_small_bwd_kernel(const T* __restrict
 
 // ---------------------------------------------------------------------------------------------------- LayerNorm
 // z = x (+ r); y = (z - mean) * rstd * gamma (+ beta).  One warp per row; rows of D <= 8192 elements.
+// vec: all rows start on a multiple of four elements' size (widths are multiples of four), so four elements are one access.
 // RMS = true is RMSNorm: the mean is taken as zero (y = z * rsqrt(mean(z^2) + eps) * gamma) and there is no beta.
 template <typename T, bool RMS>
 __global__ void __launch_bounds__(256) ln_fwd_kernel(const T* __restrict__ x, const T* __restrict__ r, const T* __restrict__ gamma,
                                                      const T* __restrict__ beta, T* __restrict__ z, T* __restrict__ y,
-                                                     float* __restrict__ stats, int64_t rows, int D, float eps) {
+                                                     float* __restrict__ stats, int64_t rows, int D, float eps, bool vec) {
     const int lane = threadIdx.x & 31;
     const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (row >= rows) return;
@@ -182,8 +183,8 @@ __global__ void __launch_bounds__(256) ln_fwd_kernel(const T* __restrict__ x, co
     float s = 0.f, ss = 0.f;
     for (int c = lane * 4; c < D; c += 128) {
         float a[4], bres[4];
-        ld4<T>(xr, c, (D - c >= 4) ? 4 : D - c, true, a);
-        if (rr) { ld4<T>(rr, c, (D - c >= 4) ? 4 : D - c, true, bres);
+        ld4<T>(xr, c, (D - c >= 4) ? 4 : D - c, vec, a);
+        if (rr) { ld4<T>(rr, c, (D - c >= 4) ? 4 : D - c, vec, bres);
 #pragma unroll
             for (int k = 0; k < 4; ++k) a[k] = Cvt<T>::to(Cvt<T>::from(a[k] + bres[k])); }
 #pragma unroll
@@ -197,16 +198,16 @@ __global__ void __launch_bounds__(256) ln_fwd_kernel(const T* __restrict__ x, co
     for (int c = lane * 4; c < D; c += 128) {
         const int cnt = (D - c >= 4) ? 4 : D - c;
         float a[4], bres[4], g[4], bb[4], o[4];
-        ld4<T>(xr, c, cnt, true, a);
-        if (rr) { ld4<T>(rr, c, cnt, true, bres);
+        ld4<T>(xr, c, cnt, vec, a);
+        if (rr) { ld4<T>(rr, c, cnt, vec, bres);
 #pragma unroll
             for (int k = 0; k < 4; ++k) a[k] = Cvt<T>::to(Cvt<T>::from(a[k] + bres[k]));
-            st4<T>(z + row * D, c, cnt, true, a); }
-        ld4<T>(gamma, c, cnt, true, g);
-        if (beta) ld4<T>(beta, c, cnt, true, bb);
+            st4<T>(z + row * D, c, cnt, vec, a); }
+        ld4<T>(gamma, c, cnt, vec, g);
+        if (beta) ld4<T>(beta, c, cnt, vec, bb);
 #pragma unroll
         for (int k = 0; k < 4; ++k) o[k] = (a[k] - mean) * rstd * g[k] + (beta ? bb[k] : 0.f);
-        st4<T>(y + row * D, c, cnt, true, o);
+        st4<T>(y + row * D, c, cnt, vec, o);
     }
 }
 
@@ -215,7 +216,7 @@ constexpr int LN_ROWS_PER_CTA = 64;
 template <typename T, bool RMS>
 __global__ void __launch_bounds__(256) ln_bwd_kernel(const T* __restrict__ z, const T* __restrict__ dy, const T* __restrict__ gamma,
                                                      const float* __restrict__ stats, const T* __restrict__ dz_in, T* __restrict__ dz,
-                                                     float* __restrict__ part, int64_t rows, int D) {
+                                                     float* __restrict__ part, int64_t rows, int D, bool vec) {
     extern __shared__ float sm[];                       // [8 warps][2][D]  per-warp column partials
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float* pg = sm + (size_t)w * 2 * D;
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const T* __restrict__ z, co
         for (int c = lane * 4; c < D; c += 128) {
             const int cnt = (D - c >= 4) ? 4 : D - c;
             float a[4], d[4], g[4];
-            ld4<T>(z + row * D, c, cnt, true, a); ld4<T>(dy + row * D, c, cnt, true, d); ld4<T>(gamma, c, cnt, true, g);
+            ld4<T>(z + row * D, c, cnt, vec, a); ld4<T>(dy + row * D, c, cnt, vec, d); ld4<T>(gamma, c, cnt, vec, g);
 #pragma unroll
             for (int k = 0; k < 4; ++k) if (k < cnt) {
                 const float xh = (a[k] - mean) * rstd, dg = d[k] * g[k];
@@ -242,16 +243,16 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const T* __restrict__ z, co
         for (int c = lane * 4; c < D; c += 128) {
             const int cnt = (D - c >= 4) ? 4 : D - c;
             float a[4], d[4], g[4], o[4];
-            ld4<T>(z + row * D, c, cnt, true, a); ld4<T>(dy + row * D, c, cnt, true, d); ld4<T>(gamma, c, cnt, true, g);
+            ld4<T>(z + row * D, c, cnt, vec, a); ld4<T>(dy + row * D, c, cnt, vec, d); ld4<T>(gamma, c, cnt, vec, g);
 #pragma unroll
             for (int k = 0; k < 4; ++k) { const float xh = (a[k] - mean) * rstd; o[k] = rstd * (d[k] * g[k] - s1 - xh * s2); }
             if (dz_in) {                                 // gradient that reached z directly (z is also the residual stream)
                 float e[4];
-                ld4<T>(dz_in + row * D, c, cnt, true, e);
+                ld4<T>(dz_in + row * D, c, cnt, vec, e);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) o[k] += e[k];
             }
-            st4<T>(dz + row * D, c, cnt, true, o);
+            st4<T>(dz + row * D, c, cnt, vec, o);
         }
     }
     __syncthreads();
@@ -617,7 +618,8 @@ __global__ void __launch_bounds__(32 * LN_RED_WARPS) ln_bwd_reduce_kernel(const 
 
 bool attn_small_supported(int S, int HD) { return (S == 4 || S == 8) && (HD == 32 || HD == 64); }
 
-static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+static bool aligned(const void* p, size_t bytes) { return reinterpret_cast<uintptr_t>(p) % bytes == 0; }
+static bool aligned16(const void* p) { return aligned(p, 16); }
 
 template <typename T>
 static void attn_dispatch(bool bwd, const T* qkv, const T* dout, T* out, int B, int S, int H, int HD, bool causal, cudaStream_t st) {
@@ -691,8 +693,10 @@ static void ln_fwd_t(bool rms, const void* x, const void* r, const void* gamma, 
         return;
     }
     const unsigned blocks = (unsigned)((rows + 7) / 8);
-    if (rms) ln_fwd_kernel<T, true><<<blocks, 256, 0, st>>>((const T*)x, (const T*)r, (const T*)gamma, nullptr, (T*)z, (T*)y, stats, rows, D, eps);
-    else ln_fwd_kernel<T, false><<<blocks, 256, 0, st>>>((const T*)x, (const T*)r, (const T*)gamma, (const T*)beta, (T*)z, (T*)y, stats, rows, D, eps);
+    constexpr size_t A = 4 * sizeof(T);
+    const bool vec = aligned(x, A) && aligned(r, A) && aligned(gamma, A) && aligned(beta, A) && aligned(z, A) && aligned(y, A);
+    if (rms) ln_fwd_kernel<T, true><<<blocks, 256, 0, st>>>((const T*)x, (const T*)r, (const T*)gamma, nullptr, (T*)z, (T*)y, stats, rows, D, eps, vec);
+    else ln_fwd_kernel<T, false><<<blocks, 256, 0, st>>>((const T*)x, (const T*)r, (const T*)gamma, (const T*)beta, (T*)z, (T*)y, stats, rows, D, eps, vec);
 }
 
 void ln_fwd(int dtype, bool rms, const void* x, const void* r, const void* gamma, const void* beta, void* z, void* y, float* stats, int64_t rows,
@@ -738,12 +742,14 @@ static void ln_bwd_t(bool rms, const void* z, const void* dy, const void* gamma,
     }
     const int parts = (int)((rows + LN_ROWS_PER_CTA - 1) / LN_ROWS_PER_CTA);
     const size_t smem = (size_t)8 * 2 * D * sizeof(float);
+    constexpr size_t A = 4 * sizeof(T);
+    const bool vec = aligned(z, A) && aligned(dy, A) && aligned(gamma, A) && aligned(dz_in, A) && aligned(dz, A);
     if (rms) {
         cudaFuncSetAttribute(ln_bwd_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        ln_bwd_kernel<T, true><<<parts, 256, smem, st>>>((const T*)z, (const T*)dy, (const T*)gamma, stats, (const T*)dz_in, (T*)dz, part, rows, D);
+        ln_bwd_kernel<T, true><<<parts, 256, smem, st>>>((const T*)z, (const T*)dy, (const T*)gamma, stats, (const T*)dz_in, (T*)dz, part, rows, D, vec);
     } else {
         cudaFuncSetAttribute(ln_bwd_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        ln_bwd_kernel<T, false><<<parts, 256, smem, st>>>((const T*)z, (const T*)dy, (const T*)gamma, stats, (const T*)dz_in, (T*)dz, part, rows, D);
+        ln_bwd_kernel<T, false><<<parts, 256, smem, st>>>((const T*)z, (const T*)dy, (const T*)gamma, stats, (const T*)dz_in, (T*)dz, part, rows, D, vec);
     }
     ln_bwd_reduce_kernel<T><<<(D + 31) / 32, 32 * LN_RED_WARPS, 0, st>>>(part, parts, D, (T*)dgamma, (T*)dbeta, accumulate);
 }

@@ -81,3 +81,37 @@ def test_short_attention_from_any_element_of_a_buffer(S, hd, off, dtype):
     (want,) = torch.autograd.grad(orf, ref, do.double())
     _close(o.detach(), orf.detach(), dtype)
     _close(got, want, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", [64, 512, 132])
+@pytest.mark.parametrize("off", [1, 2, 3, 4])
+@pytest.mark.parametrize("which", ["x", "r", "w", "b", "dy", "all"])
+def test_norm_from_any_element_of_a_buffer(which, off, D, dtype):
+    """Each operand, and all of them, start ``off`` elements into a buffer: every alignment that a contiguous view can have."""
+    rows = 37
+    gen = torch.Generator(device="cuda").manual_seed(off + D)
+
+    def make(name, *shape):
+        o = off if which in (name, "all") else 0
+        n = 1
+        for k in shape:
+            n *= k
+        return torch.randn(n + o, generator=gen, device="cuda").to(dtype)[o:].view(shape)
+    x, r, dy = (make(k, rows, D) for k in ("x", "r", "dy"))
+    w, b = make("w", D), make("b", D)
+    leaves = [t.requires_grad_() for t in (x, r, w, b)]
+    y = nn_ops.layer_norm(x, r, w, b)
+    got = torch.autograd.grad(y, leaves, dy)
+    ref = [t.detach().double().requires_grad_() for t in leaves]
+    zr = ref[0] + ref[1]
+    zr = zr + ((x.detach() + r.detach()).double() - zr.detach())          # the stored sum is what the norm sees
+    yr = F.layer_norm(zr, (D,), ref[2], ref[3], 1e-5)
+    _close(y.detach(), yr.detach(), dtype)
+    for a, c in zip(got, torch.autograd.grad(yr, ref, dy.double())):
+        _close(a, c, dtype, sums=a.dim() == 1)
+    y, z = nn_ops.norm_residual(x, r, w, None, 1e-5, rms=True)
+    got = torch.autograd.grad((y, z), leaves[:3], (dy, dy))
+    yr = zr * torch.rsqrt(zr.square().mean(-1, keepdim=True) + 1e-5) * ref[2]
+    for a, c in zip(got, torch.autograd.grad((yr, zr), ref[:3], (dy.double(), dy.double()))):
+        _close(a, c, dtype, sums=a.dim() == 1)
