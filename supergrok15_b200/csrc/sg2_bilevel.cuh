@@ -184,8 +184,8 @@ __device__ __forceinline__ void bl_advance(const HalfConst& cc, const float* __r
         const float2 v = *reinterpret_cast<const float2*>(row + 32);
         const float x = fmaf(cc.ux[0], v.x, fmaf(cc.ux[1], v.y, cc.ux[2]));
         const float dt = softplus20(fmaf(cc.ud[0], v.x, fmaf(cc.ud[1], v.y, cc.ud[2])));
-        const float ndtc = -fminf(dt, DT_CAP), dtx = dt * x;
-        const f2 ndt2 = pk(ndtc, ndtc), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
+        const float dtx = dt * x;
+        const f2 ndt2 = pk(-dt, -dt), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             if constexpr (HIST) {

@@ -218,7 +218,7 @@ __device__ __forceinline__ void pair_coeffs(float dt, float ah_e, float ah_o, fl
     // half an ulp of 1) does not change the fp32 value: it is dropped
     // One reciprocal serves both states of the pair (1/de = dn/(de*dn)): the scan is bound by the special-function pipe (two
     // reciprocals, a sine and a cosine per pair and step at 16 results per clock per SM), so a reciprocal is traded for three
-    // multiplies on the FMA pipe.  Both denominators lie in [1, 1 + 10|A|], their product cannot overflow.
+    // multiplies on the FMA pipe.
     const float de = fmaf(-dt, ah_e, 1.f), dn = fmaf(-dt, ah_o, 1.f);
     const float r2 = 2.f * rcp_approx(de * dn);
     abe = fmaf(dn, r2, -1.f);
@@ -240,8 +240,8 @@ __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { f2 r; asm("fma.rn.f32x2 %
 
 // Transitions of a group (two RoPE pairs).  One reciprocal serves both states of a pair (1/de = dn / (de dn)); sharing one among all four
 // denominators was measured equal (the special-function pipe is not what bounds the scan, see scan_phase3).
-// Denominators grow with dt; from dt = 1e8 on Abar is -1 to the last bit whatever the exact value, so dt is capped there and the
-// product of two denominators cannot overflow.
+// The same transition as pair_coeffs, which the adjoint uses: a product of denominators past the range of floats gives 1/inf = 0 and
+// Abar = -1, which is what 2/de - 1 rounds to long before.
 __device__ __forceinline__ void quad_coeffs(f2 ndt, f2 dt, f2 ah_e, f2 ah_o, f2 f, f2& abe, f2& abo, f2& cs, f2& sn) {
     const f2 one = pk(1.f, 1.f), mone = pk(-1.f, -1.f);
     const f2 de = fma2(ndt, ah_e, one), dn = fma2(ndt, ah_o, one);
@@ -287,7 +287,6 @@ struct ColPacked {
         asm volatile("" : "+f"(Dj));
     }
 };
-constexpr float DT_CAP = 1e8f;
 
 // column constants of lane j: A/2, rope frequencies, and the affine tables of x_j, z_j, dt_j
 template <int DIR>
@@ -397,8 +396,8 @@ __device__ void scan_phase3(const Item& it, const TensorDir* __restrict__ tds, c
             for (int l = 0; l < lc; ++l) {
                 float* row = tile + (l0 + l) * R3;
                 const float dt = pre[l * 48 + j], x = pre[l * 48 + 16 + j];
-                const float ndtc = -fminf(dt, DT_CAP), dtx = dt * x;
-                const f2 ndt2 = pk(ndtc, ndtc), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
+                const float dtx = dt * x;
+                const f2 ndt2 = pk(-dt, -dt), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
                 f2 ysum = pk(0.f, 0.f);
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
@@ -484,8 +483,8 @@ __device__ void scan_phase3_col(const Item& it, const TensorDir* __restrict__ td
             float* row = tile + l * ROW;
             const float x = fmaf(cc.ux[0], v.x, fmaf(cc.ux[1], v.y, cc.ux[2]));
             const float z = fmaf(cc.uz[0], v.x, fmaf(cc.uz[1], v.y, cc.uz[2]));
-            const float ndtc = -fminf(dt, DT_CAP), dtx = dt * x;
-            const f2 ndt2 = pk(ndtc, ndtc), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
+            const float dtx = dt * x;
+            const f2 ndt2 = pk(-dt, -dt), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
             // dt of the next timestep: its logarithm and exponential start a step ahead of the recurrence that needs them
             const float2 vn = *reinterpret_cast<const float2*>(row + (l + 1 < cnt ? ROW : 0) + 32);
             const float dtn = softplus20(fmaf(cc.ud[0], vn.x, fmaf(cc.ud[1], vn.y, cc.ud[2])));
@@ -569,8 +568,8 @@ __device__ void scan_phase1(const Item& it, const float2* __restrict__ gs, float
             const float2 v = *reinterpret_cast<const float2*>(row + 32);
             const float x = fmaf(cc.ux[0], v.x, fmaf(cc.ux[1], v.y, cc.ux[2]));
             const float dt = softplus20(fmaf(cc.ud[0], v.x, fmaf(cc.ud[1], v.y, cc.ud[2])));
-            const float ndtc = -fminf(dt, DT_CAP), dtx = dt * x;
-            const f2 ndt2 = pk(ndtc, ndtc), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
+            const float dtx = dt * x;
+            const f2 ndt2 = pk(-dt, -dt), dt2 = pk(dt, dt), dtx2 = pk(dtx, dtx), mone = pk(-1.f, -1.f);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const ulonglong2 B = reinterpret_cast<const ulonglong2*>(row)[q];

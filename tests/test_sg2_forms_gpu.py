@@ -41,6 +41,27 @@ def test_scan_with_a_warp_per_item_equals_the_column_form():
         torch.testing.assert_close(a, b, rtol=1e-4, atol=1e-6)
 
 
+@pytest.mark.parametrize("chunk", [16, 4096])
+def test_long_time_steps_with_slow_decay(chunk):
+    """dt = 1e10 and exp(A_log) around 1e-11: the transition depends on their product alone, whichever of the two is large.  Column form with
+    many chunks and warp form, against the CPU statement."""
+    def run(device):
+        ps = make_params([(30011,)], torch.float32, device, 5)
+        torch.manual_seed(1)
+        og = O.SuperGrok2(ps, warmup_steps=0, warmup_ramp=1)
+        with torch.no_grad():
+            for blk in (og.meta_net.mamba_fwd, og.meta_net.mamba_bwd):
+                blk.dt_proj.weight.zero_()
+                blk.dt_proj.bias.fill_(1e10)
+                blk.rope_freq.zero_()
+                blk.A_log.sub_(25.0)
+        og.scan_chunk_len = chunk
+        og.step()
+        return [og._flat_mamba_fwd_states[0].double().cpu(), og._flat_mamba_bwd_states[0].double().cpu()]
+    for a, b in zip(run("cuda"), run("cpu")):
+        assert float(b.norm()) > 0 and float((a - b).norm() / b.norm()) < 1e-4         # fp32 recurrences of some ten steps' memory; capped time steps: 0.5 and more
+
+
 @pytest.mark.parametrize("filler", [3_800_001, 9_900_001])
 def test_element_kernel_parts_agree(filler):
     """A CTA of the element kernel and of the preparation takes 512 or 2,048 elements by the size of the step: tensors around those
