@@ -4,6 +4,7 @@
 #include "bindings_decl.h"
 #include "mt_host.h"
 #include "newton_schulz.h"
+#include "per_device.h"
 #include <map>
 
 namespace sg {
@@ -182,6 +183,16 @@ void register_gemm(pybind11::module_& m) {
             order.emplace_back(mt, nt);
         }
         return order;
+    });
+    m.def("once_per_device_calls", [](const std::vector<int>& devs, int fails) {      // host-side check: which of these calls did the set-up
+        std::atomic<uint64_t> done{0};
+        std::vector<bool> ran;
+        for (int d : devs) {
+            bool set = false;
+            sg::once_per_device(done, d, [&] { set = true; return fails-- <= 0; });
+            ran.push_back(set);
+        }
+        return ran;
     });
     m.def("newton_schulz", &newton_schulz, py::arg("mats"), py::arg("inv"), py::arg("steps"), py::arg("a"), py::arg("b"), py::arg("c"), py::arg("err"));
     m.def("ns_sym_tiles", [](int64_t n, int64_t bn) {                             // (row, column, mirrored) of the tiles of a symmetric product

@@ -17,6 +17,7 @@
 // from nn.MultiheadAttention, grokking_race_v2.py:313-318) for the long-sequence decoder.
 #include "sg_native.h"
 #include "tc_sm100.cuh"
+#include "per_device.h"
 #include <cfloat>
 
 namespace sg {
@@ -681,13 +682,12 @@ int launch_fwd(const void* q, const void* k, const void* v, int64_t ld, void* ou
     constexpr size_t smem = (size_t)(5 * (HD / 64) + 2) * TILE_HALF_BYTES + sizeof(FaBars) + 1024;
     constexpr size_t smem2 = (size_t)(5 * (HD / 64)) * TILE_HALF_BYTES + sizeof(Fa2Bars) + 1024;
     constexpr size_t smem3 = (size_t)(6 * (HD / 64)) * TILE_HALF_BYTES + sizeof(Fa3Bars) + 1024;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(flash_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 2;
-        if (cudaFuncSetAttribute(flash_fwd2_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) != cudaSuccess) return 2;
-        if (cudaFuncSetAttribute(flash_fwd3_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3) != cudaSuccess) return 2;
-        configured = true;
-    }
+    static std::atomic<uint64_t> granted{0};
+    if (!once_per_device(granted, current_device(), [&] {
+            return cudaFuncSetAttribute(flash_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+                   cudaFuncSetAttribute(flash_fwd2_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2) == cudaSuccess &&
+                   cudaFuncSetAttribute(flash_fwd3_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3) == cudaSuccess;
+        })) return 2;
     count_launch();
     if (variant == 3 && S % 256 == 0)
         flash_fwd3_kernel<HD><<<dim3((S / 256) * H * B), FA3_THREADS, smem3, st>>>(mq, mk, mv, (__nv_bfloat16*)out, lse, S, H, ld_o, scale, causal ? 1 : 0, err);
@@ -1062,12 +1062,11 @@ int launch_bwd(const void* q, const void* k, const void* v, int64_t ld, const vo
     if (!make_map(&mv, v, rows, (int64_t)H * HD, ld, 128, 64, true)) return 13;
     if (!make_map(&md, dout, rows, (int64_t)H * HD, ld_o, 128, 64, true)) return 14;
     constexpr size_t smem = (size_t)(6 * (HD / 64)) * TILE_HALF_BYTES + 2048 + FB_STAGE_BYTES + sizeof(FbBars) + 1024;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(flash_bwd_kernel<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 2;
-        if (cudaFuncSetAttribute(flash_bwd_kernel<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 2;
-        configured = true;
-    }
+    static std::atomic<uint64_t> granted{0};
+    if (!once_per_device(granted, current_device(), [&] {
+            return cudaFuncSetAttribute(flash_bwd_kernel<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+                   cudaFuncSetAttribute(flash_bwd_kernel<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+        })) return 2;
     count_launch(3);
     flash_delta_kernel<<<(unsigned)((rows * H * (HD / 8) + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, rows, S, H, HD, ld_o, ld_o);
     const int64_t ld_out = (int64_t)H * HD;

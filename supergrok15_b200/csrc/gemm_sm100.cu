@@ -14,6 +14,7 @@
 // (csrc/ops.cpp:713-727) and the model's Linear layers.
 #include "sg_native.h"
 #include "tc_sm100.cuh"
+#include "per_device.h"
 
 namespace sg {
 namespace {
@@ -582,16 +583,7 @@ bool tc::make_map_batched(CUtensorMap* map, const void* base, int64_t batch, int
 int tc::last_map_error() { return g_map_error; }
 namespace {
 
-int num_sms() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 148;
-    }
-    return n;
-}
+int num_sms() { return device_sms(); }
 
 template <int BN, int STAGES, int MODE = 0, bool A_MN = false, bool B_MN = false>
 int launch(const void* A, int lda, const void* B, int ldb, int M, int N, int K, const Epilogue& ep_in, void* C, int ldc, float* ws,
@@ -617,11 +609,10 @@ int launch(const void* A, int lda, const void* B, int ldb, int M, int N, int K, 
         if (!make_map(&mc, ws, (int64_t)splits * Mpad, N, ldw, 32, 32, false)) return 4;
     } else if (!make_map(&mc, C, MODE == 2 ? M / ag.world : M, N, ldc, 32, ep.c_is_bf16 ? 64 : 32, ep.c_is_bf16 != 0)) return 4;
     constexpr size_t smem = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 4 * 2 * 4096 + 1024 + 256;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(gemm_tn_kernel<BN, STAGES, MODE, A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 2;
-        configured = true;
-    }
+    static std::atomic<uint64_t> granted{0};
+    if (!once_per_device(granted, current_device(), [&] {
+            return cudaFuncSetAttribute(gemm_tn_kernel<BN, STAGES, MODE, A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+        })) return 2;
     const int tiles = tiles_mn * splits;
     // copier CTAs (all-gather mode) come first in the grid; an SM that ran one takes a GEMM CTA afterwards
     const int grid = (tiles < num_sms() ? tiles : num_sms()) + (MODE == 1 ? ag.n_copy : 0);

@@ -19,6 +19,7 @@
 #include <cuda_fp16.h>
 #include "sg_native.h"
 #include "newton_schulz.h"
+#include "per_device.h"
 #include "optim_math.cuh"
 #include "tc_sm100.cuh"
 
@@ -317,16 +318,6 @@ __global__ void __launch_bounds__(256) ns_cast_kernel(const __grid_constant__ Ns
     }
 }
 
-int ns_sms() {
-    static const int n = [] {
-        int dev = 0, v = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-        return v > 0 ? v : 148;
-    }();
-    return n;
-}
-
 // One product over all groups.  phase 0: G, 1: P, 2: X (into xn, or out32 when `last`)
 struct NsView { const void* base; int64_t rows, cols, ld; bool mn; };
 
@@ -335,13 +326,16 @@ int ns_tiles_of(int M, int N, bool sym, int bn) { return sym ? ns_sym_tiles(M, b
 template <int BN, int STAGES, int CAP>
 int ns_go(const NsArgs<CAP>& g, int* err, cudaStream_t s) {
     constexpr size_t smem = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 4 * 2 * 4096 + 1024 + 256;
-    static const cudaError_t configured = cudaFuncSetAttribute(ns_gemm_kernel<BN, STAGES, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (configured != cudaSuccess) return 2;
+    static std::atomic<uint64_t> granted{0};
+    if (!once_per_device(granted, current_device(), [&] {
+            return cudaFuncSetAttribute(ns_gemm_kernel<BN, STAGES, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+        })) return 2;
+    const int sms = device_sms();
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(g.total < ns_sms() ? g.total : ns_sms()));
+    cfg.gridDim = dim3((unsigned)(g.total < sms ? g.total : sms));
     cfg.blockDim = dim3(NS_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -354,13 +348,14 @@ int ns_go(const NsArgs<CAP>& g, int* err, cudaStream_t s) {
 // Width of the output tiles: the widest that still gives every SM a tile.  256 columns read the least shared memory per MMA;
 // where the products are too few or too small to fill the GPU, narrower tiles spread the same work over more SMs.
 int ns_pick_bn(const NsGroup* gr, int n, int phase) {
+    const int sms = device_sms();
     for (int bn = 256; bn > 64; bn /= 2) {
         int64_t tiles = 0;
         for (int i = 0; i < n; ++i) {
             const int k = gr[i].r < gr[i].c ? gr[i].r : gr[i].c;
             tiles += (int64_t)gr[i].batch * (phase < 2 ? ns_tiles_of(k, k, true, bn) : ns_tiles_of(gr[i].r, gr[i].c, false, bn));
         }
-        if (tiles >= ns_sms()) return bn;
+        if (tiles >= sms) return bn;
     }
     return 64;
 }

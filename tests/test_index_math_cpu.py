@@ -40,3 +40,10 @@ def test_scan_chunks_fill_whole_waves():
         items = 2 * sum(max(1, -(-n // L)) for n in numels)
         waves = 1 if 2 * sum(numels) <= wave * 2048 else 2
         assert L % 16 == 0 and L >= 512 and items <= wave * waves - 8
+
+
+def test_kernels_are_set_up_once_per_device():
+    """The opt-in to large dynamic shared memory belongs to a device: the first call on each device makes it, and one that failed is repeated."""
+    assert C.once_per_device_calls([0, 0, 1, 0, 1, 7, 7], 0) == [True, False, True, False, False, True, False]
+    assert C.once_per_device_calls([0, 0, 0, 2], 1) == [True, True, False, True]
+    assert C.once_per_device_calls([64, 64], 0) == [True, True]
