@@ -19,9 +19,29 @@ from . import oracle
 NS_COEFFS = oracle.NS_COEFFS
 
 
-# Matrix elements per run of the grouped iteration: 10 to 12 bytes of workspace each (two bf16 iterates, the fp32 result, G and P), so
-# at most ~3 GB; a run of this size is several milliseconds of tensor-core work, its launches are not what bounds it.
+# Bound on the workspace of one run of the grouped iteration, in elements of a square matrix (12 bytes each: two bf16 iterates, G and P in
+# bf16, the fp32 result): ~3.2 GB.  A run of this size is several milliseconds of tensor-core work, its launches are not what bounds
+# it.  A single matrix above the bound is a run of its own.
 NS_RUN_ELEMS = 1 << 28
+
+
+def _run_elems(r: int, c: int) -> int:
+    """Workspace of a matrix [r, c] in elements of a square one: rows are padded to 8 bf16 and 4 fp32 values, and a padded result is copied
+    to a dense one (a single column takes 52 bytes per element)."""
+    k, c8, c4 = min(r, c), -(-c // 8) * 8, -(-c // 4) * 4
+    return -(-(4 * r * c8 + 4 * k * (-(-k // 8) * 8) + 4 * r * c4 + (4 * r * c if c4 != c else 0)) // 12)
+
+
+def _runs(shapes):
+    """[i, j) of the runs that a list of matrices is cut into."""
+    i = 0
+    while i < len(shapes):
+        j, elems = i, 0
+        while j < len(shapes) and (j == i or elems + _run_elems(*shapes[j]) <= NS_RUN_ELEMS):
+            elems += _run_elems(*shapes[j])
+            j += 1
+        yield i, j
+        i = j
 
 
 def newton_schulz_cuda(X: torch.Tensor, steps: int, precision: str = "bf16") -> torch.Tensor:
@@ -86,12 +106,6 @@ def muon_step(params: List[torch.Tensor], grads, bufs, lr: float, momentum: floa
         return
     # all matrices of the step share the launches of the iteration; long lists go in runs that bound the workspace
     from . import gemm
-    i = 0
-    while i < n:
-        j, elems = i, 0
-        while j < n and (j == i or elems + bufs[j].numel() <= NS_RUN_ELEMS):
-            elems += bufs[j].numel()
-            j += 1
+    for i, j in _runs([tuple(b.shape) for b in bufs]):
         xs = C.newton_schulz(list(bufs[i:j]), inv[i:j], ns_steps, *NS_COEFFS, gemm._err_flag(dev))
         C.mt_apply(C.ops["OP_MUON_UPDATE"], [list(params[i:j]), [x.contiguous() for x in xs]], [], scalars)
-        i = j

@@ -60,3 +60,16 @@ def test_long_lists_go_in_runs(monkeypatch):
         outs.append(p)
     for o in outs[1:]:
         assert all(torch.equal(x, y) for x, y in zip(outs[0], o))
+
+
+@pytest.mark.parametrize("shape", [(4096, 1), (1, 4096), (1000, 9), (64, 64), (300, 5), (8, 2048)])
+def test_runs_bound_the_workspace_that_padding_makes(shape, monkeypatch):
+    """What a run allocates, row padding and the dense copies of padded results included, stays within 12 bytes per element of the bound."""
+    r, c = shape
+    k, up = min(r, c), lambda n, m: -(-n // m) * m
+    each = 2 * 2 * r * up(c, 8) + 2 * 2 * k * up(k, 8) + 4 * r * up(c, 4) + (4 * r * c if c % 4 else 0)
+    monkeypatch.setattr(muon, "NS_RUN_ELEMS", 1 << 16)
+    runs = list(muon._runs([shape] * 50))
+    assert [i for i, _ in runs] == [0] + [j for _, j in runs[:-1]] and runs[-1][1] == 50
+    assert all((j - i) * each <= 12 << 16 or j == i + 1 for i, j in runs)
+    assert all((j - i + 1) * each > (12 << 16) - 12 * (j - i + 1) for i, j in runs[:-1])             # and no run is shorter than it has to be
