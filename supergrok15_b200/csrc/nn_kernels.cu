@@ -399,7 +399,8 @@ __global__ void __launch_bounds__(256) norm_bwd_wide_kernel(const T* __restrict_
 // which took every width that is not a power of two).
 constexpr int NORM_MAX_WPR = 24, NORM_R4_WPR = 8;      // 3072 fp32 columns; four rows per thread need the registers of a smaller CTA
 
-// sums a[0..N) over the wpr warps of this thread's row group, in warp order; `buf` is [warps][N]
+// sums a[0..N) over the wpr warps of this thread's row group; `buf` is [warps][N].  The warps' sums are added in a tree: one after the
+// other, the last of 24 additions of squares would round at the size of the whole sum.
 template <int N>
 __device__ __forceinline__ void group_totals(float (&a)[N], int wpr, float* buf) {
 #pragma unroll
@@ -410,11 +411,12 @@ __device__ __forceinline__ void group_totals(float (&a)[N], int wpr, float* buf)
 #pragma unroll
         for (int i = 0; i < N; ++i) buf[w * N + i] = a[i];
     __syncthreads();
+    const int span = 2 << (31 - __clz(wpr - 1)), k = threadIdx.x & (span - 1);       // power of two that holds wpr >= 2 warps
 #pragma unroll
-    for (int i = 0; i < N; ++i) a[i] = 0.f;
-    for (int k = 0; k < wpr; ++k)
+    for (int i = 0; i < N; ++i) a[i] = k < wpr ? buf[(w0 + k) * N + i] : 0.f;
+    for (int o = span >> 1; o > 0; o >>= 1)
 #pragma unroll
-        for (int i = 0; i < N; ++i) a[i] += buf[(w0 + k) * N + i];
+        for (int i = 0; i < N; ++i) a[i] += __shfl_xor_sync(0xffffffffu, a[i], o);
 }
 
 template <typename T, bool RMS, int R>
@@ -487,10 +489,13 @@ __global__ void __launch_bounds__(R == 1 ? 32 * NORM_MAX_WPR : 32 * NORM_R4_WPR,
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = w % wpr, groups = (blockDim.x >> 5) / wpr;
     const int col = (c * 32 + lane) * VEC;
     const bool in = col < D;
-    float g[VEC], ag[VEC], ab[VEC];
+    // Parameter gradients of this thread's columns: the R rows of a round are summed first (R > 1), or the sums of eight rounds (R = 1), so
+    // that a long call does not add its rows one by one to a sum that outgrows them.
+    float g[VEC], ag[VEC], ab[VEC], bg[VEC], bb[VEC];
 #pragma unroll
-    for (int k = 0; k < VEC; ++k) g[k] = ag[k] = ab[k] = 0.f;
+    for (int k = 0; k < VEC; ++k) g[k] = ag[k] = ab[k] = bg[k] = bb[k] = 0.f;
     if (in) RowVec<T>::get(*reinterpret_cast<const uint4*>(gamma + col), g);
+    int rounds = 0;
     const int64_t step = (int64_t)gridDim.x * groups * R;
     const float inv_d = 1.f / D;
     int par = 0;
@@ -523,11 +528,18 @@ __global__ void __launch_bounds__(R == 1 ? 32 * NORM_MAX_WPR : 32 * NORM_R4_WPR,
                 dg[i][k] = d[k] * g[k];
                 if (!RMS) s1 += dg[i][k];
                 s2 = fmaf(dg[i][k], xh[i][k], s2);
-                ag[k] = fmaf(d[k], xh[i][k], ag[k]);
-                if (!RMS) ab[k] += d[k];
+                bg[k] = fmaf(d[k], xh[i][k], bg[k]);
+                if (!RMS) bb[k] += d[k];
             }
             if constexpr (RMS) t[i] = s2;
             else { t[2 * i] = s1; t[2 * i + 1] = s2; }
+        }
+        if (R > 1 || (++rounds & 7) == 0) {
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) {
+                ag[k] += bg[k]; bg[k] = 0.f;
+                if (!RMS) { ab[k] += bb[k]; bb[k] = 0.f; }
+            }
         }
         if constexpr (RMS) {
             float u[R];
@@ -557,7 +569,7 @@ __global__ void __launch_bounds__(R == 1 ? 32 * NORM_MAX_WPR : 32 * NORM_R4_WPR,
     for (int which = 0; which < (RMS ? 1 : 2); ++which) {
         float v[VEC];
 #pragma unroll
-        for (int k = 0; k < VEC; ++k) v[k] = which == 0 ? ag[k] : ab[k];
+        for (int k = 0; k < VEC; ++k) v[k] = which == 0 ? ag[k] + bg[k] : ab[k] + bb[k];
         if (groups > 1) {
             __syncthreads();
 #pragma unroll
@@ -577,7 +589,7 @@ __global__ void __launch_bounds__(R == 1 ? 32 * NORM_MAX_WPR : 32 * NORM_R4_WPR,
 }
 
 // Second stage of the parameter gradients: column c of dgamma / dbeta is the sum of its n_part partial rows.  A CTA owns 32
-// columns; its 32 warps take the partial rows p = warp, warp + 32, ... and the 32 sub-sums are added in warp order, so the
+// columns; its 32 warps take the partial rows p = warp, warp + 32, ... and the 32 sub-sums are added in a tree, so the
 // result does not depend on timing.  (D / 32 CTAs only: with 8 warps per CTA the kernel took 9 us for 296 partial rows of 512 columns.)
 constexpr int LN_RED_WARPS = 32;
 template <typename T>
@@ -603,14 +615,14 @@ __global__ void __launch_bounds__(32 * LN_RED_WARPS) ln_bwd_reduce_kernel(const 
     }
     sh[0][w][lane] = a; sh[1][w][lane] = b;
     __syncthreads();
-    if (w == 0 && c < D) {
-        a = 0.f; b = 0.f;
-#pragma unroll
-        for (int k = 0; k < LN_RED_WARPS; ++k) { a += sh[0][k][lane]; b += sh[1][k][lane]; }
+    // warp w adds the 32 sub-sums of column w in a tree
+    a = warp_sum(sh[0][lane][w]); b = warp_sum(sh[1][lane][w]);
+    const int col = blockIdx.x * 32 + w;
+    if (lane == 0 && col < D) {
         // accumulate: dgamma / dbeta are the parameters' gradient buffers and already hold other contributions of this step
-        if (accumulate) { a += Cvt<T>::to(dgamma[c]); if (dbeta) b += Cvt<T>::to(dbeta[c]); }
-        dgamma[c] = Cvt<T>::from(a);
-        if (dbeta) dbeta[c] = Cvt<T>::from(b);
+        if (accumulate) { a += Cvt<T>::to(dgamma[col]); if (dbeta) b += Cvt<T>::to(dbeta[col]); }
+        dgamma[col] = Cvt<T>::from(a);
+        if (dbeta) dbeta[col] = Cvt<T>::from(b);
     }
 }
 

@@ -115,3 +115,21 @@ def test_norm_from_any_element_of_a_buffer(which, off, D, dtype):
     yr = zr * torch.rsqrt(zr.square().mean(-1, keepdim=True) + 1e-5) * ref[2]
     for a, c in zip(got, torch.autograd.grad((yr, zr), ref[:3], (dy.double(), dy.double()))):
         _close(a, c, dtype, sums=a.dim() == 1)
+
+
+@pytest.mark.parametrize("rows,D,y_err,w_err", [(300, 3072, 6.9e-8, 1.2e-7), (10000, 3072, 6.9e-8, 1.45e-7), (32000, 1028, 6.9e-8, 1.55e-7)])
+def test_norm_sums_do_not_grow_one_by_one(rows, D, y_err, w_err):
+    """fp32 sums over the warps of a row, the rows of a CTA and the CTAs' partial rows are added in groups.  An output is a product of
+    three factors (6.3e-8 with an exact sum of squares; 7.4e-8 when 24 warps' sums are added one after the other), a weight gradient the sum of
+    ``rows`` products (1.06e-7, 1.28e-7 and 1.37e-7 here; 1.43e-7 for 300 rows with chains, and growing)."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, r, dy = (torch.randn(rows, D, generator=g, device="cuda") for _ in range(3))
+    w = 1 + 0.1 * torch.randn(D, generator=g, device="cuda")
+    leaves = [t.requires_grad_() for t in (x, r, w)]
+    y, z = nn_ops.norm_residual(x, r, w, None, 1e-5, rms=True)
+    got = torch.autograd.grad((y, z), leaves, (dy, dy))[2].double()
+    zr = z.detach().double()
+    xh = zr * torch.rsqrt(zr.square().mean(-1, keepdim=True) + 1e-5)
+    yr, want = xh * w.detach().double(), (xh * dy.double()).sum(0)
+    assert float((y.detach().double() - yr).norm() / yr.norm()) < y_err
+    assert float((got - want).norm() / want.norm()) < w_err
