@@ -788,35 +788,42 @@ __global__ void __launch_bounds__(256) col_sum_part_kernel(const T* __restrict__
     const int c0 = (blockIdx.x * 32 + tx) * VEC;
     const int64_t r0 = (int64_t)blockIdx.y * rows_per_cta;
     const int64_t r1 = r0 + rows_per_cta < rows ? r0 + rows_per_cta : rows;
-    float acc[VEC];
+    // sub: the sum of up to 32 rows, added to acc at a time, so that a long chain of rows does not round at the size of its sum
+    float acc[VEC], sub[VEC];
 #pragma unroll
-    for (int j = 0; j < VEC; ++j) acc[j] = 0.f;
+    for (int j = 0; j < VEC; ++j) acc[j] = sub[j] = 0.f;
+    const auto flush = [&] {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) { acc[j] += sub[j]; sub[j] = 0.f; }
+    };
     if (c0 < C) {
         if (vec) {
             int64_t r = r0 + ty;
-            for (; r + 24 < r1; r += 32) {                    // four independent 16-byte loads in flight per thread
+            for (int n = 1; r + 24 < r1; r += 32, ++n) {      // four independent 16-byte loads in flight per thread
                 uint4 v[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const uint4*>(x + (r + 8 * u) * ld + c0);
+                const T *e0 = reinterpret_cast<const T*>(&v[0]), *e1 = reinterpret_cast<const T*>(&v[1]), *e2 = reinterpret_cast<const T*>(&v[2]),
+                        *e3 = reinterpret_cast<const T*>(&v[3]);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const T* e = reinterpret_cast<const T*>(&v[u]);
-#pragma unroll
-                    for (int j = 0; j < VEC; ++j) acc[j] += Cvt<T>::to(e[j]);
-                }
+                for (int j = 0; j < VEC; ++j) sub[j] += (Cvt<T>::to(e0[j]) + Cvt<T>::to(e1[j])) + (Cvt<T>::to(e2[j]) + Cvt<T>::to(e3[j]));
+                if ((n & 7) == 0) flush();
             }
             for (; r < r1; r += 8) {
                 const uint4 v = *reinterpret_cast<const uint4*>(x + r * ld + c0);
                 const T* e = reinterpret_cast<const T*>(&v);
 #pragma unroll
-                for (int j = 0; j < VEC; ++j) acc[j] += Cvt<T>::to(e[j]);
+                for (int j = 0; j < VEC; ++j) sub[j] += Cvt<T>::to(e[j]);
             }
         } else {
-            for (int64_t r = r0 + ty; r < r1; r += 8)
+            for (int64_t r = r0 + ty, n = 1; r < r1; r += 8, ++n) {
 #pragma unroll
                 for (int j = 0; j < VEC; ++j)
-                    if (c0 + j < C) acc[j] += Cvt<T>::to(x[r * ld + c0 + j]);
+                    if (c0 + j < C) sub[j] += Cvt<T>::to(x[r * ld + c0 + j]);
+                if ((n & 15) == 0) flush();
+            }
         }
+        flush();
     }
 #pragma unroll
     for (int j = 0; j < VEC; ++j) sh[ty][tx * VEC + j] = acc[j];
@@ -824,15 +831,12 @@ __global__ void __launch_bounds__(256) col_sum_part_kernel(const T* __restrict__
     for (int c = threadIdx.x; c < 32 * VEC; c += 256) {
         const int col = blockIdx.x * 32 * VEC + c;
         if (col < C) {
-            float t = 0.f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) t += sh[k][c];
-            part[(int64_t)blockIdx.y * C + col] = t;
+            part[(int64_t)blockIdx.y * C + col] = ((sh[0][c] + sh[1][c]) + (sh[2][c] + sh[3][c])) + ((sh[4][c] + sh[5][c]) + (sh[6][c] + sh[7][c]));
         }
     }
 }
 
-// Second stage: 32 columns per CTA; warp w adds the partial rows w, w + 8, ... and the 8 sub-sums are added in warp order.
+// Second stage: 32 columns per CTA; warp w adds the partial rows w, w + 8, ... and the 8 sub-sums are added in a tree.
 template <typename T>
 __global__ void __launch_bounds__(256) col_sum_final_kernel(const float* __restrict__ part, int parts, int C, T* __restrict__ out,
                                                             bool accumulate) {
@@ -846,17 +850,14 @@ __global__ void __launch_bounds__(256) col_sum_final_kernel(const float* __restr
             float v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) v[u] = part[(int64_t)(p + 8 * u) * C + c];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) t += v[u];
+            t += (v[0] + v[1]) + (v[2] + v[3]);
         }
         for (; p < parts; p += 8) t += part[(int64_t)p * C + c];
     }
     sh[w][lane] = t;
     __syncthreads();
     if (w == 0 && c < C) {
-        t = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) t += sh[k][lane];
+        t = ((sh[0][lane] + sh[1][lane]) + (sh[2][lane] + sh[3][lane])) + ((sh[4][lane] + sh[5][lane]) + (sh[6][lane] + sh[7][lane]));
         if (accumulate) t += Cvt<T>::to(out[c]);
         out[c] = Cvt<T>::from(t);
     }

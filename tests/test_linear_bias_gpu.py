@@ -62,3 +62,16 @@ def test_forms_that_the_library_takes():
     gx, gw, gb = torch.autograd.grad(nn_ops.linear(x, w0, b0).sum(), (x, w0, b0))
     assert gw.shape == w0.shape and gb.shape == b0.shape and not gx.any()
     assert not nn_ops._col_sum_bias(x, w0, b0) and nn_ops._col_sum_bias(x, w, torch.zeros(8, device="cuda", requires_grad=True))
+
+
+# 1.5e-7 to 2.0e-7 is what PyTorch's sum of these columns is off; chains of rows were 1.9e-7, 2.1e-7 and 2.8e-7 off
+@pytest.mark.parametrize("rows,out,err", [(32768, 64, 1.45e-7), (32768, 2048, 1.5e-7), (131072, 1024, 2.0e-7), (200000, 63, 2.5e-7)])
+def test_column_sums_are_as_precise_as_the_librarys(rows, out, err):
+    from supergrok15_b200 import _build
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(rows, out, generator=g, device="cuda")
+    want = x.double().sum(0)
+    got = _build.require().col_sum(x).double()
+    assert float((got - want).norm() / want.norm()) < err
+    acc = torch.ones(out, device="cuda")
+    assert torch.equal(_build.require().col_sum(x, acc), acc) and float((acc.double() - 1 - want).norm() / want.norm()) < err + 1e-7
