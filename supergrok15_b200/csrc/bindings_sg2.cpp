@@ -27,7 +27,7 @@ size_t sg2_td_bytes();
 int sg2_bilevel_ng();
 int sg2_bilevel_tile();
 void sg2_scan_backward(const void* items_dev, int n_items, int dir1_start, const void* tds_dev, int n_td, const int64_t* snap_base_dev,
-                       const float* gs_sorted, const uint32_t* vals_sorted, const float* dctx, const float* carry, float* agg, float* dcarry,
+                       const float* gs_sorted, const uint32_t* vals_sorted, const float* dctx, float* agg, float* dcarry,
                        float* snaps, float* partial, float* grads, int snap_every, cudaStream_t s);
 }
 
@@ -186,7 +186,7 @@ void write_table(Tensor dst, const std::vector<int64_t>& uints, const std::vecto
 }
 
 // Adjoint of the scan: dctx [total,16] -> grads [2, NG] (see csrc/sg2_bilevel.cuh for the layout).  Must follow a forward scan on the
-// same plan / workspace (it re-uses gs, vals and the chunk carry-in states of that forward).
+// same plan / workspace (it uses gs, vals and the state snapshots of that forward).
 void sg2_scan_backward(Tensor items, int64_t n_items, int64_t dir1_start, Tensor tds, int64_t n_td, Tensor snap_base, int64_t sorted_buf,
                        Tensor dctx, py::dict ws, Tensor snaps, Tensor partial, Tensor grads, int64_t snap_every) {
     c10::cuda::CUDAGuard guard(items.device());
@@ -194,7 +194,7 @@ void sg2_scan_backward(Tensor items, int64_t n_items, int64_t dir1_start, Tensor
     TORCH_CHECK(dctx.is_contiguous() && dctx.scalar_type() == at::kFloat, "dctx must be contiguous fp32");
     const uint32_t* vs = sorted_buf ? u32(W("vals1")) : u32(W("vals0"));
     sg::sg2_scan_backward(items.data_ptr(), (int)n_items, (int)dir1_start, tds.data_ptr(), (int)n_td, snap_base.data_ptr<int64_t>(),
-                          W("gs").data_ptr<float>(), vs, dctx.data_ptr<float>(), W("carry").data_ptr<float>(), W("agg").data_ptr<float>(),
+                          W("gs").data_ptr<float>(), vs, dctx.data_ptr<float>(), W("agg").data_ptr<float>(),
                           W("dcarry").data_ptr<float>(), snaps.data_ptr<float>(), partial.data_ptr<float>(), grads.data_ptr<float>(),
                           (int)snap_every, at::cuda::getCurrentCUDAStream());
 }

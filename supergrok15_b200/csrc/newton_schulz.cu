@@ -47,8 +47,6 @@ template <int CAP> struct NsArgs {
     float alpha, beta, diag;
 };
 
-template <int BN> constexpr int ns_sym_block() { return BN > BM ? BN : BM; }
-
 // Tiles of a symmetric [n, n] product: square blocks of max(BM, BN) on and above the diagonal, cut into BM x BN tiles.
 __host__ __device__ inline int ns_sym_tiles(int n, int bn) {
     const int S = bn > BM ? bn : BM, nb = (n + S - 1) / S;

@@ -328,8 +328,8 @@ __global__ void __launch_bounds__(256) norm_fwd_wide_kernel(const T* __restrict_
 
 template <typename T, bool RMS, int NCH>
 __global__ void __launch_bounds__(256) norm_bwd_wide_kernel(const T* __restrict__ z, const T* __restrict__ dy, const T* __restrict__ gamma,
-                                                            const float* __restrict__ stats, const T* __restrict__ dz_in, T* __restrict__ dz,
-                                                            float* __restrict__ part, int64_t rows) {
+                                                            const float* __restrict__ stats, T* __restrict__ dz, float* __restrict__ part,
+                                                            int64_t rows) {
     constexpr int VEC = RowVec<T>::VEC, D = 32 * VEC * NCH;
     extern __shared__ float sm[];                       // [8 warps][D]
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -362,12 +362,6 @@ __global__ void __launch_bounds__(256) norm_bwd_wide_kernel(const T* __restrict_
                 ag[c][k] = fmaf(d[k], xh, ag[c][k]);
                 if (!RMS) ab[c][k] += d[k];
             }
-            if (dz_in) {
-                float e[VEC];
-                row_ld<T>(dz_in + row * D + col, e);
-#pragma unroll
-                for (int k = 0; k < VEC; ++k) o[k] += e[k];
-            }
             row_st<T>(dz + row * D + col, o);
         }
     }
@@ -387,7 +381,6 @@ __global__ void __launch_bounds__(256) norm_bwd_wide_kernel(const T* __restrict_
             part[((int64_t)blockIdx.x * 2 + which) * D + col] = acc;
         }
     }
-    if (RMS) for (int col = threadIdx.x; col < D; col += 256) part[((int64_t)blockIdx.x * 2 + 1) * D + col] = 0.f;
 }
 
 // Rows of any whole number of 16-byte vectors.  A row is spread over WPR = ceil(D / (32 VEC)) warps, one vector per lane, and a thread
@@ -691,7 +684,7 @@ static void ln_fwd_t(bool rms, const void* x, const void* r, const void* gamma, 
 #define WIDE_F(N) \
             if (rms) norm_fwd_wide_kernel<T, true, N><<<g8, 256, 0, st>>>((const T*)x, (const T*)r, (const T*)gamma, nullptr, (T*)z, (T*)y, stats, rows, eps); \
             else norm_fwd_wide_kernel<T, false, N><<<g8, 256, 0, st>>>((const T*)x, (const T*)r, (const T*)gamma, (const T*)beta, (T*)z, (T*)y, stats, rows, eps);
-            switch (wpr) { case 1: WIDE_F(1) break; case 2: WIDE_F(2) break; default: WIDE_F(4) }
+            switch (wpr) { case 1: WIDE_F(1) break; case 2: WIDE_F(2) break; default: if constexpr (sizeof(T) == 4) { WIDE_F(4) } }      // 16 bits stop at two
 #undef WIDE_F
             return;
         }
@@ -735,8 +728,8 @@ static void ln_bwd_t(bool rms, const void* z, const void* dy, const void* gamma,
             const int g8 = (int)(n8 < 1 ? 1 : n8 < NORM_BWD_GRID ? n8 : NORM_BWD_GRID);
             const size_t smw = (size_t)8 * D * sizeof(float);
 #define WIDE_B(N) \
-            if (rms) norm_bwd_wide_kernel<T, true, N><<<g8, 256, smw, st>>>((const T*)z, (const T*)dy, (const T*)gamma, stats, (const T*)dz_in, (T*)dz, part, rows); \
-            else norm_bwd_wide_kernel<T, false, N><<<g8, 256, smw, st>>>((const T*)z, (const T*)dy, (const T*)gamma, stats, (const T*)dz_in, (T*)dz, part, rows);
+            if (rms) norm_bwd_wide_kernel<T, true, N><<<g8, 256, smw, st>>>((const T*)z, (const T*)dy, (const T*)gamma, stats, (T*)dz, part, rows); \
+            else norm_bwd_wide_kernel<T, false, N><<<g8, 256, smw, st>>>((const T*)z, (const T*)dy, (const T*)gamma, stats, (T*)dz, part, rows);
             switch (wpr) { case 1: WIDE_B(1) break; case 2: WIDE_B(2) break; default: WIDE_B(4) }
 #undef WIDE_B
             ln_bwd_reduce_kernel<T><<<(D + 31) / 32, 32 * LN_RED_WARPS, 0, st>>>(part, g8, D, (T*)dgamma, (T*)dbeta, accumulate);

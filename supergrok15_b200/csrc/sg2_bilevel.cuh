@@ -29,7 +29,6 @@ constexpr int BL_TILE = 16;                    // timesteps per backward tile
 constexpr int BL_ITEMS = 4;                    // items per CTA of adj 1
 constexpr int BL_THREADS = BL_ITEMS * 16;
 constexpr int BL_NG = 768;                     // gradient values per direction (layout above)
-constexpr int BL_LANE_ACC = 16 + 8 + 1 + 9 + 8;   // register-resident accumulators per lane: dah, df, dD, dUx/Uz/Udt, dWout column
 constexpr int BL_ROW = 60;                     // floats per timestep row in shared memory: B16 C16 (g,s,-,-) gout16 dctx8
 
 // g_out_j[t] = sum_d dctx[t][d] * Wout[d][j]  and  B, C of the timestep: lane l = timestep
@@ -375,11 +374,11 @@ __global__ void __launch_bounds__(1024) sg2_adj4_kernel(const float* __restrict_
 int sg2_bilevel_ng() { return BL_NG; }
 int sg2_bilevel_tile() { return BL_TILE; }
 
-// dctx [total,16] (original order) -> grads [2][BL_NG].  Uses the forward scan's carry (chunk carry-in states of THIS forward),
-// agg/dcarry scratch of the same sizes as the forward ones, snaps [sum over items of ceil(tiles / snap_every), 16, 16] and
+// dctx [total,16] (original order) -> grads [2][BL_NG].  Uses agg / dcarry scratch of the sizes of the forward's agg / carry, the states that
+// the forward scan has left in snaps [sum over items of ceil(tiles / snap_every), 16, 16] and
 // partial [n_items, BL_NG].  snap_base[item] = index of the item's first snapshot.
 void sg2_scan_backward(const void* items_dev, int n_items, int dir1_start, const void* tds_dev, int n_td, const int64_t* snap_base_dev,
-                       const float* gs_sorted, const uint32_t* vals_sorted, const float* dctx, const float* carry, float* agg, float* dcarry,
+                       const float* gs_sorted, const uint32_t* vals_sorted, const float* dctx, float* agg, float* dcarry,
                        float* snaps, float* partial, float* grads, int snap_every, cudaStream_t s) {
     if (n_items <= 0) return;
     if (snap_every < 1) snap_every = 1;
