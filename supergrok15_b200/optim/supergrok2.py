@@ -25,13 +25,13 @@ from .metanet import Mamba3PEERMetaNet
 from .supergrok15 import SuperGrok15
 
 
-def _copies(named_tensors):
-    """{name: copy}; dense tensors share the launches of one foreach copy."""
-    out = {n: torch.empty_like(t) if t.layout == torch.strided else t.clone() for n, t in named_tensors}
-    dense = [(out[n], t) for n, t in named_tensors if t.layout == torch.strided]
-    if dense:
-        torch._foreach_copy_([d for d, _ in dense], [t for _, t in dense])
-    return out
+@torch.no_grad()
+def _copies(tensors):
+    """Copies of a list of tensors.  Dense ones in one foreach call (a product with 1, which allocates its results natively): one or two
+    launches and no allocation from Python per tensor."""
+    dense = [t for t in tensors if t.layout == torch.strided]
+    made = iter(torch._foreach_mul(dense, 1.0) if dense else ())
+    return [next(made) if t.layout == torch.strided else t.clone() for t in tensors]
 
 
 class SuperGrok2(SuperGrok15):
@@ -161,12 +161,13 @@ class SuperGrok2(SuperGrok15):
         named = list(model.named_parameters())
         # A backward may fill the storage that .grad already has (buckets of a distributed wrapper, buffers of a captured graph), so the
         # training gradients are copied before the validation backward: all of them in one foreach call.
-        grads = [(n, p.grad.detach()) for n, p in named if p.grad is not None]
-        if not grads:
+        have = [n for n, p in named if p.grad is not None]
+        if not have:
             return 0.0
-        saved = _copies(grads)
+        saved = dict(zip(have, _copies([p.grad for _, p in named if p.grad is not None])))
         try:
-            model.zero_grad()
+            for _, p in named:
+                p.grad = None
             with torch.enable_grad():
                 val_loss = criterion(model(val_x), val_y)
                 val_loss.backward()
