@@ -29,7 +29,7 @@ using namespace tc;
 
 constexpr int BM = 128, BK = 64;
 constexpr int NS_THREADS = 192;
-// Shapes per launch.  A launch copies its whole parameter block (704 bytes per shape), and the short products of small models are
+// Shapes per launch.  A launch copies its whole parameter block (576 bytes per shape), and the short products of small models are
 // bound by how fast launches follow one another, so parameter lists with few shapes (a decoder has four) take the small block.
 constexpr int NS_GROUPS = 40, NS_FEW = 6;
 
@@ -41,6 +41,7 @@ struct alignas(64) NsProblem {
     int tile0, tiles;                             // first tile in the launch, tiles of one matrix
     int a_mn, b_mn, sym, c_f32;
 };
+static_assert(sizeof(NsProblem) == 576, "four tensor maps of 128 bytes and the sizes");
 template <int CAP> struct NsArgs {
     NsProblem p[CAP];
     int n, total;

@@ -6,17 +6,18 @@
 // uses the same chunk decomposition as the forward scan, so every SM works on it:
 //
 //   adj 1   per chunk: aggregate of the reverse recurrence  dh[t-1] = M_t^T (dh[t] + dy_t C_t)   (prefix product walked
-//           forwards from the chunk start, with the same 2^-100 early exit as the forward aggregates)
+//           forwards from the chunk start, with an early exit at 2^-100; the forward aggregates stop at 2^-48)
 //   adj 2   carry: dh arriving at the end of every chunk (chunks in reverse order; the last chunk receives zero)
-//   adj 3   per chunk: walk the tiles backwards from the states that the forward scan has left at their boundaries (global scratch): recompute the 16 states of the tile into shared memory, run the exact adjoint of
-//           each timestep, accumulate parameter gradients privately per lane
+//   adj 3   per chunk: walk the tiles backwards from the states that the forward scan has left at their boundaries (global scratch):
+//           recompute the 16 states of the tile into shared memory, run the exact adjoint of each timestep, accumulate parameter
+//           gradients privately per lane
 //   adj 4   fixed-order reduction of the per-item partial gradients
 //
 // Because x, z, dt, B and C are affine in (g, s) (SG2Pack::AFF* tables), their weight gradients are gradients of the
 // TABLES:  dU[j][k] += d value_j[t] * (g_t, s_t, 1)[k].  The chain rule from the tables to input_proj / in_proj / dt_proj /
 // B_proj / C_proj is a handful of tiny matrix products (sg2_meta.cu: sg2_fold_bwd_kernel).  This formulation contains the
 // cross-column terms exactly (every column's dependence on B_s and C_s goes through the shared tables).
-// Per direction the kernel produces NG = 138 + 128 gradient values:
+// Per direction the kernels produce BL_NG = 768 gradient values:
 //   [0,256)    d A_log [16][16]          [256,384)  d rope_freq [16][8]      [384,400)  d D [16]
 //   [400,448)  d U_x [16][3]   [448,496) d U_z   [496,544) d U_dt   [544,592) d U_B [16][3]   [592,640) d U_C [16][3]
 //   [640,768)  d out_proj [8][16]
@@ -207,7 +208,7 @@ __device__ __forceinline__ void bl_advance(const HalfConst& cc, const float* __r
 // State snapshots are kept at the start of every `snap_every`-th tile (checkpoint interval = snap_every * BL_TILE timesteps); a tile
 // that does not start at a snapshot is reached by re-running the forward recurrence from the snapshot before it, which trades
 // (snap_every - 1) / 2 extra tile passes on average for 1 / snap_every of the snapshot memory.  The gradients do not depend on it.
-// A warp per chunk: the states before the 16 steps of a tile take 16 KB of shared memory per chunk, which leaves room for eleven chunks on
+// A warp per chunk: the states before the 16 steps of a tile take 16 KB of shared memory per chunk, which leaves room for ten chunks on
 // an SM; with half a warp each that was 1.25 warps per scheduler and latency all the way (422,755 parameters: 1,395 -> 940 us).
 template <int DIR>
 __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uint32_t* __restrict__ vals_sorted, const float* __restrict__ dctx,

@@ -26,13 +26,14 @@ constexpr int XSEG = XH + 1;      // linear pieces of an expert = row pitch of i
 
 // An expert is a piecewise linear function of the scalar g: hidden unit j switches at t_j = -b1_j / W1_j.  The tables hold the sorted
 // switching points and, per piece, slope and intercept (summed in fp64), so that a value takes five comparisons and a compensated
-// multiply-add instead of 16 hidden units with three table words each; both forms were bound by the shared-memory reads (54 against 9
-// per value).
-// slope * g and the intercept cancel where g lies near the switching points of the units that are on (each unit then has a
-// small value, which 16 separate units would round relative to itself).  So slope and intercept are pairs of floats (value and remainder) and the
-// product and the sum keep their rounding errors: what is lost is 2^-47 of |slope * g|.  The switching points are rounded towards
+// multiply-add instead of 16 hidden units with three table words each; both forms are bound by the shared-memory reads (54 against 9 words
+// per value).  Forward at 422,755 elements 385 us with units, 113 us with the table.
+// slope * g and the intercept cancel where g lies near the switching points of the units that are on: each unit then has a small value,
+// which the sum over the units rounds relative to itself.  So slope and intercept are pairs of floats (value and remainder) and the
+// product and the sum keep their rounding errors: what is lost is 2^-47 of |slope * g|.  (Plain floats take 81 us and are 8e-6 off with
+// all switching points within 1e-4 of the gradients, where the units are 6e-8 off.)  The switching points are rounded towards
 // -infinity: for every float g, g > t_j then decides exactly as the sign of g * W1_j + b1_j does.
-struct XTable { const float4* v; const float* t; };                                                     // v: slope, its remainder, intercept, its remainder
+struct XTable { const float4* v; const float* t; };                            // v: slope, its remainder, intercept, its remainder
 size_t __host__ __device__ constexpr x_table_floats(int E) { return (size_t)E * XSEG * 5; }
 
 // sixteen lanes per expert: lane j ranks its switching point, lane s sums piece s (lane 0 also piece 16)

@@ -3,8 +3,8 @@
 All parameter tensors are processed in ONE batched call: sort -> gather -> forward scan (the step kernels, with scratch
 copies of the persistent states) -> contexts ``ctx [total, 16]``.  The part after the scan (GRU, soft top-4 product-key
 routing, experts) is element-wise and runs through autograd in slices, producing d(meta_loss)/d ctx.  The scan adjoint
-kernels turn that into gradients of A_log, rope_freq, D, out_proj and of the folded affine tables; autograd through
-one small kernel (``csrc/sg2_meta.cu``) carries the table gradients to input_proj / in_proj / dt_proj / B_proj / C_proj.
+kernels turn that into gradients of A_log, rope_freq, D, out_proj and of the folded affine tables; one small kernel
+(``csrc/sg2_meta.cu``) carries the table gradients to input_proj / in_proj / dt_proj / B_proj / C_proj.
 The result equals autograd of ``Mamba3PEERMetaNet.forward_for_bilevel`` (tested), including the cross-column terms that
 the reference kernel drops.
 
@@ -114,8 +114,8 @@ def gru(x, h, W, b):
     return _Gru.apply(x, h, W, b)
 
 
-# (offset, shape) of the scan's parameters in the packed layout, in the order of ``ops/sg2.py: scan_leaves``
 def _leaf_views(flat: torch.Tensor, leaves) -> List[torch.Tensor]:
+    """Views of a vector in the packed layout, one per parameter of the scan, in the order of ``ops/sg2.py: scan_leaves``."""
     L = sg2_ops.layout()
     offs = [L["IN_W"], L["IN_B"]]
     for base in (L["DIR0"], L["DIR1"]):

@@ -110,7 +110,7 @@ def test_pack_kernel_equals_the_statement(hidden):
             p.normal_(0, 0.5)
     want = sg2_ops.pack_metanet(copy.deepcopy(mn).cpu())
     got = sg2_ops.pack_metanet(mn.cuda()).cpu()
-    torch.testing.assert_close(got, want, rtol=3e-7, atol=0.0)          # copies, and -exp(A_log) by another exp: two units
+    torch.testing.assert_close(got, want, rtol=3e-7, atol=0.0)          # copies; the folded tables are fp64 sums in another order, rounded once
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
@@ -131,3 +131,16 @@ def test_unit_vectors(dtype):
         n = float(v.norm())
         want = torch.zeros_like(v) if not torch.isfinite(v).all() else v / n if n > 1e-12 else v
         torch.testing.assert_close(out[a:b].double(), want, rtol=1e-6, atol=0.0)
+
+
+def test_unit_vectors_of_more_tensors_than_a_launch_takes():
+    """A launch takes at most 96 tensors: the others' totals and offsets belong to the next one."""
+    C = _build.require()
+    g = torch.Generator(device="cuda").manual_seed(4)
+    ts = [torch.randn(1 + 37 * i % 600, generator=g, device="cuda") * 10.0 ** (i % 7 - 3) for i in range(211)]
+    ts[100][0] = float("nan")
+    offs = torch.tensor([0] + [t.numel() for t in ts]).cumsum(0).tolist()
+    out = C.sg2_unit_vectors(ts, offs[:-1], offs[-1])
+    for i, (t, a, b) in enumerate(zip(ts, offs[:-1], offs[1:])):
+        want = torch.zeros_like(t) if i == 100 else t / t.double().norm()
+        torch.testing.assert_close(out[a:b].double(), want.double(), rtol=1e-6, atol=0.0)
