@@ -22,10 +22,17 @@ inline int current_device() {
     return dev;
 }
 
+// SMs of the current device; the answers are kept per ordinal, a launcher asks several times per launch
 inline int device_sms() {
-    int n = 0;
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, current_device());
-    return n > 0 ? n : 148;
+    static std::atomic<int> known[64];
+    const int dev = current_device(), k = dev >= 0 && dev < 64 ? dev : -1;
+    int n = k >= 0 ? known[k].load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (n <= 0) return 148;
+        if (k >= 0) known[k].store(n, std::memory_order_relaxed);
+    }
+    return n;
 }
 
 }  // namespace sg

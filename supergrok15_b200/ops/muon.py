@@ -34,6 +34,9 @@ def _run_elems(r: int, c: int) -> int:
 
 def _runs(shapes):
     """[i, j) of the runs that a list of matrices is cut into."""
+    if 8 * sum(r * c for r, c in shapes) <= NS_RUN_ELEMS:            # no matrix takes more than 84 bytes per element (a single one)
+        yield 0, len(shapes)
+        return
     i = 0
     while i < len(shapes):
         j, elems = i, 0
@@ -106,6 +109,6 @@ def muon_step(params: List[torch.Tensor], grads, bufs, lr: float, momentum: floa
         return
     # all matrices of the step share the launches of the iteration; long lists go in runs that bound the workspace
     from . import gemm
-    for i, j in _runs([tuple(b.shape) for b in bufs]):
+    for i, j in _runs([b.shape for b in bufs]):
         xs = C.newton_schulz(list(bufs[i:j]), inv[i:j], ns_steps, *NS_COEFFS, gemm._err_flag(dev))
         C.mt_apply(C.ops["OP_MUON_UPDATE"], [list(params[i:j]), [x.contiguous() for x in xs]], [], scalars)
