@@ -1,6 +1,7 @@
 // Fixed-order sum of the per-CTA partial rows of a reduction: out[c] = sum_p partial[p][c].  A CTA owns 32 columns; warp w adds the rows
-// w, w + 32, ... (four loads in flight) and the 32 sub-sums are added in warp order.  One thread per column walked up to 1,700
-// rows behind one another: 118 us for the scan adjoint, 13 to 29 us for the routing, GRU and expert gradients.
+// w, w + 32, ... (four loads in flight) and the 32 sub-sums are added in warp order; in fp64, since the partial rows are few and
+// cancel.  One thread per column walked up to 1,700 rows behind one another: 118 us for the scan adjoint, 13 to 29 us for the routing,
+// GRU and expert gradients.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -8,9 +9,9 @@
 namespace sg {
 
 __device__ __forceinline__ float column_parts_sum(const float* __restrict__ partial, int64_t first, int64_t last, int ng, int c) {
-    __shared__ float sh[32][33];
+    __shared__ double sh[32][33];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float t = 0.f;
+    double t = 0;
     if (c < ng) {
         int64_t p = first + w;
         for (; p + 96 < last; p += 128) {
@@ -24,11 +25,11 @@ __device__ __forceinline__ float column_parts_sum(const float* __restrict__ part
     }
     sh[w][lane] = t;
     __syncthreads();
-    t = 0.f;
+    t = 0;
     if (w == 0)
 #pragma unroll
         for (int k = 0; k < 32; ++k) t += sh[k][lane];
-    return t;                                             // valid in warp 0
+    return (float)t;                                      // valid in warp 0
 }
 
 namespace {

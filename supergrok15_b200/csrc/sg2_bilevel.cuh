@@ -229,7 +229,7 @@ __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uin
         for (int q = 0; q < 2; ++q) { const float4 t = reinterpret_cast<const float4*>(din)[q]; dh[4 * q] = t.x; dh[4 * q + 1] = t.y; dh[4 * q + 2] = t.z; dh[4 * q + 3] = t.w; }
     }
 #pragma unroll
-    for (int s = 0; s < 8; ++s) { dah[s] = 0.f; dwo[s] = 0.f; }
+    for (int s = 0; s < 8; ++s) dah[s] = dwo[s] = 0.f;
 #pragma unroll
     for (int p = 0; p < 4; ++p) df[p] = 0.f;
     float dbc[3] = {0.f, 0.f, 0.f};                        // dU_B (j < 8) or dU_C row of state 8 half + (j & 7), summed over the columns
@@ -252,9 +252,13 @@ __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uin
         bl_stage_a<DIR>(tile, gs, vals_sorted, dctx, it.off, it.n, u0 + j, half == 0 && j < cnt, j);
         __syncwarp();
         bl_advance<true, BL_ROW>(cc, tile, cnt, h, hist, half, lane);
-        // reverse through the tile; the table gradients are summed per tile first, so that a chunk of thousands of steps adds a sixteenth
-        // as many terms to its large sums
-        float tb[3] = {0.f, 0.f, 0.f}, tx[3] = {0.f, 0.f, 0.f}, tz[3] = {0.f, 0.f, 0.f}, td[3] = {0.f, 0.f, 0.f};
+        // reverse through the tile; the gradients are summed per tile first, so that a chunk of thousands of steps adds a sixteenth as many
+        // terms to its large sums
+        float tb[3] = {0.f, 0.f, 0.f}, tx[3] = {0.f, 0.f, 0.f}, tz[3] = {0.f, 0.f, 0.f}, td[3] = {0.f, 0.f, 0.f}, tD = 0.f, tah[8], tf[4], two[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) tah[s] = two[s] = 0.f;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) tf[p] = 0.f;
 #pragma unroll 1
         for (int l = cnt - 1; l >= 0; --l) {
             const float* row = tile + l * BL_ROW;
@@ -287,10 +291,10 @@ __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uin
                 const float dcs = fmaf(dre, he, dro * ho), dsn = fmaf(dro, he, -dre * ho);
                 const float dth = fmaf(cs, dsn, -sn * dcs);
                 ddt = fmaf(dth, f[p], ddt);
-                df[p] = fmaf(dth, dt, df[p]);
+                tf[p] = fmaf(dth, dt, tf[p]);
                 const float gae = dabe * (abe + 1.f) * (abe + 1.f) * 0.5f, gao = dabo * (abo + 1.f) * (abo + 1.f) * 0.5f;
                 ddt = fmaf(gae, ah[e], fmaf(gao, ah[o], ddt));
-                dah[e] = fmaf(gae, dt, dah[e]); dah[o] = fmaf(gao, dt, dah[o]);
+                tah[e] = fmaf(gae, dt, tah[e]); tah[o] = fmaf(gao, dt, tah[o]);
                 dh[e] = fmaf(dre, cs, dro * sn);
                 dh[o] = fmaf(dro, cs, -dre * sn);
             }
@@ -311,17 +315,22 @@ __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uin
             }
             const float outj = fmaf(y, sl, cc.Dj * x);
             const float dz = gout * y * sz * (1.f + z * (1.f - sz));
-            dD = fmaf(gout, x, dD);
+            tD = fmaf(gout, x, tD);
             const float dx = fmaf(gout, cc.Dj, ddtx * dt);
             ddt = fmaf(ddtx, x, ddt);
             const float ddtr = ddt * (dtr > 20.f ? 1.f : sigmoidf(dtr));
 #pragma unroll
             for (int k = 0; k < 3; ++k) { tx[k] = fmaf(dx, in3[k], tx[k]); tz[k] = fmaf(dz, in3[k], tz[k]); td[k] = fmaf(ddtr, in3[k], td[k]); }
 #pragma unroll
-            for (int d = 0; d < 8; ++d) dwo[d] = fmaf(row[52 + d], outj, dwo[d]);
+            for (int d = 0; d < 8; ++d) two[d] = fmaf(row[52 + d], outj, two[d]);
         }
 #pragma unroll
         for (int k = 0; k < 3; ++k) { dbc[k] += tb[k]; dux[k] += tx[k]; duz[k] += tz[k]; dud[k] += td[k]; }
+#pragma unroll
+        for (int s = 0; s < 8; ++s) { dah[s] += tah[s]; dwo[s] += two[s]; }
+#pragma unroll
+        for (int p = 0; p < 4; ++p) df[p] += tf[p];
+        dD += tD;
         __syncwarp();
     }
     // ---- per-item partial gradients: [item][BL_NG]

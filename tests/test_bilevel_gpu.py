@@ -253,3 +253,21 @@ def test_routing_kernels_match_cpu_loop(n, heads, P, pk):
     assert torch.allclose(outs[0][2][same], outs[1][2][same], rtol=1e-4, atol=1e-5)
     for a, b in zip(outs[0][4:], outs[1][4:]):
         assert (a - b).abs().max() <= 2e-3 * a.abs().max() + 1e-6
+
+
+@pytest.mark.parametrize("n", [3000, 300001])
+def test_gru_parameter_gradients_do_not_grow_one_by_one(n):
+    """Sums over all elements of an input, added sixteen products at a time: 1.4e-7 to 1.7e-7 off the 64-bit sums at either size (a chain over a
+    CTA's elements: 3.1e-7 and 4.6e-7)."""
+    from supergrok15_b200.ops import sg2_bilevel
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, h, dh = torch.randn(n, 18, generator=g, device="cuda"), 0.3 * torch.randn(n, 4, generator=g, device="cuda"), torch.randn(n, 4, generator=g, device="cuda")
+    W, b = (0.2 * torch.randn(3, 4, 22, generator=g, device="cuda")).requires_grad_(), (0.1 * torch.randn(3, 4, generator=g, device="cuda")).requires_grad_()
+    got = torch.autograd.grad(sg2_bilevel.gru(x, h, W, b), (W, b), dh)
+    Wd, bd, xd, hd = W.detach().double().requires_grad_(), b.detach().double().requires_grad_(), x.double(), h.double()
+    xh = torch.cat([xd, hd], -1)
+    z, r = torch.sigmoid(xh @ Wd[0].T + bd[0]), torch.sigmoid(xh @ Wd[1].T + bd[1])
+    c = torch.tanh(torch.cat([xd, r * hd], -1) @ Wd[2].T + bd[2])
+    want = torch.autograd.grad((1 - z) * hd + z * c, (Wd, bd), dh.double())
+    for a, ref in zip(got, want):
+        assert float((a.double() - ref).norm() / ref.norm()) < 2.6e-7
