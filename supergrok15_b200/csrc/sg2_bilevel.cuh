@@ -209,7 +209,7 @@ __device__ __forceinline__ void bl_advance(const HalfConst& cc, const float* __r
 // that does not start at a snapshot is reached by re-running the forward recurrence from the snapshot before it, which trades
 // (snap_every - 1) / 2 extra tile passes on average for 1 / snap_every of the snapshot memory.  The gradients do not depend on it.
 // A warp per chunk: the states before the 16 steps of a tile take 16 KB of shared memory per chunk, which leaves room for ten chunks on
-// an SM; with half a warp each that was 1.25 warps per scheduler and latency all the way (422,755 parameters: 1,395 -> 940 us).
+// an SM; with half a warp each that was 1.25 warps per scheduler and latency all the way (422,755 parameters: 1,395 -> 950 us).
 template <int DIR>
 __device__ void bl_adj3(const Item& it, const float2* __restrict__ gs, const uint32_t* __restrict__ vals_sorted, const float* __restrict__ dctx,
                         const float* __restrict__ dcarry, const float* __restrict__ snaps, int64_t snap_base,
