@@ -27,11 +27,11 @@ from .supergrok15 import SuperGrok15
 
 @torch.no_grad()
 def _copies(tensors):
-    """Copies of a list of tensors.  Dense ones in one foreach call (a product with 1, which allocates its results natively): one or two
+    """Copies of a list of tensors.  Plain dense ones in one foreach call (a product with 1, which allocates its results natively): one or two
     launches and no allocation from Python per tensor."""
-    dense = [t for t in tensors if t.layout == torch.strided]
-    made = iter(torch._foreach_mul(dense, 1.0) if dense else ())
-    return [next(made) if t.layout == torch.strided else t.clone() for t in tensors]
+    plain = [type(t) is torch.Tensor and t.layout == torch.strided for t in tensors]
+    made = iter(torch._foreach_mul([t for t, ok in zip(tensors, plain) if ok], 1.0) if any(plain) else ())
+    return [next(made) if ok else t.detach().clone() for t, ok in zip(tensors, plain)]
 
 
 class SuperGrok2(SuperGrok15):

@@ -47,3 +47,17 @@ def test_bilevel_step_keeps_gradients_that_live_in_reused_buffers(tmp_path):
     assert len(res[True]["meta"]) > 0
     for a, b in zip(res[False]["meta"], res[True]["meta"]):
         assert torch.equal(a, b)
+
+
+def test_copies_are_exact_and_own_their_storage():
+    from supergrok15_b200.optim.supergrok2 import _copies
+    odd = torch.tensor([0.0, -0.0, float("inf"), float("-inf"), float("nan"), 1e-45, 3e38])
+    ts = [odd, odd.double(), odd.bfloat16(), odd.half(), torch.randn(3, 4).t(), torch.zeros(0), torch.eye(3).to_sparse(), torch.nn.Parameter(torch.ones(2))]
+    for a, b in zip(ts, _copies(ts)):
+        assert a.dtype == b.dtype and a.shape == b.shape and a.layout == b.layout and not b.requires_grad
+        if a.layout == torch.strided:
+            assert a.stride() == b.stride() and (a.numel() == 0 or a.data_ptr() != b.data_ptr())
+            number = ~a.isnan()                            # which NaN it is does not matter
+            assert torch.equal(number, ~b.isnan()) and torch.equal(a[number], b[number]) and torch.equal(torch.signbit(a[number]), torch.signbit(b[number]))
+        else:
+            assert torch.equal(a.to_dense(), b.to_dense())
